@@ -37,8 +37,7 @@
 // 4i + 3 in CT_FIELD_EDGES<i>: 0-10, 12, 15, 19, 24, 30.  A cell stores the
 // largest code whose edge does not exceed its cube's edge.  Edges up to 30
 // instead of 0-15 cut the shadow-ray steps of the DI spatial rounds at 1080p
-// from 8.48 to 7.80 per ray, and the walker from 5.06 to 4.86 ms per frame;
-// the build's extra pass (k_field_grow) costs 1.4 ms.
+// from 8.48 to 7.80 per ray, and the walker from 5.06 to 4.86 ms per frame.
 #ifndef CT_FIELD_EDGES0
 #define CT_FIELD_EDGES0 0x03020100u
 #define CT_FIELD_EDGES1 0x07060504u

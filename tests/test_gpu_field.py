@@ -55,3 +55,21 @@ def test_field_arguments_checked():
     assert lib.ct_accel_field(sb.accel.handle, n, 0, None, ctypes.byref(g), ctypes.byref(c), None) == 1
     assert lib.ct_accel_field(sb.accel.handle, 0, 8, None, ctypes.byref(g), ctypes.byref(c), None) == 1
     assert lib.ct_accel_field(sb.accel.handle, 0, 0, None, None, ctypes.byref(c), None) == 1
+
+
+# Grids at the edges of the kernel's tiles (32 cells along x, 64 rows along y
+# and z, 93 with the margin): a row shorter than a word, rows ending inside a
+# word, one row or one tile more, and cubes that reach into a second and a
+# third tile.  Few voxels, so that every edge class occurs.
+@pytest.mark.gpu
+@pytest.mark.parametrize("edge,occupancy", [(5, 0.1), (22, 0.003), (54, 0.0005), (62, 0.0005), (63, 0.3), (94, 0.0002),
+                                            (133, 0.0001)])
+def test_field_at_tile_edges(edge, occupancy):
+    from cube_tracing.frame import SceneBuffers
+    sc = scenes.random_grid_scene(edge, occupancy, emissive_fraction=0.0, seed=edge)
+    sb = SceneBuffers(sc)
+    for octant in range(8):
+        got, gmin = sb.accel.field(0, octant)
+        occ = fieldref.grid_occupancy(sc, 0, gmin, got.shape)
+        assert np.array_equal(got, fieldref.coded_edges(occ, octant)), octant
+    assert sb.accel.info().voxel_count == sc.voxel_count
