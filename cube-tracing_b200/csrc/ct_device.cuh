@@ -175,28 +175,276 @@ __device__ __forceinline__ f3 voxel_center(const DevAccel &A, const DevGrid &g, 
   return (ld3(b.minimum) + ld3(b.maximum)) * 0.5f;
 }
 
+// primitive id of a voxel known to be occupied (its field code is 0)
+__device__ __forceinline__ uint32_t voxel_prim_occupied(const DevAccel &A, const DevGrid &g, int x, int y, int z) {
+  const uint32_t local = (uint32_t)(x & 7) + 8u * (uint32_t)(y & 7) + 64u * (uint32_t)(z & 7);
+  return __ldg(&A.brick_prim[__ldg(&A.brick_pslot[cell_index(g, x >> 3, y >> 3, z >> 3)]) * 512u + local]);
+}
+
 // ---------------------------------------------------------------------------
-// DDA over one instance's brick map, offering every voxel whose box the ray
-// passes within `eps` voxels of.  The box test (and therefore which voxel is
-// hit and at what distance) is rounding-sensitive near voxel edges; visiting
-// this superset of candidates makes the result depend only on the box test
-// itself, never on the traversal order or on how the DDA rounds.
+// The walk over one instance's cell field, offering every voxel whose box the
+// ray passes within `eps` voxels of.  The box test (and therefore which voxel
+// is hit and at what distance) is rounding-sensitive near voxel edges;
+// visiting this superset of candidates makes the result depend only on the
+// box test itself, never on the traversal order or on how the walk rounds.
 //
-// Visitor interface:
-//   bool visit(int x, int y, int z, uint32_t prim)   returns true to stop
-//   float stop_t()                                    cells entered later are skipped
-struct DdaRay {
-  f3 o, d;       // grid-local voxel units (origin relative to the grid's first voxel)
-  f3 inv;        // 1/d (inf for zero components)
-  float eps;
+// Every step leaves one axis-aligned box of cells through its exit face: the
+// cube without occupied cells that the field gives for the ray's octant, with
+// the current cell as its corner, taken when the ray stays clear of the
+// cube's side faces (so that no voxel beside the cube comes within eps of the
+// ray inside it), or a single cell: an occupied one, or the current one when
+// the ray passes near a side face of its cube.  A single cell's voxel is
+// tested, and its neighbours when the ray passes within eps of their faces.
+//
+// What bounds the walks is instruction issue, so a step is built from few and
+// full-rate instructions:
+//  * the ray is mirrored, axis by axis, so that no component of its direction
+//    is negative: every box then begins at the current cell, the far faces
+//    are the exit candidates and the near ones lie behind the ray;
+//  * cells are floats holding whole numbers; adding 2^23 turns one into an
+//    index (and, rounding down, a position into its cell), which takes the
+//    place of the conversions between integers and floats that run at an
+//    eighth of the rate (12 of them a step before);
+//  * the distances to the box's lower faces are carried from the step that
+//    entered it, the entry face's as a large number, so that the near-face
+//    screen is two minima and a compare.
+// On the 1080p terrain frame the shadow walker went from 4.80 to 3.04 ms with
+// this step, the bounce walker from 1.20 to 0.73 ms and the primary rays from
+// 0.98 to 0.78 ms.
+#define CT_WALK_FAR 1e30f
+#define CT_WALK_MAGIC 8388608.0f  // 2^23
+
+// A ray in grid-local voxel units, mirrored.
+//   o.w  margin of the near-face screen, 2 eps + 1e-3
+//   d.w  the stop test's allowance per |1/d| of the exit axis
+//   inv  1 / d (infinity for an axis the ray does not move along);
+//        inv.w (bits) 28 when x is mirrored, else 0
+//   g    cells per axis; g.w (bits) first word of the octant's field, less
+//        the magic numbers of the cell indices
+//   st   word strides of the field along x (+-1 per 8 cells), y and z,
+//        negative on mirrored axes; st.w (bits) t at which the ray leaves
+//        the grid or its range
+struct __align__(16) WalkRay {
+  float4 o, d, inv, g;
+  int4 st;
 };
 
-template <class V>
-__device__ bool dda_visit_cell(const DevAccel &A, const DevGrid &g, int x, int y, int z, V &vis) {
-  int32_t pr = voxel_prim(A, g, x, y, z);
-  if (pr < 0) return false;
-  vis.tests++;
-  return vis.visit(x, y, z, (uint32_t)pr);
+struct WalkState {
+  float cx, cy, cz;  // current cell
+  float qx, qy, qz;  // ray's distance past the cell's lower faces where it entered; CT_WALK_FAR for the entry face
+  float t;           // where it entered
+  float ie;          // |1/d| of the entry axis (-infinity: the walk began in this cell)
+  int steps;
+  int bkey;          // brick of the current cell (work counters)
+};
+
+// one box: its far faces, where and on which axis the ray leaves it
+struct WalkBox {
+  float hx, hy, hz;
+  float t, px, py, pz;
+  float ib;  // |1/d| of the exit axis
+  int ax;
+};
+
+enum { WALK_MORE = 0, WALK_DONE = 1, WALK_LIMIT = 2, WALK_TEST_OWN = 3, WALK_TEST_NEAR = 4 };
+
+__device__ __forceinline__ float walk_eps(const WalkRay &R) { return (R.o.w - 1e-3f) * 0.5f; }
+
+// false: the ray does not overlap the grid within [tmin, tmax].  `ird`: the
+// caller's safe_inverse(d_obj), whose reciprocals are the walk's where the
+// voxel edge is 1.
+__device__ __forceinline__ bool walk_init(const DevAccel &A, const DevGrid &g, f3 o_obj, f3 d_obj, f3 ird, float tmin,
+                                          float tmax, WalkRay &R, WalkState &s) {
+  const float e = A.extent;
+  float o[3], d[3], inv[3];
+  // x / e is x * (1 / e) exactly when e is a power of two (the usual voxel
+  // edges 1 and 2^-5), and one multiply is far cheaper than an IEEE division
+  if ((__float_as_uint(e) & 0x007FFFFFu) == 0u && e > 1e-30f && e < 1e30f) {
+    const float ie = 1.0f / e;
+    o[0] = o_obj.x * ie; o[1] = o_obj.y * ie; o[2] = o_obj.z * ie;
+    d[0] = d_obj.x * ie; d[1] = d_obj.y * ie; d[2] = d_obj.z * ie;
+  } else {
+    o[0] = o_obj.x / e; o[1] = o_obj.y / e; o[2] = o_obj.z / e;
+    d[0] = d_obj.x / e; d[1] = d_obj.y / e; d[2] = d_obj.z / e;
+  }
+  if (e == 1.0f) {
+    inv[0] = ird.x; inv[1] = ird.y; inv[2] = ird.z;
+  } else {
+    inv[0] = 1.f / d[0]; inv[1] = 1.f / d[1]; inv[2] = 1.f / d[2];
+  }
+  const int cells[3] = {g.bdim[0] * CT_BRICK, g.bdim[1] * CT_BRICK, g.bdim[2] * CT_BRICK};
+  float t0 = tmin, t1 = tmax, L = 0.f;
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const float G = (float)cells[a], gm = (float)g.gmin[a];
+    o[a] = o[a] - gm;
+    if (d[a] == 0.f) {
+      if (o[a] < 0.f || o[a] > G) return false;
+      inv[a] = INFINITY;
+    } else {
+      const float ta = (0.f - o[a]) * inv[a], tb = (G - o[a]) * inv[a];
+      t0 = fmaxf(t0, fminf(ta, tb));
+      t1 = fminf(t1, fmaxf(ta, tb));
+    }
+  }
+  if (!(t0 <= t1)) return false;
+  // rounding allowance of the box test (see the comment above)
+  uint32_t oct = 0;
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const float w = o[a] + (float)g.gmin[a];
+    L = fmaxf(L, fmaxf(fabsf(w), fabsf(w + d[a] * t1)));
+    if (d[a] < 0.f) {
+      oct |= 1u << a;
+      o[a] = (float)cells[a] - o[a];
+      d[a] = -d[a];
+    }
+    inv[a] = fabsf(inv[a]);
+  }
+  const float eps = 2e-4f + 4e-6f * L;
+  float c[3], q[3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const float p = __fmaf_rn(d[a], t0, o[a]);
+    c[a] = fmaxf(0.f, fminf(floorf(p), (float)(cells[a] - 1)));
+    q[a] = p - c[a];
+  }
+  const uint32_t Y = (uint32_t)cells[1], Z = (uint32_t)cells[2], bx = (uint32_t)g.bdim[0];
+  const int sy = (oct & 2u) ? -(int)bx : (int)bx, sz = (oct & 4u) ? -(int)(bx * Y) : (int)(bx * Y);
+  uint32_t base = oct * Z * Y * bx;
+  if (oct & 1u) base += bx - 1u;
+  if (oct & 2u) base += (Y - 1u) * bx;
+  if (oct & 4u) base += (Z - 1u) * Y * bx;
+  base -= 0x4B000000u * ((uint32_t)sy + (uint32_t)sz);
+  R.o = make_float4(o[0], o[1], o[2], 2.0f * eps + 1e-3f);
+  // see walk_advance
+  R.d = make_float4(d[0], d[1], d[2], (eps - 2e-4f) * 0.25f + 1e-6f);
+  R.inv = make_float4(inv[0], inv[1], inv[2], __uint_as_float((oct & 1u) ? 28u : 0u));
+  R.g = make_float4((float)cells[0], (float)cells[1], (float)cells[2], __uint_as_float(base));
+  R.st = make_int4((oct & 1u) ? -1 : 1, sy, sz, __float_as_int(t1));
+  s.cx = c[0]; s.cy = c[1]; s.cz = c[2];
+  s.qx = q[0]; s.qy = q[1]; s.qz = q[2];
+  s.t = t0;
+  s.ie = -INFINITY;
+  s.bkey = -1;
+  // the walk's cap: CT_DDA_MAX_STEPS counts from here, so a smaller
+  // A.max_steps (a test's) ends the walk after that many cells
+  s.steps = CT_DDA_MAX_STEPS - (int)A.max_steps;
+  return true;
+}
+
+// The t past which the walk's boxes hold nothing that matters, for a stop
+// distance `stop`: a box further than its allowance past it cannot beat it.
+// Capped below infinity so that a walk whose box the ray never leaves (no
+// direction) ends.
+__device__ __forceinline__ float walk_limit(const WalkRay &R, float stop) {
+  return fminf(fminf(stop + 1e-5f * fabsf(stop) + 1e-6f, __int_as_float(R.st.w)), CT_WALK_FAR);
+}
+
+// bits of a cell's whole-number float in the low mantissa
+__device__ __forceinline__ uint32_t walk_bits(float c) { return __float_as_uint(c + CT_WALK_MAGIC); }
+
+// the field's edge at the current cell, as a float
+__device__ __forceinline__ float walk_field(const uint32_t *field, const WalkRay &R, const WalkState &s) {
+  const uint32_t xb = walk_bits(s.cx);
+  const uint32_t w = __float_as_uint(R.g.w) + (uint32_t)R.st.x * ((xb & 1023u) >> 3) +
+                     (uint32_t)R.st.y * walk_bits(s.cy) + (uint32_t)R.st.z * walk_bits(s.cz);
+  const uint32_t code = (__ldg(field + w) >> (((xb << 2) & 28u) ^ __float_as_uint(R.inv.w))) & 15u;
+  const bool lo = code < 8u;
+  const uint32_t b =
+      __byte_perm(lo ? CT_FIELD_EDGES0 : CT_FIELD_EDGES2, lo ? CT_FIELD_EDGES1 : CT_FIELD_EDGES3, code & 7u);
+  return __uint_as_float(__byte_perm(b, 0x4B000000u, 0x7440u)) - CT_WALK_MAGIC;  // byte 0 of b
+}
+
+// the box of `k` cells per axis from the current cell, clipped to the grid
+__device__ __forceinline__ WalkBox walk_box(const WalkRay &R, const WalkState &s, float k) {
+  WalkBox b;
+  b.hx = fminf(s.cx + k, R.g.x);
+  b.hy = fminf(s.cy + k, R.g.y);
+  b.hz = fminf(s.cz + k, R.g.z);
+  // 0 * infinity (on a face the ray does not move towards) is no exit
+  const float tx = (b.hx - R.o.x) * R.inv.x, ty = (b.hy - R.o.y) * R.inv.y, tz = (b.hz - R.o.z) * R.inv.z;
+  b.t = fminf(fminf(tx, ty), fminf(tz, INFINITY));
+  b.ax = tx == b.t ? 0 : (ty == b.t ? 1 : 2);
+  b.ib = b.ax == 0 ? R.inv.x : (b.ax == 1 ? R.inv.y : R.inv.z);
+  b.px = __fmaf_rn(R.d.x, b.t, R.o.x);
+  b.py = __fmaf_rn(R.d.y, b.t, R.o.y);
+  b.pz = __fmaf_rn(R.d.z, b.t, R.o.z);
+  return b;
+}
+
+// Screen on a box: false only when the ray stays well clear (2 eps + 1e-3
+// voxels) of every face of the box other than its entry and exit faces, and
+// crosses the box too far from the entry/exit edge to pass near it.  The ray
+// does not cross those other faces' planes inside the box and moves away
+// from the lower ones, so it is nearest to them where it enters, and to the
+// upper ones where it leaves.  A voxel outside the box that the ray passes
+// within eps of, while inside the box, lies beyond one of these faces: none
+// when this is false.
+__device__ __forceinline__ bool walk_near(const WalkRay &R, const WalkState &s, const WalkBox &b) {
+  const float ex = b.ax == 0 ? CT_WALK_FAR : b.hx - b.px, ey = b.ax == 1 ? CT_WALK_FAR : b.hy - b.py,
+              ez = b.ax == 2 ? CT_WALK_FAR : b.hz - b.pz;
+  const float q = fminf(fminf(s.qx, s.qy), s.qz), h = fminf(fminf(ex, ey), ez);
+  // eps + margin = 1.5 margin - 5e-4
+  return fminf(q, h) < R.o.w || !(b.t - s.t > __fmaf_rn(1.5f, R.o.w, -5e-4f) * (s.ie + b.ib));
+}
+
+// Moves on to the cell behind the box's exit face; false when the walk ends.
+//
+// The next box begins at b.t, computed in grid-local coordinates whose
+// rounding (a few ulps of the coordinate scale L, with eps = 2e-4 + 4e-6 L) is
+// amplified by |1/d| on the exit axis: a voxel behind that face has box-test
+// distance at least b.t - 1e-6 L |1/d|.  The walk ends only when that bound
+// (R.d.w holds the allowance) lies past the limit, so that a voxel on the
+// same face plane as the best hit (an exact tie) is still seen.
+__device__ __forceinline__ bool walk_advance(const WalkRay &R, WalkState &s, const WalkBox &b, float lim) {
+  if (b.t - fminf(R.d.w * b.ib, CT_WALK_FAR) > lim) return false;
+  // the ray's cell clamped to the box; rounding down to a whole number by the
+  // magic addition (positions are within [-1, 1025])
+  const float fx = __fadd_rd(b.px, CT_WALK_MAGIC) - CT_WALK_MAGIC, fy = __fadd_rd(b.py, CT_WALK_MAGIC) - CT_WALK_MAGIC,
+              fz = __fadd_rd(b.pz, CT_WALK_MAGIC) - CT_WALK_MAGIC;
+  s.cx = b.ax == 0 ? b.hx : fmaxf(s.cx, fminf(fx, b.hx - 1.0f));
+  s.cy = b.ax == 1 ? b.hy : fmaxf(s.cy, fminf(fy, b.hy - 1.0f));
+  s.cz = b.ax == 2 ? b.hz : fmaxf(s.cz, fminf(fz, b.hz - 1.0f));
+  s.qx = b.ax == 0 ? CT_WALK_FAR : b.px - s.cx;
+  s.qy = b.ax == 1 ? CT_WALK_FAR : b.py - s.cy;
+  s.qz = b.ax == 2 ? CT_WALK_FAR : b.pz - s.cz;
+  s.t = b.t;
+  s.ie = b.ib;
+  return s.cx < R.g.x && s.cy < R.g.y && s.cz < R.g.z;
+}
+
+// One step.  WALK_TEST_OWN / WALK_TEST_NEAR: the walk stands in a single cell
+// whose voxel (and near neighbours) / near neighbours are to be tested before
+// it moves on (box: that cell).
+template <bool COUNT>
+__device__ __forceinline__ int walk_step(const uint32_t *field, const WalkRay &R, WalkState &s, float lim,
+                                         RayStats &rs, WalkBox &b) {
+  if (++s.steps > CT_DDA_MAX_STEPS) return WALK_LIMIT;
+  if (COUNT) {
+    // bricks per axis < 128; a mirrored grid's bricks are its bricks
+    const int key = (int)(((walk_bits(s.cx) >> 3) & 127u) | (((walk_bits(s.cy) >> 3) & 127u) << 7) |
+                          (((walk_bits(s.cz) >> 3) & 127u) << 14));
+    if (key != s.bkey) {
+      rs.bricks++;
+      s.bkey = key;
+    }
+  }
+  const float k = walk_field(field, R, s);
+  b = walk_box(R, s, fmaxf(k, 1.0f));
+  if (k == 0.0f) return WALK_TEST_OWN;
+  if (walk_near(R, s, b)) {
+    // the cell alone: a test only when the ray passes near one of its faces
+    b = walk_box(R, s, 1.0f);
+    if (walk_near(R, s, b)) return WALK_TEST_NEAR;
+  }
+  return walk_advance(R, s, b, lim) ? WALK_MORE : WALK_DONE;
+}
+
+// the grid's cell of a mirrored one
+__device__ __forceinline__ int3 walk_cell(const WalkRay &R, int x, int y, int z) {
+  return make_int3(R.st.x < 0 ? (int)R.g.x - 1 - x : x, R.st.y < 0 ? (int)R.g.y - 1 - y : y,
+                   R.st.z < 0 ? (int)R.g.z - 1 - z : z);
 }
 
 // t interval over which the ray lies within eps of the plane coordinate c on
@@ -212,16 +460,16 @@ __device__ __forceinline__ void near_interval(float o, float d, float inv, float
   hi = fminf(fmaxf(ta, tb), t1);
 }
 
-// Neighbours of cell c that the ray passes within eps of while it crosses c
-// (t in [t_in, t_out]), except the previous and the next cell of the walk,
-// as a mask over the 3x3x3 block (bit (dz+1)*9 + (dy+1)*3 + (dx+1)); the walk
-// visits them in increasing bit order.  A pure function of its arguments, out
-// of line: the walk calls it only after dda_near_faces found the ray close to
-// a face.
-__device__ __noinline__ uint32_t dda_neighbour_mask(DdaRay r, int c0, int c1, int c2, float t_in, float t_out,
-                                                    int entry_axis, int exit_axis, int s0, int s1, int s2) {
-  const int c[3] = {c0, c1, c2}, step[3] = {s0, s1, s2};
-  const float o[3] = {r.o.x, r.o.y, r.o.z}, d[3] = {r.d.x, r.d.y, r.d.z}, inv[3] = {r.inv.x, r.inv.y, r.inv.z};
+// Neighbours of the (mirrored) cell c that the ray passes within eps of while
+// it crosses c (t in [t_in, t_out]), except the previous and the next cell of
+// the walk, as a mask over the 3x3x3 block (bit (dz+1)*9 + (dy+1)*3 +
+// (dx+1)).  Axis 3: none.  Out of line: the walk calls it only after
+// walk_near found the ray close to a face.
+__device__ __noinline__ uint32_t walk_neighbour_mask(float4 ro, float4 rd, float4 ri, float c0, float c1, float c2,
+                                                     float t_in, float t_out, int entry_axis, int exit_axis) {
+  const float c[3] = {c0, c1, c2};
+  const float o[3] = {ro.x, ro.y, ro.z}, d[3] = {rd.x, rd.y, rd.z}, inv[3] = {ri.x, ri.y, ri.z};
+  const float eps = (ro.w - 1e-3f) * 0.5f;
   // near-face intervals: [axis][0 = lower face, 1 = upper face]
   float lo[3][2], hi[3][2];
   bool any_other = false;
@@ -229,22 +477,26 @@ __device__ __noinline__ uint32_t dda_neighbour_mask(DdaRay r, int c0, int c1, in
   for (int a = 0; a < 3; a++) {
 #pragma unroll
     for (int f = 0; f < 2; f++) {
-      near_interval(o[a], d[a], inv[a], (float)(c[a] + f), r.eps, t_in, t_out, lo[a][f], hi[a][f]);
-      bool is_entry = (a == entry_axis) && (f == (step[a] > 0 ? 0 : 1));
-      bool is_exit = (a == exit_axis) && (f == (step[a] > 0 ? 1 : 0));
+      near_interval(o[a], d[a], inv[a], c[a] + (float)f, eps, t_in, t_out, lo[a][f], hi[a][f]);
+      const bool is_entry = a == entry_axis && f == 0, is_exit = a == exit_axis && f == 1;
       if (!is_entry && !is_exit && lo[a][f] <= hi[a][f]) any_other = true;
     }
   }
   if (!any_other) {
     // only the corner between the entry and exit faces can be near
-    if (entry_axis < 0 || entry_axis == exit_axis) return 0u;
-    int fe = step[entry_axis] > 0 ? 0 : 1, fx = step[exit_axis] > 0 ? 1 : 0;
-    float l = fmaxf(lo[entry_axis][fe], lo[exit_axis][fx]), h = fminf(hi[entry_axis][fe], hi[exit_axis][fx]);
+    if (entry_axis > 2 || entry_axis == exit_axis) return 0u;
+    float l = t_in, h = t_out;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      if (a == entry_axis) { l = fmaxf(l, lo[a][0]); h = fminf(h, hi[a][0]); }
+      if (a == exit_axis) { l = fmaxf(l, lo[a][1]); h = fminf(h, hi[a][1]); }
+    }
     if (l > h) return 0u;
-    int n[3] = {0, 0, 0};
-    n[entry_axis] -= step[entry_axis];
-    n[exit_axis] += step[exit_axis];
-    return 1u << ((n[2] + 1) * 9 + (n[1] + 1) * 3 + (n[0] + 1));
+    const int w[3] = {1, 3, 9};
+    int bit = 13;
+#pragma unroll
+    for (int a = 0; a < 3; a++) bit += (a == exit_axis ? w[a] : 0) - (a == entry_axis ? w[a] : 0);
+    return 1u << bit;
   }
   // general case: every neighbour whose touching faces are all near at a
   // common time, except the previous and the next cell of the walk
@@ -254,17 +506,17 @@ __device__ __noinline__ uint32_t dda_neighbour_mask(DdaRay r, int c0, int c1, in
       for (int dx = -1; dx <= 1; dx++) {
         const int dd[3] = {dx, dy, dz};
         if (dx == 0 && dy == 0 && dz == 0) continue;
-        int nz = (dx != 0) + (dy != 0) + (dz != 0);
+        const int nz = (dx != 0) + (dy != 0) + (dz != 0);
         if (nz == 1) {
-          int a = dx != 0 ? 0 : (dy != 0 ? 1 : 2);
-          if (a == entry_axis && dd[a] == -step[a]) continue;
-          if (a == exit_axis && dd[a] == step[a]) continue;
+          const int a = dx != 0 ? 0 : (dy != 0 ? 1 : 2);
+          if (a == entry_axis && dd[a] < 0) continue;
+          if (a == exit_axis && dd[a] > 0) continue;
         }
         float l = t_in, h = t_out;
 #pragma unroll
         for (int a = 0; a < 3; a++) {
           if (dd[a] == 0) continue;
-          int f = dd[a] > 0 ? 1 : 0;
+          const int f = dd[a] > 0 ? 1 : 0;
           l = fmaxf(l, lo[a][f]);
           h = fminf(h, hi[a][f]);
         }
@@ -273,274 +525,80 @@ __device__ __noinline__ uint32_t dda_neighbour_mask(DdaRay r, int c0, int c1, in
       }
   return mask;
 }
-
-// Cheap screen for dda_neighbour_mask, on a box of cells [lo, hi]: false
-// only when the ray stays well clear (2 eps + 1e-3 voxels) of every face of
-// the box other than its entry and exit faces, and crosses the box too far
-// from the entry/exit edge to pass near it.  The segment does not cross
-// those other faces' planes, so its distance to each is smallest at an end
-// point.  A voxel outside the box that the ray passes within eps of, while
-// inside the box, lies beyond one of these faces: none when this is false.
-__device__ __forceinline__ bool dda_near_box(const DdaRay &r, const int lo[3], const int hi[3], float t_in, float t_out,
-                                             int entry_axis, int exit_axis, const int step[3]) {
-  const float m = 2.0f * r.eps + 1e-3f;
-  const float o[3] = {r.o.x, r.o.y, r.o.z}, d[3] = {r.d.x, r.d.y, r.d.z};
-  bool near = false;
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    const float p0 = o[a] + d[a] * t_in, p1 = o[a] + d[a] * t_out;
-    const float dlo = fminf(p0, p1) - (float)lo[a], dhi = (float)(hi[a] + 1) - fmaxf(p0, p1);
-    const bool lo_excl = (a == entry_axis && step[a] > 0) || (a == exit_axis && step[a] < 0);
-    const bool hi_excl = (a == entry_axis && step[a] < 0) || (a == exit_axis && step[a] > 0);
-    near = near || (!lo_excl && !(dlo >= m)) || (!hi_excl && !(dhi >= m));
-  }
-  if (near) return true;
-  if (entry_axis >= 0 && entry_axis != exit_axis) {
-    const float inv[3] = {r.inv.x, r.inv.y, r.inv.z};
-    float ie = 0.f, ix = 0.f;
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      if (a == entry_axis) ie = fabsf(inv[a]);
-      if (a == exit_axis) ix = fabsf(inv[a]);
-    }
-    if (!(t_out - t_in > (r.eps + m) * (ie + ix))) return true;
-  }
-  return false;
-}
-// the same screen on the single cell c
-__device__ __forceinline__ bool dda_near_faces(const DdaRay &r, const int c[3], float t_in, float t_out, int entry_axis,
-                                               int exit_axis, const int step[3]) {
-  return dda_near_box(r, c, c, t_in, t_out, entry_axis, exit_axis, step);
+// the axis of the face the walk entered the cell through (3: it began there)
+__device__ __forceinline__ int walk_entry(const WalkState &s) {
+  return s.qx >= CT_WALK_FAR ? 0 : (s.qy >= CT_WALK_FAR ? 1 : (s.qz >= CT_WALK_FAR ? 2 : 3));
 }
 
-// Walk state, resumable: dda_run advances it by a bounded number of cells so
-// that a warp can refill lanes whose walk has ended (k_trace_shadow).  Kept
-// in named scalars so that a walk lives in registers.
-struct DdaState {
-  DdaRay r;
-  int cx, cy, cz;  // current cell
-  float t_in, t1;
-  int entry_axis;
-  int cur_bkey;
-  uint32_t cur_ent;
-  int steps;
-};
-
-__device__ __forceinline__ int ct_step_of(float d) { return d > 0.f ? 1 : (d < 0.f ? -1 : 0); }
-
-// false: the ray does not overlap the grid within [tmin, tmax]
-__device__ __forceinline__ bool dda_init(const DevAccel &A, const DevGrid &g, f3 o_obj, f3 d_obj, float tmin,
-                                         float tmax, DdaState &s) {
-  const float e = A.extent;
-  DdaRay &r = s.r;
-  // x / e is x * (1 / e) exactly when e is a power of two (the usual voxel
-  // edges 1 and 2^-5), and one multiply is far cheaper than an IEEE division
-  if ((__float_as_uint(e) & 0x007FFFFFu) == 0u && e > 1e-30f && e < 1e30f) {
-    const float ie = 1.0f / e;
-    r.o = f3{o_obj.x * ie - (float)g.gmin[0], o_obj.y * ie - (float)g.gmin[1], o_obj.z * ie - (float)g.gmin[2]};
-    r.d = f3{d_obj.x * ie, d_obj.y * ie, d_obj.z * ie};
-  } else {
-    r.o = f3{o_obj.x / e - (float)g.gmin[0], o_obj.y / e - (float)g.gmin[1], o_obj.z / e - (float)g.gmin[2]};
-    r.d = f3{d_obj.x / e, d_obj.y / e, d_obj.z / e};
-  }
-  r.inv = f3{1.f / r.d.x, 1.f / r.d.y, 1.f / r.d.z};
-  const float G[3] = {(float)(g.bdim[0] * CT_BRICK), (float)(g.bdim[1] * CT_BRICK), (float)(g.bdim[2] * CT_BRICK)};
-  const float o[3] = {r.o.x, r.o.y, r.o.z}, d[3] = {r.d.x, r.d.y, r.d.z}, inv[3] = {r.inv.x, r.inv.y, r.inv.z};
-  float t0 = tmin, t1 = tmax;
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    if (d[a] == 0.f) {
-      if (o[a] < 0.f || o[a] > G[a]) return false;
-    } else {
-      float ta = (0.f - o[a]) * inv[a], tb = (G[a] - o[a]) * inv[a];
-      t0 = fmaxf(t0, fminf(ta, tb));
-      t1 = fminf(t1, fmaxf(ta, tb));
-    }
-  }
-  if (!(t0 <= t1)) return false;
-  // rounding allowance of the box test (see the comment above)
-  float L = 0.f;
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    float g0 = (float)g.gmin[a];
-    L = fmaxf(L, fmaxf(fabsf(o[a] + g0), fabsf(o[a] + g0 + d[a] * t1)));
-  }
-  r.eps = 2e-4f + 4e-6f * L;
-  int cc[3];
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    float p = __fmaf_rn(d[a], t0, o[a]);
-    int ci = (int)floorf(p);
-    int gi = g.bdim[a] * CT_BRICK;
-    cc[a] = ci < 0 ? 0 : (ci >= gi ? gi - 1 : ci);
-  }
-  s.cx = cc[0]; s.cy = cc[1]; s.cz = cc[2];
-  s.t_in = t0;
-  s.t1 = t1;
-  s.entry_axis = -1;
-  s.cur_bkey = -1;
-  s.cur_ent = 0;
-  // the walk's cap: CT_DDA_MAX_STEPS counts from here, so a smaller
-  // A.max_steps (a test's) ends the walk after that many cells
-  s.steps = CT_DDA_MAX_STEPS - (int)A.max_steps;
-  return true;
-}
-
-enum { DDA_DONE = 0, DDA_MORE = 1, DDA_LIMIT = 2 };
-
-// leaving the box [lo, hi] (cells) along one axis
-__device__ __forceinline__ void ct_box_exit(int a, int st, int lo, int hi, float o, float inv, float &tb, int &ax) {
-  if (st == 0) return;
-  const float tt = ((float)(st > 0 ? hi + 1 : lo) - o) * inv;
-  if (tt < tb) { tb = tt; ax = a; }
-}
-// the cell after leaving the box at tb: across the exit face on the exit
-// axis, the ray's cell clamped to the box on the others
-__device__ __forceinline__ int ct_box_next(bool exit_axis, int st, int lo, int hi, float d, float tb, float o) {
-  if (exit_axis) return st > 0 ? hi + 1 : lo - 1;
-  const int ci = (int)floorf(__fmaf_rn(d, tb, o));
-  return ci < lo ? lo : (ci > hi ? hi : ci);
-}
-
-// Advances the walk by at most `budget` steps.  Every step leaves one
-// axis-aligned box of cells through its exit face: a brick that is not NEAR
-// (no voxel in or next to it: nothing to test), a cube of cells with no
-// occupied cell that has the current cell as its corner and extends in the
-// ray's directions (the brick's octant field, see DevAccel), taken when the
-// ray stays clear of the cube's side faces (so that no voxel beside the cube
-// comes within eps of the ray inside it), or a single cell: an occupied one,
-// or the current one when the ray passes near a side face of its cube.  A
-// single cell's voxel is tested, and its neighbours when the ray passes
-// within eps of their faces.  DDA_DONE: the walk ended (left the grid,
-// passed stop_t, or the visitor stopped it).
+// Visitor interface of the walks that test in place:
+//   bool visit(int x, int y, int z, uint32_t prim)   returns true to stop
+//   float stop_t()                                    boxes entered later are skipped
+//   uint32_t tests                                    voxels offered
 //
-// ct_ray_octant: the field of the ray's octant (an axis the ray does not
-// move along counts as increasing); cell_field: the field's edge k at cell
-// (x, y, z); ct_box_axis: the box on one axis, the cube of edge k from cell
-// c towards the ray's direction, clipped to the grid's `cells`.
-__device__ __forceinline__ uint32_t ct_ray_octant(int sx, int sy, int sz) {
-  return (sx < 0 ? 1u : 0u) | (sy < 0 ? 2u : 0u) | (sz < 0 ? 4u : 0u);
-}
-__device__ __forceinline__ int cell_field(const DevAccel &A, const DevGrid &g, uint32_t octant, int x, int y, int z) {
-  // a grid has at most 1024^3 cells (10-bit voxel coordinates), so the words
-  // of its 8 octants (one per 8 cells each) index in 32 bits
-  const uint32_t Y = (uint32_t)g.bdim[1] * CT_BRICK, Z = (uint32_t)g.bdim[2] * CT_BRICK;
-  const uint32_t w = ((octant * Z + (uint32_t)z) * Y + (uint32_t)y) * (uint32_t)g.bdim[0] + ((uint32_t)x >> 3);
-  return ct_field_edge((__ldg(A.cell_field + g.field_offset + w) >> ((x & 7) * 4)) & 15u);
-}
-__device__ __forceinline__ void ct_box_axis(int c, int st, int k, int cells, int &lo, int &hi) {
-  const int e = k > 0 ? k - 1 : 0;
-  if (st < 0) {
-    lo = max(c - e, 0);
-    hi = c;
-  } else {
-    lo = c;
-    hi = min(c + e, cells - 1);
-  }
-}
-
-// A box (the occupied-free cube from the cell field) is taken whole only when
-// the ray stays clear of its side faces (dda_near_box); otherwise the step
-// is the current cell alone.  Returns true when the step is a single cell
-// whose voxel and near neighbours must be tested: an occupied cell (k == 0)
-// or a fallback cell.  Updates the box and its exit.
-__device__ __forceinline__ bool ct_screen_box(const DdaRay &r, int k, int cx, int cy, int cz, int sx, int sy, int sz,
-                                              float t_in, int entry_axis, int &lox, int &hix, int &loy, int &hiy,
-                                              int &loz, int &hiz, float &tb, int &ax) {
-  if (k == 0) return true;
-  const int lo3[3] = {lox, loy, loz}, hi3[3] = {hix, hiy, hiz}, st3[3] = {sx, sy, sz};
-  if (!dda_near_box(r, lo3, hi3, t_in, tb, entry_axis, ax, st3)) return false;
-  lox = hix = cx;
-  loy = hiy = cy;
-  loz = hiz = cz;
-  tb = INFINITY;
-  ax = 0;
-  ct_box_exit(0, sx, lox, hix, r.o.x, r.inv.x, tb, ax);
-  ct_box_exit(1, sy, loy, hiy, r.o.y, r.inv.y, tb, ax);
-  ct_box_exit(2, sz, loz, hiz, r.o.z, r.inv.z, tb, ax);
-  return true;
-}
-
+// The tests of the single cell a walk stands in (box b), then the step out of
+// it; `st` is what walk_step returned.
 template <class V>
-__device__ __forceinline__ int dda_run(const DevAccel &A, const DevGrid &g, DdaState &s, V &vis, RayStats &rs,
-                                       int budget) {
-  const DdaRay &r = s.r;
-  const int sx = ct_step_of(r.d.x), sy = ct_step_of(r.d.y), sz = ct_step_of(r.d.z);
-  const uint32_t octant = ct_ray_octant(sx, sy, sz);
-  const int gx = g.bdim[0] * CT_BRICK, gy = g.bdim[1] * CT_BRICK, gz = g.bdim[2] * CT_BRICK;
-  int cx = s.cx, cy = s.cy, cz = s.cz;
-  float t_in = s.t_in;
-  int entry_axis = s.entry_axis;
-  int result = DDA_MORE;
-  for (int it = 0; it < budget; it++) {
-    if (++s.steps > CT_DDA_MAX_STEPS) { result = DDA_LIMIT; break; }
-    const int bkey = (cx >> 3) | ((cy >> 3) << 10) | ((cz >> 3) << 20);  // bricks per axis < 1024
-    if (bkey != s.cur_bkey) {
-      rs.bricks++;
-      s.cur_bkey = bkey;
-    }
-    const int k = cell_field(A, g, octant, cx, cy, cz);
-    int lox, hix, loy, hiy, loz, hiz;
-    ct_box_axis(cx, sx, k, gx, lox, hix);
-    ct_box_axis(cy, sy, k, gy, loy, hiy);
-    ct_box_axis(cz, sz, k, gz, loz, hiz);
-    float tb = INFINITY;
-    int ax = 0;
-    ct_box_exit(0, sx, lox, hix, r.o.x, r.inv.x, tb, ax);
-    ct_box_exit(1, sy, loy, hiy, r.o.y, r.inv.y, tb, ax);
-    ct_box_exit(2, sz, loz, hiz, r.o.z, r.inv.z, tb, ax);
-    if (ct_screen_box(r, k, cx, cy, cz, sx, sy, sz, t_in, entry_axis, lox, hix, loy, hiy, loz, hiz, tb, ax)) {
-      // a single cell: its voxel, then the neighbours the ray passes near
-      if (k == 0) {
-        const int32_t pr = voxel_prim(A, g, cx, cy, cz);
-        if (pr >= 0) {
-          vis.tests++;
-          if (vis.visit(cx, cy, cz, (uint32_t)pr)) { result = DDA_DONE; break; }
-        }
-      }
-      const int c3[3] = {cx, cy, cz}, st3[3] = {sx, sy, sz};
-      if (dda_near_faces(r, c3, t_in, tb, entry_axis, ax, st3)) {
-        bool stop = false;
-        for (uint32_t m = dda_neighbour_mask(r, cx, cy, cz, t_in, tb, entry_axis, ax, sx, sy, sz); m; m &= m - 1u) {
-          const int nb = __ffs(m) - 1;
-          if (dda_visit_cell(A, g, cx + nb % 3 - 1, cy + (nb / 3) % 3 - 1, cz + nb / 9 - 1, vis)) {
-            stop = true;
-            break;
-          }
-        }
-        if (stop) { result = DDA_DONE; break; }
-      }
-    }
-    // The next box begins at tb, computed in grid-local coordinates whose
-    // rounding (a few ulps of the coordinate scale L, with r.eps = 2e-4 +
-    // 4e-6 L) is amplified by |1/d| on the exit axis: a voxel behind that
-    // face has box-test distance at least tb - 1e-6 L |1/d|.  The walk ends
-    // only when that bound lies past the stop distance, so that a voxel on
-    // the same face plane as the best hit (an exact tie) is still seen.
-    const float st = vis.stop_t();
-    const float slack = ((r.eps - 2e-4f) * 0.25f + 1e-6f) * fabsf(ax == 0 ? r.inv.x : (ax == 1 ? r.inv.y : r.inv.z));
-    if (tb - slack > st + 1e-5f * fabsf(st) + 1e-6f || tb - slack >= s.t1) { result = DDA_DONE; break; }
-    cx = ct_box_next(ax == 0, sx, lox, hix, r.d.x, tb, r.o.x);
-    cy = ct_box_next(ax == 1, sy, loy, hiy, r.d.y, tb, r.o.y);
-    cz = ct_box_next(ax == 2, sz, loz, hiz, r.d.z, tb, r.o.z);
-    const bool out = ax == 0 ? (cx < 0 || cx >= gx) : (ax == 1 ? (cy < 0 || cy >= gy) : (cz < 0 || cz >= gz));
-    if (out) { result = DDA_DONE; break; }
-    t_in = tb;
-    entry_axis = ax;
+__device__ __forceinline__ int walk_test(const DevAccel &A, const DevGrid &g, const WalkRay &R, WalkState &s,
+                                         const WalkBox &b, int st, float &lim, V &vis) {
+  const int cx = (int)(walk_bits(s.cx) & 1023u), cy = (int)(walk_bits(s.cy) & 1023u),
+            cz = (int)(walk_bits(s.cz) & 1023u);
+  bool near = true;
+  if (st == WALK_TEST_OWN) {
+    const int3 c = walk_cell(R, cx, cy, cz);
+    vis.tests++;
+    if (vis.visit(c.x, c.y, c.z, voxel_prim_occupied(A, g, c.x, c.y, c.z))) return WALK_DONE;
+    near = walk_near(R, s, b);
   }
-  s.cx = cx; s.cy = cy; s.cz = cz;
-  s.t_in = t_in;
-  s.entry_axis = entry_axis;
-  return result;
+  if (near) {
+    for (uint32_t m = walk_neighbour_mask(R.o, R.d, R.inv, s.cx, s.cy, s.cz, s.t, b.t, walk_entry(s), b.ax); m;
+         m &= m - 1u) {
+      const int nb = __ffs(m) - 1;
+      const int3 c = walk_cell(R, cx + nb % 3 - 1, cy + (nb / 3) % 3 - 1, cz + nb / 9 - 1);
+      const int32_t pr = voxel_prim(A, g, c.x, c.y, c.z);
+      if (pr < 0) continue;
+      vis.tests++;
+      if (vis.visit(c.x, c.y, c.z, (uint32_t)pr)) return WALK_DONE;
+    }
+  }
+  lim = walk_limit(R, vis.stop_t());
+  return walk_advance(R, s, b, lim) ? WALK_MORE : WALK_DONE;
 }
 
+// Runs the walk for at most `rounds` rounds of up to `inner` steps and the
+// tests of the cell they end in.  The lanes of a warp leave the steps
+// together, so that the tests (long, and needed by most walks once) run side
+// by side instead of one lane at a time: with the tests inside the step loop
+// 5.9 of 32 lanes were active per instruction in the path tracer (512x512,
+// 8 samples of depth 3 in a 128^3 grid at 25%, forward: 4.8 -> 1.9 ms).
+template <bool COUNT, class V>
+__device__ __forceinline__ int walk_run(const DevAccel &A, const DevGrid &g, const WalkRay &R, WalkState &s, V &vis,
+                                        RayStats &rs, int rounds, int inner) {
+  const uint32_t *field = A.cell_field + g.field_offset;
+  float lim = walk_limit(R, vis.stop_t());
+  for (int it = 0; it < rounds; it++) {
+    int st = WALK_MORE;
+    WalkBox b;
+#pragma unroll 1
+    for (int k = 0; k < inner && st == WALK_MORE; k++) st = walk_step<COUNT>(field, R, s, lim, rs, b);
+    if (st >= WALK_TEST_OWN) st = walk_test(A, g, R, s, b, st, lim, vis);
+    if (st != WALK_MORE) return st;
+  }
+  return WALK_MORE;
+}
+
+// Steps per round of a walk that runs to its end in place: 8 (primary rays
+// 0.757 ms per 1080p frame against 0.776 ms at 4 and 0.800 ms at 2).
+#ifndef CT_WALK_INNER
+#define CT_WALK_INNER 8
+#endif
 // Returns false if the walk hit its step cap (error latched by the caller).
 template <class V>
-__device__ bool dda_traverse(const DevAccel &A, const DevGrid &g, f3 o_obj, f3 d_obj, float tmin, float tmax, V &vis,
-                             RayStats &rs) {
-  DdaState s;
-  if (!dda_init(A, g, o_obj, d_obj, tmin, tmax, s)) return true;
-  return dda_run(A, g, s, vis, rs, CT_DDA_MAX_STEPS + 1) != DDA_LIMIT;
+__device__ __forceinline__ bool walk_traverse(const DevAccel &A, const DevGrid &g, f3 o_obj, f3 d_obj, f3 ird,
+                                              float tmin, float tmax, V &vis, RayStats &rs) {
+  WalkRay R;
+  WalkState s;
+  if (!walk_init(A, g, o_obj, d_obj, ird, tmin, tmax, R, s)) return true;
+  return walk_run<true>(A, g, R, s, vis, rs, CT_DDA_MAX_STEPS + 1, CT_WALK_INNER) != WALK_LIMIT;
 }
 
 // ---------------------------------------------------------------------------
@@ -660,8 +718,9 @@ __device__ HitRecord trace_primary(const DevAccel &A, f3 o, f3 d, float tmin, fl
     const DevGrid &g = A.grids[i];
     f3 ro = xyz(mul(g.world2obj_tlas, mk4(o, 1.0f)));
     f3 rd = xyz(mul(g.world2obj_tlas, mk4(d, 0.0f)));
-    PrimaryVisitor v{A, g, ro, rd, safe_inverse(rd), radius, inv_radius, tmin, tmax, i, best, 0u};
-    if (!dda_traverse(A, g, ro, rd, tmin, best.hit ? best.t : tmax, v, rs)) ct_latch_error(CT_ERR_ITER_LIMIT, 1, pixel);
+    const f3 ird = safe_inverse(rd);
+    PrimaryVisitor v{A, g, ro, rd, ird, radius, inv_radius, tmin, tmax, i, best, 0u};
+    if (!walk_traverse(A, g, ro, rd, ird, tmin, best.hit ? best.t : tmax, v, rs)) ct_latch_error(CT_ERR_ITER_LIMIT, 1, pixel);
     rs.voxel_tests += v.tests;
   }
   return best;
@@ -696,7 +755,7 @@ __device__ bool vertex_visible(const DevAccel &A, f3 o, f3 d, float distance, ui
     QueryVisitor<FixedRay> v{A, g, FixedRay{ro, rd}, radius, inv_radius, false, distance, i, true, target_t,
                              target_g, has_target, t_inst, t_prim, blk, 0u};
     float tlim = fminf(distance, target_t);
-    if (!dda_traverse(A, g, ro, rd, 0.f, tlim, v, rs)) ct_latch_error(CT_ERR_ITER_LIMIT, 2, pixel);
+    if (!walk_traverse(A, g, ro, rd, safe_inverse(rd), 0.f, tlim, v, rs)) ct_latch_error(CT_ERR_ITER_LIMIT, 2, pixel);
     rs.voxel_tests += v.tests;
     if (blk.hit) return false;
   }
@@ -778,7 +837,7 @@ __device__ bool vertex_visible_prev(const DevAccel &A, const FrameView &F, f3 o,
     const f3 rd = xyz(mul(g.world2obj_inst, mk4(d, 0.0f)));
     PrevQueryVisitor v{A, g, F.aabbs, F.instances[i].first_primitive_index, ro, rd, safe_inverse(rd), radius,
                        inv_radius, distance, i, target_t, target_g, has_target, t_inst, t_prim, false, 0u};
-    if (!dda_traverse(A, g, ro, rd, 0.f, distance, v, rs)) ct_latch_error(CT_ERR_ITER_LIMIT, 3, pixel);
+    if (!walk_traverse(A, g, ro, rd, safe_inverse(rd), 0.f, distance, v, rs)) ct_latch_error(CT_ERR_ITER_LIMIT, 3, pixel);
     rs.voxel_tests += v.tests;
     if (v.blocked) return false;
   }
@@ -791,18 +850,18 @@ __device__ bool vertex_visible_prev(const DevAccel &A, const FrameView &F, f3 o,
 // candidates are tested: the stop distance is fixed (min(distance, target
 // t)), and the ray is blocked when ANY candidate voxel other than the target
 // passes the box test with t in [0, distance] and a key below the target's.
-// So a lane may step on past a dilated cell and leave that cell's tests (its
-// own voxel and the neighbours the ray passes within eps of, exactly the
-// candidates dda_run offers) to a job that the warp tests later, 32 jobs at a
-// time, one per lane.  The stepping phase keeps only the cheap part of a
-// dilated cell (its occupancy bit and the near-face screen, which rule out
-// nearly all of them); the box tests and neighbour masks, rare and long, run
-// with full warps instead of one lane at a time.  A lane may enumerate a few
-// cells past its first blocker; the decision is the same.
+// So a lane may step on past a cell with tests to make (its own voxel and the
+// neighbours the ray passes within eps of, exactly the candidates walk_run
+// offers) and leave them to a job that the warp tests later, 32 jobs at a
+// time, one per lane.  The stepping phase keeps only the cheap part (the
+// field's word and the near-face screen, which rule out nearly all cells);
+// the box tests and neighbour masks, rare and long, run with full warps
+// instead of one lane at a time.  A lane may enumerate a few cells past its
+// first blocker; the decision is the same.
 
 // a lane's ray as both phases read it, kept in shared memory
 struct ShadowRay {
-  DdaRay r;               // grid-local, as dda_init made it
+  WalkRay r;              // as walk_init made it
   f3 ro, rd, ird;         // object space, and safe_inverse(rd) as the box test takes it
   float tmax;             // the query distance
   float target_t;         // key of the target voxel (INFINITY: none)
@@ -812,47 +871,37 @@ struct ShadowRay {
   uint32_t inst;          // instance being walked
 };
 
-// The ray's object-space form for instance `inst`, then dda_init over that
-// instance's grid (false: no overlap).  `known`: the caller already has the
-// object-space origin `kro`, direction `krd` and safe_inverse(krd) `kird`
-// for this instance (the target test's), which are used as they are.
-__device__ __forceinline__ bool shadow_ray_instance(const DevAccel &A, ShadowRay &R, DdaState &s, uint32_t inst, f3 o,
-                                                    f3 d, bool known = false, f3 kro = f3{}, f3 krd = f3{},
-                                                    f3 kird = f3{}) {
-  const DevGrid &g = A.grids[inst];
-  const f3 ro = known ? kro : xyz(mul(g.world2obj_inst, mk4(o, 1.0f)));
-  const f3 rd = known ? krd : xyz(mul(g.world2obj_inst, mk4(d, 0.0f)));
-  if (!dda_init(A, g, ro, rd, 0.f, fminf(R.tmax, R.target_t), s)) return false;
-  R.r = s.r;
+// walk_init over instance `inst`'s grid (false: no overlap) for the ray's
+// object-space form in that instance
+__device__ __forceinline__ bool shadow_ray_instance(const DevAccel &A, ShadowRay &R, WalkState &s, uint32_t inst,
+                                                    f3 ro, f3 rd, f3 ird) {
+  WalkRay r;
+  if (!walk_init(A, A.grids[inst], ro, rd, ird, 0.f, fminf(R.tmax, R.target_t), r, s)) return false;
+  R.r = r;
   R.ro = ro;
   R.rd = rd;
-  if (known) {
-    R.ird = kird;
-  } else if (A.extent == 1.0f) {
-    // with a voxel edge of 1 the walk's direction is rd itself (rd * 1), so
-    // its reciprocals are safe_inverse's wherever rd is not 0
-    R.ird = f3{rd.x == 0.0f ? 1e12f : s.r.inv.x, rd.y == 0.0f ? 1e12f : s.r.inv.y,
-               rd.z == 0.0f ? 1e12f : s.r.inv.z};
-  } else {
-    R.ird = safe_inverse(rd);
-  }
+  R.ird = ird;
   R.inst = inst;
   return true;
 }
 
 // the first instance from `inst` on whose grid the ray overlaps; false when
 // none is left
-__device__ __forceinline__ bool shadow_ray_next(const DevAccel &A, ShadowRay &R, DdaState &s, uint32_t inst, f3 o,
+__device__ __forceinline__ bool shadow_ray_next(const DevAccel &A, ShadowRay &R, WalkState &s, uint32_t inst, f3 o,
                                                 f3 d) {
-  for (; inst < A.n_grids; inst++)
-    if (shadow_ray_instance(A, R, s, inst, o, d)) return true;
+  for (; inst < A.n_grids; inst++) {
+    const DevGrid &g = A.grids[inst];
+    const f3 ro = xyz(mul(g.world2obj_inst, mk4(o, 1.0f)));
+    const f3 rd = xyz(mul(g.world2obj_inst, mk4(d, 0.0f)));
+    if (shadow_ray_instance(A, R, s, inst, ro, rd, safe_inverse(rd))) return true;
+  }
   return false;
 }
 
 // is_vertex_visible's set-up (light.glsl:82-105): the target voxel's key by
 // its own box test, then the first instance to walk.  False: nothing to walk
 // (the ray is visible).
-__device__ __forceinline__ bool shadow_ray_begin(const DevAccel &A, ShadowRay &R, DdaState &s, f3 o, f3 d,
+__device__ __forceinline__ bool shadow_ray_begin(const DevAccel &A, ShadowRay &R, WalkState &s, f3 o, f3 d,
                                                  float distance, uint32_t t_inst, uint32_t t_prim,
                                                  bool check_instance) {
   R.tmax = distance;
@@ -876,7 +925,7 @@ __device__ __forceinline__ bool shadow_ray_begin(const DevAccel &A, ShadowRay &R
       // the first instance to walk is usually the target's: its
       // object-space ray is the one just made
       if (t_inst == 0u) {
-        if (shadow_ray_instance(A, R, s, 0u, o, d, true, ro, rd, ird)) return true;
+        if (shadow_ray_instance(A, R, s, 0u, ro, rd, ird)) return true;
         return shadow_ray_next(A, R, s, 1u, o, d);
       }
     }
@@ -898,92 +947,56 @@ __device__ __forceinline__ bool shadow_blocks(const DevAccel &A, const DevGrid &
   return t < R.target_t || (t == R.target_t && gp < R.target_g);
 }
 
-// A dilated cell's job: cell (cx, cy, cz) crossed over [t_in, t_out],
-// entered across `entry` (-1: the walk began in it) and left across `exit`.
-// Packed: x = cx | cy << 16, y = cz | lane << 16 | (entry + 1) << 24 | exit << 28.
-__device__ __forceinline__ uint4 shadow_job(int cx, int cy, int cz, float t_in, float t_out, int entry, int exit,
+// A cell's job: the (mirrored) cell crossed over [t_in, t_out], entered
+// across axis `entry` (3: the walk began in it) and left across `exit`, with
+// its own voxel to test or its near neighbours alone.
+// Packed: x = cx | cy << 10 | cz << 20 | entry << 30, y = lane | exit << 5 | own << 7 | near << 8.
+__device__ __forceinline__ uint4 shadow_job(const WalkRay &R, const WalkState &s, const WalkBox &b, bool own,
                                             uint32_t lane) {
-  return make_uint4((uint32_t)cx | ((uint32_t)cy << 16),
-                    (uint32_t)cz | (lane << 16) | ((uint32_t)(entry + 1) << 24) | ((uint32_t)exit << 28),
-                    __float_as_uint(t_in), __float_as_uint(t_out));
+  const uint32_t near = !own || walk_near(R, s, b) ? 1u : 0u;
+  return make_uint4((walk_bits(s.cx) & 1023u) | ((walk_bits(s.cy) & 1023u) << 10) |
+                        ((walk_bits(s.cz) & 1023u) << 20) | ((uint32_t)walk_entry(s) << 30),
+                    lane | ((uint32_t)b.ax << 5) | (own ? 128u : 0u) | (near << 8), __float_as_uint(s.t),
+                    __float_as_uint(b.t));
 }
-__device__ __forceinline__ uint32_t shadow_job_lane(uint4 j) { return (j.y >> 16) & 31u; }
+__device__ __forceinline__ uint32_t shadow_job_lane(uint4 j) { return j.y & 31u; }
 
-// The tests of one job, those dda_run makes in a dilated cell: the cell's own
+// The tests of one job, those walk_run makes in a single cell: the cell's own
 // voxel, then the neighbours the ray passes within eps of.
 __device__ __forceinline__ bool shadow_job_blocked(const DevAccel &A, const ShadowRay &R, uint4 j, uint32_t &tests) {
   const DevGrid &g = A.grids[R.inst];
-  const int cx = (int)(j.x & 0xFFFFu), cy = (int)(j.x >> 16), cz = (int)(j.y & 0xFFFFu);
-  const int entry = (int)((j.y >> 24) & 15u) - 1, ax = (int)(j.y >> 28);
-  const float t_in = __uint_as_float(j.z), t_out = __uint_as_float(j.w);
-  const int32_t own = voxel_prim(A, g, cx, cy, cz);
-  if (own >= 0) {
+  const int cx = (int)(j.x & 0x3FFu), cy = (int)((j.x >> 10) & 0x3FFu), cz = (int)((j.x >> 20) & 0x3FFu);
+  if (j.y & 128u) {
+    const int3 c = walk_cell(R.r, cx, cy, cz);
     tests++;
-    if (shadow_blocks(A, g, R, cx, cy, cz, (uint32_t)own)) return true;
+    if (shadow_blocks(A, g, R, c.x, c.y, c.z, voxel_prim_occupied(A, g, c.x, c.y, c.z))) return true;
   }
-  const int sx = ct_step_of(R.r.d.x), sy = ct_step_of(R.r.d.y), sz = ct_step_of(R.r.d.z);
-  const int c3[3] = {cx, cy, cz}, st3[3] = {sx, sy, sz};
-  if (!dda_near_faces(R.r, c3, t_in, t_out, entry, ax, st3)) return false;
-  for (uint32_t m = dda_neighbour_mask(R.r, cx, cy, cz, t_in, t_out, entry, ax, sx, sy, sz); m; m &= m - 1u) {
+  if (!(j.y & 256u)) return false;
+  for (uint32_t m = walk_neighbour_mask(R.r.o, R.r.d, R.r.inv, (float)cx, (float)cy, (float)cz, __uint_as_float(j.z),
+                                        __uint_as_float(j.w), (int)(j.x >> 30), (int)((j.y >> 5) & 3u));
+       m; m &= m - 1u) {
     const int k = __ffs(m) - 1;
-    const int x = cx + k % 3 - 1, y = cy + (k / 3) % 3 - 1, z = cz + k / 9 - 1;
-    const int32_t pr = voxel_prim(A, g, x, y, z);
+    const int3 c = walk_cell(R.r, cx + k % 3 - 1, cy + (k / 3) % 3 - 1, cz + k / 9 - 1);
+    const int32_t pr = voxel_prim(A, g, c.x, c.y, c.z);
     if (pr < 0) continue;
     tests++;
-    if (shadow_blocks(A, g, R, x, y, z, (uint32_t)pr)) return true;
+    if (shadow_blocks(A, g, R, c.x, c.y, c.z, (uint32_t)pr)) return true;
   }
   return false;
 }
 
-// One step of dda_run without its visits: leaves the current box; a single
-// cell with a test to make sets `job` (its tests are the caller's).  `stop`
-// is the visitor's fixed stop distance.  DDA_MORE, DDA_DONE (left the grid or
-// passed the stop distance) or DDA_LIMIT.  A step makes one dependent load,
-// the cell field's word, and spends the rest of its issue slots on box
-// arithmetic and the side-face screen.
-__device__ __forceinline__ int shadow_step(const DevAccel &A, const DevGrid &g, const DdaRay &r, DdaState &s, float stop,
+// One step of the walk without its visits: leaves the current box; a single
+// cell with a test to make sets `job` (its tests are the caller's).
+// WALK_MORE, WALK_DONE (left the grid or passed the limit) or WALK_LIMIT.
+template <bool COUNT>
+__device__ __forceinline__ int shadow_step(const uint32_t *field, const WalkRay &R, WalkState &s, float lim,
                                            uint32_t lane, RayStats &rs, bool &job, uint4 &jb) {
-  job = false;
-  if (++s.steps > CT_DDA_MAX_STEPS) return DDA_LIMIT;
-  const int sx = ct_step_of(r.d.x), sy = ct_step_of(r.d.y), sz = ct_step_of(r.d.z);
-  const int cx = s.cx, cy = s.cy, cz = s.cz;
-  const int bkey = (cx >> 3) | ((cy >> 3) << 10) | ((cz >> 3) << 20);  // bricks per axis < 1024
-  if (bkey != s.cur_bkey) {
-    rs.bricks++;
-    s.cur_bkey = bkey;
-  }
-  const int k = cell_field(A, g, ct_ray_octant(sx, sy, sz), cx, cy, cz);
-  const int gx = g.bdim[0] * CT_BRICK, gy = g.bdim[1] * CT_BRICK, gz = g.bdim[2] * CT_BRICK;
-  int lox, hix, loy, hiy, loz, hiz;
-  ct_box_axis(cx, sx, k, gx, lox, hix);
-  ct_box_axis(cy, sy, k, gy, loy, hiy);
-  ct_box_axis(cz, sz, k, gz, loz, hiz);
-  float tb = INFINITY;
-  int ax = 0;
-  ct_box_exit(0, sx, lox, hix, r.o.x, r.inv.x, tb, ax);
-  ct_box_exit(1, sy, loy, hiy, r.o.y, r.inv.y, tb, ax);
-  ct_box_exit(2, sz, loz, hiz, r.o.z, r.inv.z, tb, ax);
-  if (ct_screen_box(r, k, cx, cy, cz, sx, sy, sz, s.t_in, s.entry_axis, lox, hix, loy, hiy, loz, hiz, tb, ax)) {
-    // a job only when it has a test to make: the cell's own voxel, or a
-    // neighbour face the ray passes near
-    const int c3[3] = {cx, cy, cz}, st3[3] = {sx, sy, sz};
-    if (k == 0 || dda_near_faces(r, c3, s.t_in, tb, s.entry_axis, ax, st3)) {
-      job = true;
-      jb = shadow_job(cx, cy, cz, s.t_in, tb, s.entry_axis, ax, lane);
-    }
-  }
-  // dda_run's end test (see there for the slack)
-  const float slack = ((r.eps - 2e-4f) * 0.25f + 1e-6f) * fabsf(ax == 0 ? r.inv.x : (ax == 1 ? r.inv.y : r.inv.z));
-  if (tb - slack > stop + 1e-5f * fabsf(stop) + 1e-6f || tb - slack >= s.t1) return DDA_DONE;
-  const int nx = ct_box_next(ax == 0, sx, lox, hix, r.d.x, tb, r.o.x);
-  const int ny = ct_box_next(ax == 1, sy, loy, hiy, r.d.y, tb, r.o.y);
-  const int nz = ct_box_next(ax == 2, sz, loz, hiz, r.d.z, tb, r.o.z);
-  const bool out = ax == 0 ? (nx < 0 || nx >= gx) : (ax == 1 ? (ny < 0 || ny >= gy) : (nz < 0 || nz >= gz));
-  if (out) return DDA_DONE;
-  s.cx = nx; s.cy = ny; s.cz = nz;
-  s.t_in = tb;
-  s.entry_axis = ax;
-  return DDA_MORE;
+  WalkBox b;
+  const int st = walk_step<COUNT>(field, R, s, lim, rs, b);
+  job = st >= WALK_TEST_OWN;
+  if (!job) return st;
+  jb = shadow_job(R, s, b, st == WALK_TEST_OWN, lane);
+  return walk_advance(R, s, b, lim) ? WALK_MORE : WALK_DONE;
 }
 
 // ---------------------------------------------------------------------------

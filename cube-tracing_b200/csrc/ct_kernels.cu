@@ -99,11 +99,11 @@ __device__ __forceinline__ void pixel_of(uint32_t &x, uint32_t &y) {
 // ---------------------------------------------------------------------------
 // pass 1, front half: primary visibility (rgen.glsl:46-201, 319) with the
 // closest-hit shader (rchit.glsl:18-54) and miss shader (rmiss.glsl:25-28)
-// 10 blocks of 128 per SM (48 registers, spills to L1): 0.97 ms per 1080p
-// frame against 1.02 ms at 8 blocks (64 registers), 1.09 ms at 6 and 1.07
-// ms when the register count is left free
+// 6 blocks of 128 per SM (80 registers): 0.77 ms for a 1277x719 frame over
+// four instances against 0.86 ms at 8 blocks and 0.89 ms at 10 (48 registers,
+// spilling); on the 1080p terrain all three take 0.78 ms
 #ifndef CT_PRIMARY_MIN_BLOCKS
-#define CT_PRIMARY_MIN_BLOCKS 10
+#define CT_PRIMARY_MIN_BLOCKS 6
 #endif
 __global__ void __launch_bounds__(128, CT_PRIMARY_MIN_BLOCKS) k_trace_primary(ct_push_constant pc, DevAccel A, ct_params P) {
   __shared__ BlockConsts B;
@@ -833,20 +833,20 @@ __global__ void __launch_bounds__(128) k_spatial_resolve(ct_push_constant pc, ct
 //   refill: lanes without a ray take the next rays of the queue (one atomic
 //           per warp), set up the walk and store the ray in shared memory;
 //   step:   every lane with a walk leaves up to CT_WALK_BUDGET boxes of its
-//           ray (shadow_step), queueing a job per dilated cell with a test to
-//           make, until the warp's job queue holds 32 jobs or no walk
+//           ray (shadow_step), queueing a job per cell with a test to make,
+//           until the warp's job queue holds 32 jobs or no walk
 //           continues;
 //   test:   the warp tests the queued jobs, one per lane, and marks the rays
 //           they block.
 // A ray is answered once it is blocked or its walk has ended with none of its
 // jobs blocking.  Writes one byte per ray (1 = visible) at the ray's slot.
-// Boxes per round: 8 (5.07 ms per 1080p frame against 5.18 ms at 12 and
-// 5.32 ms at 16).
+// Boxes per round: 8 (3.03 ms per 1080p frame against 3.08 ms at 6, 3.13 ms
+// at 12 and 3.23 ms at 16).
 #ifndef CT_WALK_BUDGET
 #define CT_WALK_BUDGET 8
 #endif
-// blocks of 256 per SM the register budget is sized for (64 registers; at
-// five blocks, 48 registers, the spills cost more than the occupancy gains)
+// blocks of 256 per SM the register budget is sized for (64 registers; 3.03
+// ms per 1080p frame against 3.14 ms at three blocks)
 #ifndef CT_SHADOW_MIN_BLOCKS
 #define CT_SHADOW_MIN_BLOCKS 4
 #endif
@@ -866,9 +866,9 @@ __global__ void __launch_bounds__(256, CT_SHADOW_MIN_BLOCKS) k_trace_shadow(DevA
   const uint32_t n = ws.q.count[0];
   uint32_t *cursor = ws.q.count + 1;
   RayStats rs = {};
-  DdaState st;
-  float stop = 0.f;         // the walk's fixed stop distance
-  int walk = DDA_DONE;      // the lane's walk: DDA_MORE while it continues
+  WalkState st;
+  float lim = 0.f;          // the walk's fixed limit
+  int walk = WALK_DONE;     // the lane's walk: WALK_MORE while it continues
   bool active = false;      // the lane holds an unanswered ray
   bool exhausted = false;
   uint32_t slot = 0, qid = 0;
@@ -896,8 +896,8 @@ __global__ void __launch_bounds__(256, CT_SHADOW_MIN_BLOCKS) k_trace_shadow(DevA
           if (shadow_ray_begin(A, R, st, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z}, a.w, c.x & 0x7FFFFFFFu, c.y,
                                (c.x & 0x80000000u) != 0)) {
             active = true;
-            walk = DDA_MORE;
-            stop = fminf(R.tmax, R.target_t);
+            walk = WALK_MORE;
+            lim = walk_limit(R.r, fminf(R.tmax, R.target_t));
           } else {
             ws.vis[slot] = 1;  // nothing to walk: visible
           }
@@ -908,21 +908,20 @@ __global__ void __launch_bounds__(256, CT_SHADOW_MIN_BLOCKS) k_trace_shadow(DevA
     // step
     uint32_t njobs = 0;
     {
-      const DevGrid &g = A.grids[active ? rays[lane].inst : 0];
+      const uint32_t *field = A.cell_field + A.grids[active ? rays[lane].inst : 0].field_offset;
       for (int it = 0; it < CT_WALK_BUDGET; it++) {
         bool job = false;
         uint4 jb;
-        if (walk == DDA_MORE) {
-          // the ray from shared memory: the registers it frees buy a fourth
-          // block per SM (walker 10.50 ms per 1080p frame against 10.60 ms
-          // with the ray in registers at three blocks)
-          walk = shadow_step(A, g, rays[lane].r, st, stop, lane, rs, job, jb);
-          if (walk == DDA_LIMIT) ct_latch_error(CT_ERR_ITER_LIMIT, 2, slot / CT_VIS_SLOTS);
+        if (walk == WALK_MORE) {
+          // the ray from shared memory: the registers it frees buy the
+          // fourth block per SM
+          walk = shadow_step<COUNT>(field, rays[lane].r, st, lim, lane, rs, job, jb);
+          if (walk == WALK_LIMIT) ct_latch_error(CT_ERR_ITER_LIMIT, 2, slot / CT_VIS_SLOTS);
         }
         const unsigned jm = __ballot_sync(0xFFFFFFFFu, job);
         if (job) jobs[njobs + __popc(jm & lanes_below)] = jb;
         njobs += __popc(jm);
-        if (njobs >= 32u || !__any_sync(0xFFFFFFFFu, walk == DDA_MORE)) break;
+        if (njobs >= 32u || !__any_sync(0xFFFFFFFFu, walk == WALK_MORE)) break;
       }
     }
     // test
@@ -941,14 +940,15 @@ __global__ void __launch_bounds__(256, CT_SHADOW_MIN_BLOCKS) k_trace_shadow(DevA
       if ((s_blocked[warp] >> lane) & 1u) {
         ws.vis[slot] = 0;
         active = false;
-        walk = DDA_DONE;
-      } else if (walk != DDA_MORE) {
+        walk = WALK_DONE;
+      } else if (walk != WALK_MORE) {
         // the walk of this instance ended unblocked: the next instance, if any
         const float4 a = ws.q.a[qid], b = ws.q.b[qid];
         ShadowRay &R = rays[lane];
         if (R.inst + 1 < A.n_grids &&
             shadow_ray_next(A, R, st, R.inst + 1, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z})) {
-          walk = DDA_MORE;
+          walk = WALK_MORE;
+          lim = walk_limit(R.r, fminf(R.tmax, R.target_t));
         } else {
           ws.vis[slot] = 1;
           active = false;
@@ -1268,10 +1268,12 @@ __global__ void __launch_bounds__(128) k_pt_start(ct_push_constant pc, DevAccel 
 #ifndef CT_EXTEND_MIN_BLOCKS
 #define CT_EXTEND_MIN_BLOCKS 3
 #endif
-// boxes per turn: 4 (1.04-1.05 ms per 1080p frame against 1.06-1.07 ms at
-// 6, 1.10 ms at 8 and 1.15 ms at 12)
-#ifndef CT_EXTEND_BUDGET
-#define CT_EXTEND_BUDGET 4
+// per turn, 2 rounds of up to 4 steps and the tests of the cell they end in:
+// 0.73 ms per 1080p frame against 0.75 ms for 2 rounds of 2 or one of 4, and
+// 0.76 ms for one round of 8
+#ifndef CT_EXTEND_ROUNDS
+#define CT_EXTEND_ROUNDS 2
+#define CT_EXTEND_INNER 4
 #endif
 template <bool COUNT>
 __global__ void __launch_bounds__(256, CT_EXTEND_MIN_BLOCKS) k_pt_extend(DevAccel A, ct_params P, PtWork w, int qi) {
@@ -1279,8 +1281,9 @@ __global__ void __launch_bounds__(256, CT_EXTEND_MIN_BLOCKS) k_pt_extend(DevAcce
   uint32_t *cursor = w.count + 2 * qi + 1;
   const float4 *q = w.q[qi];
   const uint32_t lane = threadIdx.x & 31u;
-  __shared__ ObjRay s_ray[256];
-  ObjRay &R = s_ray[threadIdx.x];
+  __shared__ WalkRay s_walk[256];
+  __shared__ ObjRay s_obj[256];
+  const ClosestRay R{s_walk[threadIdx.x], s_obj[threadIdx.x]};
   RayStats rs = {};
   ClosestWalk cw;
   uint32_t pixel = 0, qid = 0;
@@ -1316,7 +1319,7 @@ __global__ void __launch_bounds__(256, CT_EXTEND_MIN_BLOCKS) k_pt_extend(DevAcce
       }
     }
     if (!__any_sync(0xFFFFFFFFu, active || !exhausted)) break;
-    if (active && closest_walk_advance(A, cw, CT_EXTEND_BUDGET, pixel, rs, ray, R) == DDA_DONE) {
+    if (active && closest_walk_advance<COUNT>(A, cw, CT_EXTEND_ROUNDS, CT_EXTEND_INNER, pixel, rs, ray, R) == WALK_DONE) {
       if (cw.best.hit) rs.bounce_hits++;
       w.hit[pixel] = cw.best.hit ? make_uint4(cw.best.inst, cw.best.prim, cw.best.gprim, 0u)
                                  : make_uint4(0xFFFFFFFFu, 0u, 0u, 0u);
@@ -1409,12 +1412,7 @@ __global__ void __launch_bounds__(128) k_pt_finish(ct_push_constant pc, DevAccel
     for (int round = CT_PT_TAIL_ROUND; round < CT_PT_MAX_ITER; round++) {
       rs.bounce++;
       ClosestWalk cw;
-      NoObjRay R;
-      const auto ray = [&](f3 &o, f3 &d) { o = path.origin; d = path.dir; };
-      if (!closest_walk_begin(A, cw, path.origin, path.dir, R))
-        while (closest_walk_advance(A, cw, 1 << 20, pixel, rs, ray, R) == DDA_MORE) {
-        }
-      if (cw.best.hit) rs.bounce_hits++;
+      if (closest_walk(A, cw, path.origin, path.dir, pixel, rs)) rs.bounce_hits++;
       VisRecord nee{false};
       path_shade(F, A, pp, path, cw.best.hit, cw.best.inst, cw.best.prim, cw.best.gprim, nee, pixel);
       if (nee.has) {
