@@ -852,10 +852,72 @@ __global__ void __launch_bounds__(128) k_spatial_resolve(ct_push_constant pc, ct
 #endif
 #define CT_SHADOW_WARPS 8
 #define CT_SHADOW_JOBS 64  // a step adds at most 32 jobs to fewer than 32
+// A source of rays: the frame's queue, or a caller's batch of queries.
+//   length()               rays to walk
+//   reserve(n, leader)     the next n positions, the same for the whole warp
+//   ray(i, o, d, dist)     ray i;  target(i, inst, prim): true to check it
+//   answer(i, visible)     its result;  pixel(i): for error reports
+struct QueueRays {
+  Workspace ws;
+  __device__ uint32_t length() const { return ws.q.count[0]; }
+  // one atomic per warp refill on the queue's cursor
+  __device__ uint32_t reserve(uint32_t n, uint32_t leader) {
+    uint32_t base = 0;
+    if ((threadIdx.x & 31u) == leader) base = atomicAdd(ws.q.count + 1, n);
+    return __shfl_sync(0xFFFFFFFFu, base, leader);
+  }
+  __device__ void ray(uint32_t i, f3 &o, f3 &d, float &dist) const {
+    const float4 a = ws.q.a[i], b = ws.q.b[i];
+    o = f3{a.x, a.y, a.z};
+    d = f3{b.x, b.y, b.z};
+    dist = a.w;
+  }
+  __device__ bool target(uint32_t i, uint32_t &inst, uint32_t &prim) const {
+    const uint2 c = ws.q.c[i];
+    inst = c.x & 0x7FFFFFFFu;
+    prim = c.y;
+    return (c.x & 0x80000000u) != 0;
+  }
+  __device__ uint32_t slot(uint32_t i) const { return __float_as_uint(ws.q.b[i].w); }
+  __device__ void answer(uint32_t i, uint8_t v) const { ws.vis[slot(i)] = v; }
+  __device__ uint32_t pixel(uint32_t i) const { return slot(i) / CT_VIS_SLOTS; }
+};
+// The batch is split evenly over the warps, which refill from their own part:
+// no counter to keep anywhere, and parts of tens of rays even out.
+struct BatchRays {
+  const ct_ray_query *q;
+  uint8_t *out;
+  uint32_t n, per_warp;  // rays, rays per warp
+  uint32_t next, end;    // this warp's part, set by length()
+  __device__ uint32_t length() {
+    const uint64_t w = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    next = (uint32_t)min(w * per_warp, (uint64_t)n);
+    end = (uint32_t)min((w + 1u) * per_warp, (uint64_t)n);
+    return end;
+  }
+  __device__ uint32_t reserve(uint32_t k, uint32_t) {
+    const uint32_t base = next;
+    next += k;
+    return base;
+  }
+  __device__ void ray(uint32_t i, f3 &o, f3 &d, float &dist) const {
+    o = ld3(q[i].origin);
+    d = ld3(q[i].direction);
+    dist = q[i].distance;
+  }
+  __device__ bool target(uint32_t i, uint32_t &inst, uint32_t &prim) const {
+    inst = q[i].target_instance;
+    prim = q[i].target_primitive;
+    return (q[i].flags & CT_QUERY_CHECK_TARGET) != 0;
+  }
+  __device__ void answer(uint32_t i, uint8_t v) const { out[i] = v; }
+  __device__ uint32_t pixel(uint32_t i) const { return i; }
+};
+
 // COUNT: the work counters of CT_PARAM_COUNT_RAYS, compiled out of the
-// instantiation frames run without them
-template <bool COUNT>
-__global__ void __launch_bounds__(256, CT_SHADOW_MIN_BLOCKS) k_trace_shadow(DevAccel A, ct_params P, Workspace ws) {
+// instantiations that run without them
+template <bool COUNT, class Rays>
+__device__ __forceinline__ void shadow_walker(const DevAccel &A, Rays src, RayStats &rs) {
   __shared__ ShadowRay s_ray[CT_SHADOW_WARPS][32];
   __shared__ uint4 s_job[CT_SHADOW_WARPS][CT_SHADOW_JOBS];
   __shared__ uint32_t s_blocked[CT_SHADOW_WARPS];
@@ -863,43 +925,37 @@ __global__ void __launch_bounds__(256, CT_SHADOW_MIN_BLOCKS) k_trace_shadow(DevA
   const uint32_t lanes_below = (1u << lane) - 1u;
   ShadowRay *rays = s_ray[warp];
   uint4 *jobs = s_job[warp];
-  const uint32_t n = ws.q.count[0];
-  uint32_t *cursor = ws.q.count + 1;
-  RayStats rs = {};
+  const uint32_t n = src.length();
   WalkState st;
   float lim = 0.f;          // the walk's fixed limit
   int walk = WALK_DONE;     // the lane's walk: WALK_MORE while it continues
   bool active = false;      // the lane holds an unanswered ray
   bool exhausted = false;
-  uint32_t slot = 0, qid = 0;
+  uint32_t qid = 0;
   for (;;) {
     // refill
     const bool need = !active && !exhausted;
     const unsigned needmask = __ballot_sync(0xFFFFFFFFu, need);
     if (needmask) {
-      const uint32_t leader = __ffs(needmask) - 1;
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(cursor, (uint32_t)__popc(needmask));
-      base = __shfl_sync(0xFFFFFFFFu, base, leader);
+      const uint32_t base = src.reserve((uint32_t)__popc(needmask), (uint32_t)__ffs(needmask) - 1u);
       if (need) {
-        const uint32_t id = base + __popc(needmask & lanes_below);
-        if (id >= n) {
+        qid = base + __popc(needmask & lanes_below);
+        if (qid >= n) {
           exhausted = true;
         } else {
-          const float4 a = ws.q.a[id];
-          const float4 b = ws.q.b[id];
-          const uint2 c = ws.q.c[id];
-          qid = id;
-          slot = __float_as_uint(b.w);
+          f3 o, d;
+          float dist;
+          uint32_t inst, prim;
+          src.ray(qid, o, d, dist);
+          const bool check = src.target(qid, inst, prim);
           rs.shadow++;
           ShadowRay &R = rays[lane];
-          if (shadow_ray_begin(A, R, st, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z}, a.w, c.x & 0x7FFFFFFFu, c.y,
-                               (c.x & 0x80000000u) != 0)) {
+          if (shadow_ray_begin(A, R, st, o, d, dist, inst, prim, check)) {
             active = true;
             walk = WALK_MORE;
             lim = walk_limit(R.r, fminf(R.tmax, R.target_t));
           } else {
-            ws.vis[slot] = 1;  // nothing to walk: visible
+            src.answer(qid, 1);  // nothing to walk: visible
           }
         }
       }
@@ -916,7 +972,7 @@ __global__ void __launch_bounds__(256, CT_SHADOW_MIN_BLOCKS) k_trace_shadow(DevA
           // the ray from shared memory: the registers it frees buy the
           // fourth block per SM
           walk = shadow_step<COUNT>(field, rays[lane].r, st, lim, lane, rs, job, jb);
-          if (walk == WALK_LIMIT) ct_latch_error(CT_ERR_ITER_LIMIT, 2, slot / CT_VIS_SLOTS);
+          if (walk == WALK_LIMIT) ct_latch_error(CT_ERR_ITER_LIMIT, 2, src.pixel(qid));
         }
         const unsigned jm = __ballot_sync(0xFFFFFFFFu, job);
         if (job) jobs[njobs + __popc(jm & lanes_below)] = jb;
@@ -938,27 +994,44 @@ __global__ void __launch_bounds__(256, CT_SHADOW_MIN_BLOCKS) k_trace_shadow(DevA
     // answer
     if (active) {
       if ((s_blocked[warp] >> lane) & 1u) {
-        ws.vis[slot] = 0;
+        src.answer(qid, 0);
         active = false;
         walk = WALK_DONE;
       } else if (walk != WALK_MORE) {
         // the walk of this instance ended unblocked: the next instance, if any
-        const float4 a = ws.q.a[qid], b = ws.q.b[qid];
+        f3 o, d;
+        float dist;
         ShadowRay &R = rays[lane];
-        if (R.inst + 1 < A.n_grids &&
-            shadow_ray_next(A, R, st, R.inst + 1, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z})) {
+        bool more = false;
+        if (R.inst + 1 < A.n_grids) {
+          src.ray(qid, o, d, dist);
+          more = shadow_ray_next(A, R, st, R.inst + 1, o, d);
+        }
+        if (more) {
           walk = WALK_MORE;
           lim = walk_limit(R.r, fminf(R.tmax, R.target_t));
         } else {
-          ws.vis[slot] = 1;
+          src.answer(qid, 1);
           active = false;
         }
       }
     }
     __syncwarp();
   }
+}
+
+template <bool COUNT>
+__global__ void __launch_bounds__(256, CT_SHADOW_MIN_BLOCKS) k_trace_shadow(DevAccel A, ct_params P, Workspace ws) {
+  RayStats rs = {};
+  shadow_walker<COUNT>(A, QueueRays{ws}, rs);
   rs.walker_bricks = rs.bricks;
   if constexpr (COUNT) count_rays(P, rs);
+}
+
+// ct_trace_visibility: one thread per ray kept 5.7 of 32 lanes busy
+__global__ void __launch_bounds__(256, CT_SHADOW_MIN_BLOCKS) k_query_visibility(DevAccel A, BatchRays rays) {
+  RayStats rs = {};
+  shadow_walker<false>(A, rays, rs);
 }
 
 // The rays k_di_gen1 queued against the previous scene after an edit
@@ -1796,14 +1869,6 @@ __global__ void __launch_bounds__(128, CT_PT_SPATIAL_MIN_BLOCKS) k_pt_spatial(ct
 
 // ---------------------------------------------------------------------------
 // batch queries (ct_trace_visibility / ct_trace_closest)
-__global__ void __launch_bounds__(256) k_query_visibility(DevAccel A, const ct_ray_query *q, uint32_t n, uint8_t *out) {
-  RayStats rs = {};
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const ct_ray_query r = q[i];
-    out[i] = vertex_visible(A, ld3(r.origin), ld3(r.direction), r.distance, r.target_instance, r.target_primitive,
-                            (r.flags & CT_QUERY_CHECK_TARGET) != 0, i, rs) ? 1 : 0;
-  }
-}
 __global__ void __launch_bounds__(256) k_query_closest(DevAccel A, const ct_ray_query *q, uint32_t n, ct_ray_hit *out) {
   RayStats rs = {};
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1817,12 +1882,32 @@ __global__ void __launch_bounds__(256) k_query_closest(DevAccel A, const ct_ray_
     out[i] = o;
   }
 }
+static int sm_count() {
+  static int n_sm = 0;
+  if (n_sm == 0) {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    n_sm = v > 0 ? v : 148;
+  }
+  return n_sm;
+}
+
 cudaError_t ct_launch_queries(const DevAccel &A, const ct_ray_query *q, uint32_t n, void *out, int closest,
                               cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   const uint32_t blocks = (n + 255) / 256 < 65535 ? (n + 255) / 256 : 65535;
-  if (closest) CT_TIMED(CT_K_QUERIES, s, k_query_closest<<<blocks, 256, 0, s>>>(A, q, n, (ct_ray_hit *)out));
-  else CT_TIMED(CT_K_QUERIES, s, k_query_visibility<<<blocks, 256, 0, s>>>(A, q, n, (uint8_t *)out));
+  if (closest) {
+    CT_TIMED(CT_K_QUERIES, s, k_query_closest<<<blocks, 256, 0, s>>>(A, q, n, (ct_ray_hit *)out));
+  } else {
+    // one ray per lane until the resident warps are full, then longer parts
+    const uint32_t resident = (uint32_t)sm_count() * CT_SHADOW_MIN_BLOCKS * CT_SHADOW_WARPS;
+    const uint32_t per_warp = (uint32_t)max((uint64_t)32u, ((uint64_t)n + resident - 1u) / resident);
+    const uint32_t warps = (n + per_warp - 1u) / per_warp;
+    CT_TIMED(CT_K_QUERIES, s,
+             k_query_visibility<<<(warps + CT_SHADOW_WARPS - 1u) / CT_SHADOW_WARPS, 256, 0, s>>>(
+                 A, BatchRays{q, (uint8_t *)out, n, per_warp, 0u, 0u}));
+  }
   return cudaGetLastError();
 }
 
@@ -1849,17 +1934,6 @@ static Workspace make_ws(const CtWorkspace &w) {
   ws.nbr = w.nbr;
   ws.smeta = (uint2 *)w.smeta;
   return ws;
-}
-
-static int sm_count() {
-  static int n_sm = 0;
-  if (n_sm == 0) {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    n_sm = v > 0 ? v : 148;
-  }
-  return n_sm;
 }
 
 // blocks of the persistent walkers: ct_params.walker_blocks, else 8 per SM
