@@ -614,113 +614,158 @@ __device__ __forceinline__ bool hit_better(float t, uint32_t g, const HitRecord 
   return !b.hit || t < b.t || (t == b.t && g < b.gprim);
 }
 
-// Intersection shader semantics (rint.glsl:10-43 with
+// Closest hit.  PRIMARY: intersection shader semantics (rint.glsl:10-43 with
 // is_hit_from_ray_providing_model, primitives.glsl:357-382): object-space ray
-// from the instance's TLAS transform, oriented box test (division), rays may
-// start inside a box, hits reported for t > 0 within [tmin, current tmax].
-struct PrimaryVisitor {
+// from the instance's TLAS transform, oriented box test (division), hits
+// reported for t > 0.  Otherwise ray-query semantics (bounce.glsl:85-119):
+// candidates are tested with is_hit_from_ray (primitives.glsl:412-453):
+// object-space ray from the inverse of INSTANCE.transform, non-oriented box
+// test (multiplication by safeInverse(direction)), hits for t >= 0.  Rays may
+// start inside a box; hits lie within [0, tmax].
+// a walk's object-space ray and the reciprocal direction the box test takes
+struct ObjRay {
+  f3 ro, rd, ird;
+};
+template <bool PRIMARY>
+struct ClosestVisitor {
   const DevAccel &A; const DevGrid &g;
-  f3 ro, rd, inv_rd;  // object space
+  const ObjRay &R;
   f3 radius, inv_radius;
-  float tmin, tmax;
+  float tmax;
   uint32_t inst;
   HitRecord &best;
   uint32_t tests;
   __device__ float stop_t() const { return best.hit ? best.t : tmax; }
   __device__ bool visit(int x, int y, int z, uint32_t prim) {
     f3 c = voxel_center(A, g, x, y, z, prim);
-    BoxHit h = box_test(c, radius, inv_radius, ro, rd, true, true, inv_rd);
-    float t = h.hit ? h.t : -1.0f;
-    if (!(t > 0.f)) return false;
-    float cur = best.hit ? best.t : tmax;
-    if (!(t >= tmin && t <= cur)) return false;
+    BoxHit h = box_test(c, radius, inv_radius, R.ro, R.rd, true, PRIMARY, R.ird);
+    if (!h.hit) return false;
+    const float t = h.t;
+    if (PRIMARY ? !(t > 0.f) : !(t >= 0.f)) return false;
+    if (!(t <= (best.hit ? best.t : tmax))) return false;
     uint32_t gp = g.first_primitive_index + prim;
     if (hit_better(t, gp, best)) { best.hit = true; best.t = t; best.inst = inst; best.prim = prim; best.gprim = gp; }
     return false;
   }
 };
 
-// Ray-query semantics (light.glsl:106-137, bounce.glsl:85-119): candidates
-// are tested with is_hit_from_ray (primitives.glsl:412-453): object-space ray
-// from the inverse of INSTANCE.transform, non-oriented box test
-// (multiplication by safeInverse(direction)).  Visibility: the first hit in
-// (t, primitive) order with t in [0, t_max] decides; it blocks unless it is
-// the light's own voxel.  Closest query: the first such hit is the result.
-// The object-space ray and its reciprocal are asked of `ray` at every box
-// test: a FixedRay, or an ObjRayRef to a ray held elsewhere.
-struct FixedRay {
-  f3 ro, rd;
-  __device__ void operator()(f3 &o, f3 &d) const { o = ro; d = rd; }
-  __device__ f3 inv(f3 d) const { return safe_inverse(d); }
-};
-// a walk's object-space ray and the reciprocal direction the box test takes,
-// held once (in shared memory by the bounce walker) instead of derived again
-// at every box test
-struct ObjRay {
-  f3 ro, rd, ird;
-};
-struct ObjRayRef {
-  const ObjRay &R;
-  __device__ void operator()(f3 &o, f3 &d) const { o = R.ro; d = R.rd; }
-  __device__ f3 inv(f3) const { return R.ird; }
-};
-template <class RayObj>
-struct QueryVisitor {
+// Visibility with ray-query semantics (light.glsl:106-137): the first hit in
+// (t, primitive) order with t in [0, tmax] decides; it blocks unless it is
+// the light's own voxel.
+struct VisibilityVisitor {
   const DevAccel &A; const DevGrid &g;
-  RayObj ray;  // object space
+  f3 ro, rd, ird;  // object space
   f3 radius, inv_radius;
-  bool can_start;
   float tmax;
   uint32_t inst;
-  // visibility mode: decisive key of the target
-  bool visibility;
+  // decisive key of the target
   float target_t; uint32_t target_g; bool has_target; uint32_t target_inst, target_prim;
-  HitRecord &best;  // closest mode result / visibility: blocking hit
+  bool blocked;
   uint32_t tests;
-  __device__ float stop_t() const {
-    if (visibility) return fminf(tmax, target_t);
-    return best.hit ? best.t : tmax;
-  }
+  __device__ float stop_t() const { return fminf(tmax, target_t); }
   __device__ bool visit(int x, int y, int z, uint32_t prim) {
-    if (visibility && has_target && inst == target_inst && prim == target_prim) return false;
-    f3 c = voxel_center(A, g, x, y, z, prim);
-    f3 ro, rd;
-    ray(ro, rd);
-    BoxHit h = box_test(c, radius, inv_radius, ro, rd, can_start, false, ray.inv(rd));
+    if (has_target && inst == target_inst && prim == target_prim) return false;
+    BoxHit h = box_test(voxel_center(A, g, x, y, z, prim), radius, inv_radius, ro, rd, false, false, ird);
     if (!h.hit) return false;
-    float t = h.t;
+    const float t = h.t;
     if (!(t >= 0.f && t <= tmax)) return false;
-    uint32_t gp = g.first_primitive_index + prim;
-    if (visibility) {
-      if (t < target_t || (t == target_t && gp < target_g)) {
-        best.hit = true; best.t = t; best.inst = inst; best.prim = prim; best.gprim = gp;
-        return true;  // blocked
-      }
-      return false;
-    }
-    if (t <= (best.hit ? best.t : tmax) && hit_better(t, gp, best)) {
-      best.hit = true; best.t = t; best.inst = inst; best.prim = prim; best.gprim = gp;
-    }
-    return false;
+    const uint32_t gp = g.first_primitive_index + prim;
+    blocked = t < target_t || (t == target_t && gp < target_g);
+    return blocked;
   }
 };
-
-
 
 __device__ __forceinline__ f3 half_extent_v(const DevAccel &A) { float h = A.extent * 0.5f; return f3{h, h, h}; }
 
-// closest hit of a camera ray (traceRayEXT with the RIS_SELECTION hit group)
-__device__ HitRecord trace_primary(const DevAccel &A, f3 o, f3 d, float tmin, float tmax, uint32_t pixel,
-                                   RayStats &rs) {
+// A closest hit as a resumable walk over every instance in turn, so that a
+// warp can refill lanes whose ray is done.  PRIMARY: a camera ray (traceRayEXT
+// with the RIS_SELECTION hit group); otherwise intersect()'s bounce ray
+// (bounce.glsl:9-125), whose origin compute_ray_origin(origin, direction)
+// moves.  The walk's ray and the object-space one the box tests read lie in
+// memory the caller places (shared memory in the walkers).
+struct ClosestRay {
+  WalkRay &r;
+  ObjRay &obj;
+};
+struct ClosestWalk {
+  uint32_t inst;     // instance being walked
+  WalkState s;
+  HitRecord best;
+};
+// The first instance from w.inst on whose grid the ray overlaps; false when
+// none is left.  `ray(o, d)` gives the world-space ray, which the walk does
+// not keep (the walkers are register bound).
+template <bool PRIMARY, class RayFn>
+__device__ __forceinline__ bool closest_walk_instance(const DevAccel &A, ClosestWalk &w, float tmax, const RayFn &ray,
+                                                      const ClosestRay &R) {
+  for (; w.inst < A.n_grids; w.inst++) {
+    const DevGrid &g = A.grids[w.inst];
+    f3 o, d;
+    ray(o, d);
+    const m4 &m = PRIMARY ? g.world2obj_tlas : g.world2obj_inst;
+    const f3 ro = xyz(mul(m, mk4(PRIMARY ? o : compute_ray_origin(o, d), 1.0f)));
+    const f3 rd = xyz(mul(m, mk4(d, 0.0f)));
+    const f3 ird = safe_inverse(rd);
+    WalkRay r;
+    if (walk_init(A, g, ro, rd, ird, 0.f, w.best.hit ? w.best.t : tmax, r, w.s)) {
+      R.r = r;
+      R.obj.ro = ro;
+      R.obj.rd = rd;
+      R.obj.ird = ird;
+      return true;
+    }
+  }
+  return false;
+}
+// true when the ray is already decided (no instance to walk)
+template <bool PRIMARY, class RayFn>
+__device__ __forceinline__ bool closest_walk_begin(const DevAccel &A, ClosestWalk &w, float tmax, const RayFn &ray,
+                                                   const ClosestRay &R) {
+  w.best = HitRecord{false, 0.f, 0u, 0u, 0u};
+  w.inst = 0;
+  return !closest_walk_instance<PRIMARY>(A, w, tmax, ray, R);
+}
+template <bool PRIMARY, bool COUNT, class RayFn>
+__device__ __forceinline__ int closest_walk_advance(const DevAccel &A, ClosestWalk &w, float tmax, int rounds,
+                                                    int inner, uint32_t pixel, RayStats &rs, const RayFn &ray,
+                                                    const ClosestRay &R) {
+  const f3 radius = half_extent_v(A), inv_radius = safe_inverse(radius);
+  const DevGrid &g = A.grids[w.inst];
+  ClosestVisitor<PRIMARY> v{A, g, R.obj, radius, inv_radius, tmax, w.inst, w.best, 0u};
+  const int st = walk_run<COUNT>(A, g, R.r, w.s, v, rs, rounds, inner);
+  rs.voxel_tests += v.tests;
+  if (st == WALK_LIMIT) ct_latch_error(CT_ERR_ITER_LIMIT, PRIMARY ? 1 : 4, pixel);
+  if (st == WALK_MORE) return WALK_MORE;
+  w.inst++;
+  return closest_walk_instance<PRIMARY>(A, w, tmax, ray, R) ? WALK_MORE : WALK_DONE;
+}
+// the whole walk in place; false: no hit
+template <bool PRIMARY>
+__device__ __forceinline__ bool closest_walk(const DevAccel &A, ClosestWalk &w, f3 origin, f3 dir, float tmax,
+                                             uint32_t pixel, RayStats &rs) {
+  WalkRay r;
+  ObjRay obj;
+  const ClosestRay R{r, obj};
+  const auto ray = [&](f3 &o, f3 &d) { o = origin; d = dir; };
+  if (!closest_walk_begin<PRIMARY>(A, w, tmax, ray, R))
+    while (closest_walk_advance<PRIMARY, true>(A, w, tmax, 1 << 20, CT_WALK_INNER, pixel, rs, ray, R) == WALK_MORE) {
+    }
+  return w.best.hit;
+}
+
+// closest hit of a camera ray in place
+__device__ HitRecord trace_primary(const DevAccel &A, f3 o, f3 d, float tmax, uint32_t pixel, RayStats &rs) {
   HitRecord best = {false, 0.f, 0u, 0u, 0u};
   const f3 radius = half_extent_v(A), inv_radius = safe_inverse(radius);
   for (uint32_t i = 0; i < A.n_grids; i++) {
     const DevGrid &g = A.grids[i];
-    f3 ro = xyz(mul(g.world2obj_tlas, mk4(o, 1.0f)));
-    f3 rd = xyz(mul(g.world2obj_tlas, mk4(d, 0.0f)));
-    const f3 ird = safe_inverse(rd);
-    PrimaryVisitor v{A, g, ro, rd, ird, radius, inv_radius, tmin, tmax, i, best, 0u};
-    if (!walk_traverse(A, g, ro, rd, ird, tmin, best.hit ? best.t : tmax, v, rs)) ct_latch_error(CT_ERR_ITER_LIMIT, 1, pixel);
+    ObjRay R;
+    R.ro = xyz(mul(g.world2obj_tlas, mk4(o, 1.0f)));
+    R.rd = xyz(mul(g.world2obj_tlas, mk4(d, 0.0f)));
+    R.ird = safe_inverse(R.rd);
+    ClosestVisitor<true> v{A, g, R, radius, inv_radius, tmax, i, best, 0u};
+    if (!walk_traverse(A, g, R.ro, R.rd, R.ird, 0.f, best.hit ? best.t : tmax, v, rs))
+      ct_latch_error(CT_ERR_ITER_LIMIT, 1, pixel);
     rs.voxel_tests += v.tests;
   }
   return best;
@@ -751,13 +796,13 @@ __device__ bool vertex_visible(const DevAccel &A, f3 o, f3 d, float distance, ui
     const DevGrid &g = A.grids[i];
     f3 ro = xyz(mul(g.world2obj_inst, mk4(o, 1.0f)));
     f3 rd = xyz(mul(g.world2obj_inst, mk4(d, 0.0f)));
-    HitRecord blk = {false, 0.f, 0u, 0u, 0u};
-    QueryVisitor<FixedRay> v{A, g, FixedRay{ro, rd}, radius, inv_radius, false, distance, i, true, target_t,
-                             target_g, has_target, t_inst, t_prim, blk, 0u};
+    const f3 ird = safe_inverse(rd);
+    VisibilityVisitor v{A, g, ro, rd, ird, radius, inv_radius, distance, i, target_t, target_g, has_target, t_inst,
+                        t_prim, false, 0u};
     float tlim = fminf(distance, target_t);
-    if (!walk_traverse(A, g, ro, rd, safe_inverse(rd), 0.f, tlim, v, rs)) ct_latch_error(CT_ERR_ITER_LIMIT, 2, pixel);
+    if (!walk_traverse(A, g, ro, rd, ird, 0.f, tlim, v, rs)) ct_latch_error(CT_ERR_ITER_LIMIT, 2, pixel);
     rs.voxel_tests += v.tests;
-    if (blk.hit) return false;
+    if (v.blocked) return false;
   }
   return true;
 }

@@ -708,85 +708,12 @@ __device__ void path_shade(const FrameView &F, const DevAccel &A, const PtParams
   }
 }
 
-// Closest hit of a bounce ray as a resumable walk (the walker refills lanes
-// whose ray is done): intersect()'s candidate test and commit rule
-// (QueryVisitor, closest mode) over every instance in turn.  The walk's ray
-// and the object-space one the box tests read lie in memory the caller places
-// (shared memory in the bounce walker).
-struct ClosestRay {
-  WalkRay &r;
-  ObjRay &obj;
-};
-struct ClosestWalk {
-  uint32_t inst;     // instance being walked
-  WalkState s;
-  HitRecord best;
-};
-// The first instance from w.inst on whose grid the ray overlaps; false when
-// none is left.  `ray(o, d)` gives the world-space bounce ray, which the walk
-// does not keep (the walkers are register bound).
-template <class RayFn>
-__device__ __forceinline__ bool closest_walk_instance(const DevAccel &A, ClosestWalk &w, const RayFn &ray,
-                                                      const ClosestRay &R) {
-  for (; w.inst < A.n_grids; w.inst++) {
-    const DevGrid &g = A.grids[w.inst];
-    f3 o, d;
-    ray(o, d);
-    const f3 key_o = compute_ray_origin(o, d);
-    const f3 ro = xyz(mul(g.world2obj_inst, mk4(key_o, 1.0f)));
-    const f3 rd = xyz(mul(g.world2obj_inst, mk4(d, 0.0f)));
-    const f3 ird = safe_inverse(rd);
-    WalkRay r;
-    if (walk_init(A, g, ro, rd, ird, 0.f, w.best.hit ? w.best.t : 1e9f, r, w.s)) {
-      R.r = r;
-      R.obj.ro = ro;
-      R.obj.rd = rd;
-      R.obj.ird = ird;
-      return true;
-    }
-  }
-  return false;
-}
-// true when the ray is already decided (no instance to walk)
-__device__ __forceinline__ bool closest_walk_begin(const DevAccel &A, ClosestWalk &w, f3 origin, f3 dir,
-                                                   const ClosestRay &R) {
-  w.best = HitRecord{false, 0.f, 0u, 0u, 0u};
-  w.inst = 0;
-  return !closest_walk_instance(A, w, [&](f3 &o, f3 &d) { o = origin; d = dir; }, R);
-}
-template <bool COUNT, class RayFn>
-__device__ __forceinline__ int closest_walk_advance(const DevAccel &A, ClosestWalk &w, int rounds, int inner,
-                                                    uint32_t pixel, RayStats &rs, const RayFn &ray, const ClosestRay &R) {
-  const f3 radius = half_extent_v(A), inv_radius = safe_inverse(radius);
-  const DevGrid &g = A.grids[w.inst];
-  QueryVisitor<ObjRayRef> v{A, g, ObjRayRef{R.obj}, radius, inv_radius, true, 1e9f, w.inst, false, INFINITY,
-                            0xFFFFFFFFu, false, 0u, 0u, w.best, 0u};
-  const int st = walk_run<COUNT>(A, g, R.r, w.s, v, rs, rounds, inner);
-  rs.voxel_tests += v.tests;
-  if (st == WALK_LIMIT) ct_latch_error(CT_ERR_ITER_LIMIT, 4, pixel);
-  if (st == WALK_MORE) return WALK_MORE;
-  w.inst++;
-  return closest_walk_instance(A, w, ray, R) ? WALK_MORE : WALK_DONE;
-}
-// the whole walk in place; false: no hit
-__device__ __forceinline__ bool closest_walk(const DevAccel &A, ClosestWalk &w, f3 origin, f3 dir, uint32_t pixel,
-                                             RayStats &rs) {
-  WalkRay r;
-  ObjRay obj;
-  const ClosestRay R{r, obj};
-  const auto ray = [&](f3 &o, f3 &d) { o = origin; d = dir; };
-  if (!closest_walk_begin(A, w, origin, dir, R))
-    while (closest_walk_advance<true>(A, w, 1 << 20, CT_WALK_INNER, pixel, rs, ray, R) == WALK_MORE) {
-    }
-  return w.best.hit;
-}
-
 // intersect() (bounce.glsl:9-125) run to the end in place
 __device__ Isect intersect_closest(const FrameView &F, const DevAccel &A, f3 origin, f3 dir, uint32_t pixel,
                                    RayStats &rs) {
   ClosestWalk w;
   rs.bounce++;
-  if (!closest_walk(A, w, origin, dir, pixel, rs)) return isect_empty();
+  if (!closest_walk<false>(A, w, origin, dir, CT_MAX_DISTANCE, pixel, rs)) return isect_empty();
   rs.bounce_hits++;
   return bounce_vertex(F, A, origin, dir, w.best.inst, w.best.prim, w.best.gprim);
 }

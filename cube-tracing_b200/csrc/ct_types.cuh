@@ -11,6 +11,7 @@
 #define CT_MASK_WORDS 16u  // occupancy words per NEAR brick
 #define CT_DDA_MAX_STEPS (1 << 16)
 #define CT_SAMPLER_MAX_TRIES 4096
+#define CT_MAX_DISTANCE 1e9f  // MAX_DISTANCE: range of camera and bounce rays
 
 // ---------------------------------------------------------------------------
 // acceleration structure (built by ct_build_accel)
