@@ -58,7 +58,7 @@ __device__ __forceinline__ void camera_ray_jittered(const Desc &D, const Camera 
 __device__ __forceinline__ bool closest_voxel(const DevAccel &A, f3 o, f3 d, uint32_t pixel, RayStats &rs,
                                               uint32_t &gprim, f3 &pos, f3 &nrm) {
   ClosestWalk w;
-  if (!closest_walk(A, w, o, d, pixel, rs)) return false;
+  if (!closest_walk<false>(A, w, o, d, CT_MAX_DISTANCE, pixel, rs)) return false;
   gprim = w.best.gprim;
   bounce_geometry(A, o, d, w.best.inst, w.best.prim, w.best.gprim, pos, nrm);
   return true;
