@@ -29,19 +29,31 @@ struct RayStats {
 };
 
 // ---------------------------------------------------------------------------
-// per-frame view of the caller's buffers (WORLD / RESTIR / Status tables)
+// per-frame view of the caller's buffers (WORLD / RESTIR / Status tables).
+// From `instances` on the members are WORLD's and RESTIR's addresses and then
+// Status's words from frame_number to max_depth, in those tables' order, which
+// load_frame_view copies word by word.
 struct FrameView {
+  float4 *swapchain;
+  const float4 *previous_swapchain;
+  float4 *taa_frame;
   uint32_t W, H;
+  ct_light_config light_config;
+  uint32_t _pad0;
+  // WORLD
   const ct_instance *instances;
   const ct_instance *instances_prev;
   const ct_primitive *primitives;
+  const ct_primitive *primitives_prev;
   const ct_aabb *aabbs;
+  const ct_aabb *aabbs_prev;
   const uint32_t *remap_p;    // WORLD.remapped_primitive_address (CT_REMAP_BIT)
   const uint32_t *remap_l;    // WORLD.remapped_cube_light_address
   const ct_material *materials;
   const ct_light *point_lights;
   const ct_light *cube_lights;
   const ct_light *env_lights;
+  // RESTIR
   ct_reservoir *prev_reservoir;
   ct_reservoir *int_reservoir;
   ct_reservoir *cur_reservoir;
@@ -51,13 +63,15 @@ struct FrameView {
   ct_path_reservoir *out_path_reservoir;
   ct_path_reservoir *temporal_path_reservoir;
   float *indirect_color;
-  float4 *swapchain;
-  const float4 *previous_swapchain;
-  float4 *taa_frame;
-  ct_light_config light_config;
-  uint32_t frame_number, is_active, obj_count, is_afternoon, max_depth;
+  // Status
+  uint32_t frame_number, _pad1;
+  uint64_t num_accumulated_frames;
+  uint32_t pixel[2];
+  uint32_t is_active, _pad2;
+  uint64_t light_config_address;
+  uint32_t obj_count;
   float time;
-  const ct_camera_view *camera;
+  uint32_t is_afternoon, max_depth;
 };
 
 __device__ __forceinline__ f3 ld3(const float *p) { return f3{p[0], p[1], p[2]}; }

@@ -16,51 +16,114 @@
 // per-block frame constants
 struct BlockConsts {
   FrameView F;
-  m4 inv_view, inv_proj, inv_prev_mvp;
+  m4 inv_view, inv_proj;
 };
+// 8-byte words of load_frame_view: WORLD, RESTIR, Status from frame_number to
+// max_depth, and the camera's inv_view and inv_proj go one behind the other
+// to FrameView::instances onwards
+constexpr uint32_t kViewWorld = sizeof(ct_world) / 8, kViewRestir = kViewWorld + sizeof(ct_restir) / 8;
+constexpr uint32_t kStatusFirst = offsetof(ct_status_block, frame_number);
+constexpr uint32_t kViewStatus =
+    kViewRestir + (offsetof(ct_status_block, max_depth) + 4 - kStatusFirst) / 8;
+constexpr uint32_t kViewWords = kViewStatus + 2 * sizeof(m4) / 8;
+static_assert(kViewWords < 64 && kStatusFirst % 8 == 0 && sizeof(ct_light_config) / 4 <= 32, "threads of load_frame_view");
+#define CT_VIEW_AT(member, status_member)                                       \
+  (offsetof(FrameView, member) - offsetof(FrameView, instances) == 8 * kViewRestir + \
+                                                                       offsetof(ct_status_block, status_member) - kStatusFirst)
+static_assert(offsetof(FrameView, prev_reservoir) - offsetof(FrameView, instances) == sizeof(ct_world) &&
+                  CT_VIEW_AT(frame_number, frame_number) && CT_VIEW_AT(is_active, is_active) &&
+                  CT_VIEW_AT(light_config_address, light_config_address) && CT_VIEW_AT(obj_count, obj_count) &&
+                  CT_VIEW_AT(time, time) && CT_VIEW_AT(is_afternoon, is_afternoon) &&
+                  CT_VIEW_AT(max_depth, max_depth) && sizeof(FrameView) == offsetof(FrameView, max_depth) + 4 &&
+                  offsetof(BlockConsts, inv_view) == sizeof(FrameView) &&
+                  offsetof(ct_camera_view, inv_proj) == offsetof(ct_camera_view, inv_view) + sizeof(m4),
+              "load_frame_view copies the tables in their own layouts");
 
-__device__ void load_frame_view(const ct_push_constant &pc, BlockConsts &B) {
+__device__ __forceinline__ uint32_t block_thread() { return threadIdx.y * blockDim.x + threadIdx.x; }
+
+// Every thread of the block calls this, then the block synchronises: a word
+// per thread of the first two warps (and of the third for LIGHTS, the light
+// configuration), so that a block waits for two dependent loads.  One thread
+// reading all of it, with the two 4x4 inverses that only the primary rays
+// need, held each block for thousands of cycles: a fifth of the stalls of the
+// primary rays and a tenth of RIS's (1080p terrain frame 11.5 -> 10.7 ms).
+template <bool LIGHTS = true>
+__device__ __forceinline__ void load_frame_view(const ct_push_constant &pc, BlockConsts &B) {
   FrameView &F = B.F;
-  const ct_world *w = (const ct_world *)(uintptr_t)pc.world_buffer;
-  const ct_restir *r = (const ct_restir *)(uintptr_t)pc.restir_buffer;
-  const ct_status_block *s = (const ct_status_block *)(uintptr_t)pc.status_buffer;
+  const uint32_t t = block_thread();
+  if (t < kViewWords) {
+    const uint64_t src = t < kViewWorld    ? pc.world_buffer + 8u * t
+                         : t < kViewRestir ? pc.restir_buffer + 8u * (t - kViewWorld)
+                         : t < kViewStatus ? pc.status_buffer + kStatusFirst + 8u * (t - kViewRestir)
+                                           : pc.camera_buffer + offsetof(ct_camera_view, inv_view) +
+                                                 8u * (t - kViewStatus);
+    *((uint64_t *)&F.instances + t) = *(const uint64_t *)(uintptr_t)src;
+  } else if (t == kViewWords) {
+    F.W = pc.size[0];
+    F.H = pc.size[1];
+    F.swapchain = (float4 *)pc.swapchain;
+    F.previous_swapchain = (const float4 *)pc.previous_swapchain;
+    F.taa_frame = (float4 *)pc.taa_frame;
+  } else if (LIGHTS && t >= 64u && t < 64u + sizeof(ct_light_config) / 4u) {
+    const ct_status_block *s = (const ct_status_block *)(uintptr_t)pc.status_buffer;
+    ((uint32_t *)&F.light_config)[t - 64u] = ((const uint32_t *)(uintptr_t)s->light_config_address)[t - 64u];
+  }
+}
+
+// ct_inverse by 16 lanes of a warp, element k = lane % 16 (column k / 4, row k
+// % 4): the products of each cofactor in ct_inverse's order, term by term (3
+// indices of 4 bits, then the sign).
+__device__ const uint16_t kCofactor[16][6] = {
+    {0x0fa5, 0x1eb5, 0x1f69, 0x0e79, 0x0b6d, 0x1a7d},
+    {0x1fa1, 0x0eb1, 0x0f29, 0x1e39, 0x1b2d, 0x0a3d},
+    {0x0f61, 0x1e71, 0x1f25, 0x0e35, 0x072d, 0x163d},
+    {0x1b61, 0x0a71, 0x0b25, 0x1a35, 0x1729, 0x0639},
+    {0x1fa4, 0x0eb4, 0x0f68, 0x1e78, 0x1b6c, 0x0a7c},
+    {0x0fa0, 0x1eb0, 0x1f28, 0x0e38, 0x0b2c, 0x1a3c},
+    {0x1f60, 0x0e70, 0x0f24, 0x1e34, 0x172c, 0x063c},
+    {0x0b60, 0x1a70, 0x1b24, 0x0a34, 0x0728, 0x1638},
+    {0x0f94, 0x1db4, 0x1f58, 0x0d78, 0x0b5c, 0x197c},
+    {0x1f90, 0x0db0, 0x0f18, 0x1d38, 0x1b1c, 0x093c},
+    {0x0f50, 0x1d70, 0x1f14, 0x0d34, 0x071c, 0x153c},
+    {0x1b50, 0x0970, 0x0b14, 0x1934, 0x1718, 0x0538},
+    {0x1e94, 0x0da4, 0x0e58, 0x1d68, 0x1a5c, 0x096c},
+    {0x0e90, 0x1da0, 0x1e18, 0x0d28, 0x0a1c, 0x192c},
+    {0x1e50, 0x0d60, 0x0e14, 0x1d24, 0x161c, 0x052c},
+    {0x0a50, 0x1960, 0x1a14, 0x0924, 0x0618, 0x1528}};
+__device__ __forceinline__ float inverse_element(const float *m, uint32_t lane) {
+  const uint32_t k = lane & 15u;
+  float inv = 0.f;
+#pragma unroll
+  for (int j = 0; j < 6; j++) {
+    const uint32_t t = __ldg(&kCofactor[k][j]);
+    const float a = m[t & 15u];
+    const float p = ((t >> 12) ? -a : a) * m[(t >> 4) & 15u] * m[(t >> 8) & 15u];
+    inv = j == 0 ? p : inv + p;
+  }
+  float det = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const float p = m[j] * __shfl_sync(0xFFFFFFFFu, inv, 4 * j, 16);
+    det = j == 0 ? p : det + p;
+  }
+  return inv / det;
+}
+// inverse(prev_inv_proj) * inverse(prev_inv_view) (motion_vectors.glsl:78), by
+// the block's fourth warp
+__device__ __forceinline__ void load_inv_prev_mvp(const ct_push_constant &pc, m4 &out) {
+  __shared__ float m[32], inv[32];
+  if (block_thread() >> 5 != 3u) return;
+  const uint32_t lane = block_thread() & 31u;
   const ct_camera_view *c = (const ct_camera_view *)(uintptr_t)pc.camera_buffer;
-  F.W = pc.size[0];
-  F.H = pc.size[1];
-  F.instances = (const ct_instance *)(uintptr_t)w->instance_address;
-  F.instances_prev = (const ct_instance *)(uintptr_t)w->instance_address_prev;
-  F.primitives = (const ct_primitive *)(uintptr_t)w->primitive_address;
-  F.aabbs = (const ct_aabb *)(uintptr_t)w->aabb_address;
-  F.remap_p = (const uint32_t *)(uintptr_t)w->remapped_primitive_address;
-  F.remap_l = (const uint32_t *)(uintptr_t)w->remapped_cube_light_address;
-  F.materials = (const ct_material *)(uintptr_t)w->material_address;
-  F.point_lights = (const ct_light *)(uintptr_t)w->point_light_address;
-  F.cube_lights = (const ct_light *)(uintptr_t)w->cube_light_address;
-  F.env_lights = (const ct_light *)(uintptr_t)w->env_light_address;
-  F.prev_reservoir = (ct_reservoir *)(uintptr_t)r->previous_reservoir_address;
-  F.int_reservoir = (ct_reservoir *)(uintptr_t)r->intermediate_reservoir_address;
-  F.cur_reservoir = (ct_reservoir *)(uintptr_t)r->reservoir_address;
-  F.prev_di = (ct_di_info *)(uintptr_t)r->previous_di_address;
-  F.di = (ct_di_info *)(uintptr_t)r->di_address;
-  F.velocity = (ct_velocity *)(uintptr_t)r->velocity_address;
-  F.out_path_reservoir = (ct_path_reservoir *)(uintptr_t)r->output_path_reservoir_address;
-  F.temporal_path_reservoir = (ct_path_reservoir *)(uintptr_t)r->temporal_path_reservoir_address;
-  F.indirect_color = (float *)(uintptr_t)r->indirect_color_address;
-  F.swapchain = (float4 *)pc.swapchain;
-  F.previous_swapchain = (const float4 *)pc.previous_swapchain;
-  F.taa_frame = (float4 *)pc.taa_frame;
-  F.frame_number = s->frame_number;
-  F.is_active = s->is_active;
-  F.obj_count = s->obj_count;
-  F.is_afternoon = s->is_afternoon;
-  F.max_depth = s->max_depth;
-  F.time = s->time;
-  F.light_config = *(const ct_light_config *)(uintptr_t)s->light_config_address;
-  F.camera = c;
-  B.inv_view = load_m4(c->inv_view);
-  B.inv_proj = load_m4(c->inv_proj);
-  // inverse(prev_inv_proj) * inverse(prev_inv_view) (motion_vectors.glsl:78)
-  B.inv_prev_mvp = mul(ct_inverse(load_m4(c->prev_inv_proj)), ct_inverse(load_m4(c->prev_inv_view)));
+  m[lane] = lane < 16u ? c->prev_inv_proj[lane] : c->prev_inv_view[lane - 16u];
+  __syncwarp();
+  const float e = inverse_element(m + (lane & 16u), lane);
+  inv[lane] = e;
+  __syncwarp();
+  if (lane < 16u) {
+    const float *a = inv + (lane & 3u), *b = inv + 16u + (lane & 12u);
+    ((float *)&out)[lane] = a[0] * b[0] + a[4] * b[1] + a[8] * b[2] + a[12] * b[3];
+  }
 }
 
 // get_ray_from_current_pixel (rgen.glsl:18-42), no jitter
@@ -107,7 +170,9 @@ __device__ __forceinline__ void pixel_of(uint32_t &x, uint32_t &y) {
 #endif
 __global__ void __launch_bounds__(128, CT_PRIMARY_MIN_BLOCKS) k_trace_primary(ct_push_constant pc, DevAccel A, ct_params P) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0 && threadIdx.y == 0) load_frame_view(pc, B);
+  __shared__ m4 inv_prev_mvp;
+  load_frame_view(pc, B);
+  load_inv_prev_mvp(pc, inv_prev_mvp);
   __syncthreads();
   const FrameView &F = B.F;
   uint32_t x, y;
@@ -154,7 +219,7 @@ __global__ void __launch_bounds__(128, CT_PRIMARY_MIN_BLOCKS) k_trace_primary(ct
       m4 obj2world = load_m4(F.instances[h.inst].transform);
       m4 prev_model = load_m4(F.instances_prev[h.inst].transform);
       m4 geometry_T = mul(prev_model, ct_inverse(obj2world));
-      f4 prev_S = mul(mul(B.inv_prev_mvp, geometry_T), mk4(world_pos, 1.0f));
+      f4 prev_S = mul(mul(inv_prev_mvp, geometry_T), mk4(world_pos, 1.0f));
       f2 xi1 = f2{prev_S.x, prev_S.y} / prev_S.w;
       xi1 = 0.5f * xi1 + 0.5f;
       f2 xi = f2{(float)x, (float)y} + 0.5f;
@@ -417,16 +482,12 @@ template <bool BRDF>
 __global__ void __launch_bounds__(128, BRDF ? 1 : CT_GEN0_MIN_BLOCKS) k_di_gen0(ct_push_constant pc, ct_params P,
                                                                           Workspace ws, DevAccel A) {
   __shared__ BlockConsts B;
-  __shared__ int other_variant;
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    // the flag first: the instantiation that does not run returns before
-    // building the frame view
-    const ct_status_block *st = (const ct_status_block *)(uintptr_t)pc.status_buffer;
-    other_variant = ((st->is_active & CT_RIS_BRDF_BIT) != 0) != BRDF;
-    if (!other_variant) load_frame_view(pc, B);
-  }
+  // the flag first: the instantiation that does not run returns before
+  // building the frame view
+  const ct_status_block *st = (const ct_status_block *)(uintptr_t)pc.status_buffer;
+  if (((st->is_active & CT_RIS_BRDF_BIT) != 0) != BRDF) return;  // the same for the whole block
+  load_frame_view(pc, B);
   __syncthreads();
-  if (other_variant) return;  // the same for the whole block
   const FrameView &F = B.F;
   uint32_t x, y;
   pixel_of(x, y);
@@ -484,7 +545,7 @@ __global__ void __launch_bounds__(128, BRDF ? 1 : CT_GEN0_MIN_BLOCKS) k_di_gen0(
 // k_trace_prev.
 __global__ void __launch_bounds__(128) k_di_gen1(ct_push_constant pc, ct_params P, Workspace ws) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0 && threadIdx.y == 0) load_frame_view(pc, B);
+  load_frame_view(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   uint32_t x, y;
@@ -555,7 +616,7 @@ __global__ void __launch_bounds__(128) k_di_gen1(ct_push_constant pc, ct_params 
 #endif
 __global__ void __launch_bounds__(128, CT_DI_RESOLVE0_MIN_BLOCKS) k_di_resolve0(ct_push_constant pc, ct_params P, Workspace ws) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0 && threadIdx.y == 0) load_frame_view(pc, B);
+  load_frame_view(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   uint32_t x, y;
@@ -625,7 +686,7 @@ __device__ uint32_t spatial_select(const FrameView &F, const ct_params &P, float
 
 __global__ void __launch_bounds__(128) k_spatial_select(ct_push_constant pc, ct_params P, Workspace ws, int src_sel) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0 && threadIdx.y == 0) load_frame_view(pc, B);
+  load_frame_view<false>(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   const ct_reservoir *src = src_sel ? F.cur_reservoir : F.int_reservoir;
@@ -670,7 +731,7 @@ struct VisCapture {
 __global__ void __launch_bounds__(CT_SPATIAL_SAMPLE_THREADS, CT_SPATIAL_SAMPLE_MIN_BLOCKS) k_spatial_sample(ct_push_constant pc, ct_params P, Workspace ws, int src_sel,
                                                        uint32_t R) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0) load_frame_view(pc, B);
+  load_frame_view<false>(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   const ct_reservoir *src = src_sel ? F.cur_reservoir : F.int_reservoir;
@@ -728,7 +789,7 @@ __global__ void __launch_bounds__(CT_SPATIAL_SAMPLE_THREADS, CT_SPATIAL_SAMPLE_M
 __global__ void __launch_bounds__(128) k_spatial_resolve(ct_push_constant pc, ct_params P, Workspace ws, int src_sel,
                                                         int final_pass, int dst_sel) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0 && threadIdx.y == 0) load_frame_view(pc, B);
+  load_frame_view<false>(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   const ct_reservoir *src = src_sel ? F.cur_reservoir : F.int_reservoir;
@@ -1066,10 +1127,7 @@ __global__ void __launch_bounds__(128) k_trace_prev(ct_push_constant pc, DevAcce
 // reference dispatch.
 __global__ void __launch_bounds__(64) k_taa(ct_push_constant pc, ct_params P) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    // only the frame view is needed
-    load_frame_view(pc, B);
-  }
+  load_frame_view<false>(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   uint32_t x, y;
@@ -1304,7 +1362,7 @@ static_assert(kPathCols * 16 <= CT_PT_STATE_BYTES, "PathState outgrew its worksp
 // first bounce ray goes to queue 0
 __global__ void __launch_bounds__(128) k_pt_start(ct_push_constant pc, DevAccel A, ct_params P, PtWork w) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0 && threadIdx.y == 0) load_frame_view(pc, B);
+  load_frame_view(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   uint32_t x, y;
@@ -1415,7 +1473,7 @@ __global__ void __launch_bounds__(256, CT_EXTEND_MIN_BLOCKS) k_pt_extend(DevAcce
 __global__ void __launch_bounds__(256, CT_SHADE_MIN_BLOCKS) k_pt_shade(ct_push_constant pc, DevAccel A, ct_params P, Workspace ws,
                                                   PtWork w, int qi) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0) load_frame_view(pc, B);
+  load_frame_view(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   const PtParams pp = pt_params(F, P, A);
@@ -1475,7 +1533,7 @@ __global__ void __launch_bounds__(256, CT_SHADE_MIN_BLOCKS) k_pt_shade(ct_push_c
 __global__ void __launch_bounds__(128) k_pt_finish(ct_push_constant pc, DevAccel A, ct_params P, Workspace ws,
                                                    PtWork w, int qi) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0) load_frame_view(pc, B);
+  load_frame_view(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   const PtParams pp = pt_params(F, P, A);
@@ -1608,7 +1666,7 @@ __device__ __forceinline__ bool needs_replay(const PathRes &src) {
 // marks the others as not asked for.
 __global__ void __launch_bounds__(128) k_pt_replay_jobs(ct_push_constant pc, PtWork w) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0 && threadIdx.y == 0) load_frame_view(pc, B);
+  load_frame_view(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   uint32_t x, y;
@@ -1638,7 +1696,7 @@ __global__ void __launch_bounds__(128) k_pt_replay_jobs(ct_push_constant pc, PtW
 // on one lane of a pixel kernel.
 __global__ void __launch_bounds__(128) k_pt_replay(ct_push_constant pc, DevAccel A, ct_params P, PtWork w) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0 && threadIdx.y == 0) load_frame_view(pc, B);
+  load_frame_view(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   const uint32_t n = w.count[4];
@@ -1710,7 +1768,7 @@ template <int PHASE, bool HYBRID>
 __global__ void __launch_bounds__(128, PHASE == 0 ? CT_PT_TEMPORAL0_MIN_BLOCKS : CT_PT_TEMPORAL1_MIN_BLOCKS) k_pt_temporal(ct_push_constant pc, DevAccel A, ct_params P, Workspace ws,
                                                      PtWork w) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0 && threadIdx.y == 0) load_frame_view(pc, B);
+  load_frame_view(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   uint32_t x, y;
@@ -1772,7 +1830,7 @@ __global__ void __launch_bounds__(128, PHASE == 0 ? CT_PT_TEMPORAL0_MIN_BLOCKS :
 template <bool HYBRID>
 __global__ void __launch_bounds__(128, CT_PT_SPATIAL_MIN_BLOCKS) k_pt_spatial(ct_push_constant pc, DevAccel A, ct_params P) {
   __shared__ BlockConsts B;
-  if (threadIdx.x == 0 && threadIdx.y == 0) load_frame_view(pc, B);
+  load_frame_view(pc, B);
   __syncthreads();
   const FrameView &F = B.F;
   uint32_t x, y;
