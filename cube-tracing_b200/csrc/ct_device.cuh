@@ -1226,7 +1226,7 @@ struct LightSample {
 // sample_lights: chooses a point on `l` as seen from the shading point, its
 // pdf update, and (when `visibility`) asks the visibility provider `vp` about
 // the shadow ray; `slot` names the call site so that a later pass can find
-// the answer (see VisEmit / VisRead).
+// the answer (see VisCapture / VisRead).
 template <class VP>
 __device__ LightSample sample_lights(const FrameView &F, f3 P, f3 n, uint32_t hit_inst, uint32_t hit_prim, Light l,
                                      float &pdf, uint32_t &seed, bool calc_pdf, bool visibility, uint32_t pixel,
@@ -1408,7 +1408,7 @@ __device__ f3 reservoir_get_radiance(const FrameView &F, const Reservoir &r, f3 
 
 // ---------------------------------------------------------------------------
 // Visibility providers.  The shading passes run twice over a pixel: the
-// generating pass records every shadow ray the shader would trace (VisEmit,
+// generating pass records every shadow ray the shader would trace (VisCapture,
 // into a compacted queue traced by k_trace_shadow), the resolving pass
 // replays the same deterministic light samples and reads the answers back
 // (VisRead).  A call site traces at most one ray and owns one fixed slot.
@@ -1424,30 +1424,6 @@ struct RayQueue {
 
 struct VisNever {  // for samplers called with visibility off
   __device__ bool operator()(f3, f3, float, uint32_t, uint32_t, bool, uint32_t) { return true; }
-};
-
-// Generating passes run their shadow-ray call sites twice: VisCount counts
-// the rays a thread will emit, block_reserve (a block-wide scan, one atomic
-// per block) turns the counts into queue positions, and VisEmit writes the
-// rays there.  Every thread of the block must reach block_reserve.
-struct VisCount {
-  uint32_t n;
-  __device__ bool operator()(f3, f3, float, uint32_t, uint32_t, bool, uint32_t) { n++; return true; }
-};
-
-struct VisEmit {
-  RayQueue q;
-  uint32_t base;  // pixel * CT_VIS_SLOTS
-  uint32_t pixel;
-  uint32_t next;  // queue position of this thread's next ray
-  __device__ bool operator()(f3 o, f3 d, float dist, uint32_t inst, uint32_t prim, bool check, uint32_t slot) {
-    const uint32_t i = next++;
-    if (i >= q.capacity) { ct_latch_error(CT_ERR_CAPACITY, 5, pixel); return true; }
-    q.a[i] = make_float4(o.x, o.y, o.z, dist);
-    q.b[i] = make_float4(d.x, d.y, d.z, __uint_as_float(base + slot));
-    q.c[i] = make_uint2(inst | (check ? 0x80000000u : 0u), prim);
-    return true;
-  }
 };
 
 // Exclusive prefix of `n` over the block plus one atomicAdd on `counter`;

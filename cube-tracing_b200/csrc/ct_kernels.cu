@@ -466,6 +466,32 @@ __device__ void temporal_prev_sample_ray(const FrameView &F, const ct_params &P,
   if (prev.Y != 0xFFFFFFFFu) reservoir_get_radiance(F, prev, ray_dir, S, mat, pixel, vp, 1u);
 }
 
+// Captures the one shadow ray a call site would trace.
+struct VisCapture {
+  bool traced;
+  f3 o, d;
+  float dist;
+  uint32_t inst, prim;
+  bool check;
+  __device__ bool operator()(f3 o_, f3 d_, float dist_, uint32_t i_, uint32_t p_, bool c_, uint32_t) {
+    traced = true; o = o_; d = d_; dist = dist_; inst = i_; prim = p_; check = c_;
+    return true;
+  }
+  __device__ void store(const RayQueue &q, uint32_t i, uint32_t slot) const {
+    q.a[i] = make_float4(o.x, o.y, o.z, dist);
+    q.b[i] = make_float4(d.x, d.y, d.z, __uint_as_float(slot));
+    q.c[i] = make_uint2(inst | (check ? 0x80000000u : 0u), prim);
+  }
+};
+
+// a captured ray into queue position i, for slot `site` of the pixel
+__device__ __forceinline__ void emit_ray(const RayQueue &q, const VisCapture &ray, uint32_t i, uint32_t pixel,
+                                         uint32_t site) {
+  if (!ray.traced) return;
+  if (i >= q.capacity) ct_latch_error(CT_ERR_CAPACITY, 5, pixel);
+  else ray.store(q, i, pixel * CT_VIS_SLOTS + site);
+}
+
 // stage 0, generate: RIS, then ask for the RIS visibility ray (slot 0) and
 // the previous sample's ray (slot 1).  Writes the pre-visibility reservoir to
 // RESTIR.intermediate_reservoir and the seed/confidence to the DI record.
@@ -522,16 +548,18 @@ __global__ void __launch_bounds__(128, BRDF ? 1 : CT_GEN0_MIN_BLOCKS) k_di_gen0(
       dref.confidence = T.confidence;
     }
   }
-  auto rays = [&](auto &vp) {
-    if (!active) return;
+  // both rays captured, then queued (asking for them twice, once to count and
+  // once to write, replayed two light samples)
+  VisCapture ray0, ray1;
+  ray0.traced = ray1.traced = false;
+  if (active) {
     Reservoir tmp = res;
-    if (ris_vis) ris_visibility(F, tmp, S, screen_pos, vp);
-    if (T.prev.W_y > 0.0f) temporal_prev_sample_ray(F, P, d, S, mat, res, T.prev, screen_pos, vp);
-  };
-  VisCount cnt{0};
-  rays(cnt);
-  VisEmit emit{ws.q, screen_pos * CT_VIS_SLOTS, screen_pos, block_reserve(cnt.n, ws.q.count)};
-  rays(emit);
+    if (ris_vis) ris_visibility(F, tmp, S, screen_pos, ray0);
+    if (T.prev.W_y > 0.0f) temporal_prev_sample_ray(F, P, d, S, mat, res, T.prev, screen_pos, ray1);
+  }
+  const uint32_t pos = block_reserve((ray0.traced ? 1u : 0u) + (ray1.traced ? 1u : 0u), ws.q.count);
+  emit_ray(ws.q, ray0, pos, screen_pos, 0u);
+  emit_ray(ws.q, ray1, pos + (ray0.traced ? 1u : 0u), screen_pos, 1u);
   count_rays(P, rs);
 }
 
@@ -584,26 +612,17 @@ __global__ void __launch_bounds__(128) k_di_gen1(ct_push_constant pc, ct_params 
       }
     }
   }
-  auto rays = [&](auto &vp, RayStats &st) {
-    if (!active) return;
+  VisCapture ray;
+  ray.traced = false;
+  if (active) {
     Reservoir r2 = res;
     uint32_t s2 = seed;
-    temporal_reuse(F, P, d, S, mat, r2, T.prev, T.prev_index, s2, screen_pos, vp, true, st);
-  };
-  if (F.is_active & CT_REMAP_BIT) {  // the same for every thread
-    // rays against the previous scene: their own count, walked by k_trace_prev
-    VisCount cnt{0};
-    RayStats dummy = {};
-    rays(cnt, dummy);
-    VisEmit emit{ws.q, screen_pos * CT_VIS_SLOTS, screen_pos, block_reserve(cnt.n, ws.q.count + CT_PREV_COUNT)};
-    rays(emit, rs);
-  } else {
-    VisCount cnt{0};
-    RayStats dummy = {};
-    rays(cnt, dummy);
-    VisEmit emit{ws.q, screen_pos * CT_VIS_SLOTS, screen_pos, block_reserve(cnt.n, ws.q.count)};
-    rays(emit, rs);
+    temporal_reuse(F, P, d, S, mat, r2, T.prev, T.prev_index, s2, screen_pos, ray, true, rs);
   }
+  // rays against the previous scene have their own count, walked by
+  // k_trace_prev
+  const uint32_t prev = (F.is_active & CT_REMAP_BIT) ? CT_PREV_COUNT : 0u;
+  emit_ray(ws.q, ray, block_reserve(ray.traced ? 1u : 0u, ws.q.count + prev), screen_pos, 2u);
   count_rays(P, rs);
 }
 
@@ -704,19 +723,6 @@ __global__ void __launch_bounds__(128) k_spatial_select(ct_push_constant pc, ct_
   ws.smeta[screen_pos] = make_uint2(n, seed);
 }
 
-// Captures the one shadow ray a call site would trace.
-struct VisCapture {
-  bool traced;
-  f3 o, d;
-  float dist;
-  uint32_t inst, prim;
-  bool check;
-  __device__ bool operator()(f3 o_, f3 d_, float dist_, uint32_t i_, uint32_t p_, bool c_, uint32_t) {
-    traced = true; o = o_; d = d_; dist = dist_; inst = i_; prim = p_; check = c_;
-    return true;
-  }
-};
-
 // one thread per (pixel, sample j < R)
 // 48 registers, 1280 threads per SM: 1.43 ms per 1080p frame against 1.50
 // ms at 1024, 1.80 ms at 768 and 1.79 ms with the register count left free;
@@ -774,9 +780,7 @@ __global__ void __launch_bounds__(CT_SPATIAL_SAMPLE_THREADS, CT_SPATIAL_SAMPLE_M
         ct_latch_error(CT_ERR_CAPACITY, 5, pixel);
         ws.vis[slot] = 0;
       } else {
-        ws.q.a[pos] = make_float4(cap.o.x, cap.o.y, cap.o.z, cap.dist);
-        ws.q.b[pos] = make_float4(cap.d.x, cap.d.y, cap.d.z, __uint_as_float(slot));
-        ws.q.c[pos] = make_uint2(cap.inst | (cap.check ? 0x80000000u : 0u), cap.prim);
+        cap.store(ws.q, pos, slot);
       }
     } else {
       ws.vis[slot] = 0;
