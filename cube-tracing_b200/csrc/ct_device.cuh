@@ -930,69 +930,60 @@ struct ShadowRay {
   uint32_t inst;          // instance being walked
 };
 
-// walk_init over instance `inst`'s grid (false: no overlap) for the ray's
-// object-space form in that instance
-__device__ __forceinline__ bool shadow_ray_instance(const DevAccel &A, ShadowRay &R, WalkState &s, uint32_t inst,
-                                                    f3 ro, f3 rd, f3 ird) {
-  WalkRay r;
-  if (!walk_init(A, A.grids[inst], ro, rd, ird, 0.f, fminf(R.tmax, R.target_t), r, s)) return false;
-  R.r = r;
-  R.ro = ro;
-  R.rd = rd;
-  R.ird = ird;
-  R.inst = inst;
-  return true;
-}
-
-// the first instance from `inst` on whose grid the ray overlaps; false when
-// none is left
-__device__ __forceinline__ bool shadow_ray_next(const DevAccel &A, ShadowRay &R, WalkState &s, uint32_t inst, f3 o,
-                                                f3 d) {
-  for (; inst < A.n_grids; inst++) {
-    const DevGrid &g = A.grids[inst];
-    const f3 ro = xyz(mul(g.world2obj_inst, mk4(o, 1.0f)));
-    const f3 rd = xyz(mul(g.world2obj_inst, mk4(d, 0.0f)));
-    if (shadow_ray_instance(A, R, s, inst, ro, rd, safe_inverse(rd))) return true;
-  }
-  return false;
-}
-
-// is_vertex_visible's set-up (light.glsl:82-105): the target voxel's key by
-// its own box test, then the first instance to walk.  False: nothing to walk
-// (the ray is visible).
-__device__ __forceinline__ bool shadow_ray_begin(const DevAccel &A, ShadowRay &R, WalkState &s, f3 o, f3 d,
-                                                 float distance, uint32_t t_inst, uint32_t t_prim,
-                                                 bool check_instance) {
+// is_vertex_visible's set-up (light.glsl:82-105): the query, and the target
+// voxel's key by its own box test.  True: `obj` is the object-space ray of
+// instance 0, where the walk begins (the target's, usually).
+__device__ __forceinline__ bool shadow_ray_target(const DevAccel &A, ShadowRay &R, ObjRay &obj, f3 o, f3 d,
+                                                  float distance, uint32_t t_inst, uint32_t t_prim,
+                                                  bool check_instance) {
   R.tmax = distance;
   R.target_t = INFINITY;
   R.target_g = 0xFFFFFFFFu;
   const bool has_target = check_instance && t_inst < A.n_grids;
   R.target_inst = has_target ? t_inst : 0xFFFFFFFFu;
   R.target_prim = t_prim;
-  if (has_target) {
-    const DevGrid &g = A.grids[t_inst];
-    if (t_prim < g.primitive_count) {
-      const f3 radius = half_extent_v(A), inv_radius = safe_inverse(radius);
-      const uint32_t gp = g.first_primitive_index + t_prim;
-      const uint32_t pk = __ldg(&A.voxel_coord[gp]);
-      const int x = (int)(pk & 0x3FFu), y = (int)((pk >> 10) & 0x3FFu), z = (int)((pk >> 20) & 0x3FFu);
-      const f3 ro = xyz(mul(g.world2obj_inst, mk4(o, 1.0f)));
-      const f3 rd = xyz(mul(g.world2obj_inst, mk4(d, 0.0f)));
-      const f3 ird = safe_inverse(rd);
-      const BoxHit h = box_test(voxel_center(A, g, x, y, z, t_prim), radius, inv_radius, ro, rd, false, false, ird);
-      if (h.hit && h.t >= 0.f && h.t <= distance) { R.target_t = h.t; R.target_g = gp; }
-      // the first instance to walk is usually the target's: its
-      // object-space ray is the one just made
-      if (t_inst == 0u) {
-        if (shadow_ray_instance(A, R, s, 0u, ro, rd, ird)) return true;
-        return shadow_ray_next(A, R, s, 1u, o, d);
-      }
-    }
-  }
-  return shadow_ray_next(A, R, s, 0, o, d);
+  if (!has_target) return false;
+  const DevGrid &g = A.grids[t_inst];
+  if (t_prim >= g.primitive_count) return false;
+  const f3 radius = half_extent_v(A), inv_radius = safe_inverse(radius);
+  const uint32_t gp = g.first_primitive_index + t_prim;
+  const uint32_t pk = __ldg(&A.voxel_coord[gp]);
+  const int x = (int)(pk & 0x3FFu), y = (int)((pk >> 10) & 0x3FFu), z = (int)((pk >> 20) & 0x3FFu);
+  obj.ro = xyz(mul(g.world2obj_inst, mk4(o, 1.0f)));
+  obj.rd = xyz(mul(g.world2obj_inst, mk4(d, 0.0f)));
+  obj.ird = safe_inverse(obj.rd);
+  const BoxHit h =
+      box_test(voxel_center(A, g, x, y, z, t_prim), radius, inv_radius, obj.ro, obj.rd, false, false, obj.ird);
+  if (h.hit && h.t >= 0.f && h.t <= distance) { R.target_t = h.t; R.target_g = gp; }
+  return t_inst == 0u;
 }
 
-// QueryVisitor::visit in visibility mode on the stored ray: true when voxel
+// The first instance from `inst` on whose grid the ray overlaps; false when
+// none is left.  `known`: `obj` is the object-space ray of instance `inst`.
+__device__ __forceinline__ bool shadow_ray_next(const DevAccel &A, ShadowRay &R, ObjRay obj, WalkState &s,
+                                                uint32_t inst, f3 o, f3 d, bool known) {
+#pragma unroll 1
+  for (; inst < A.n_grids; inst++, known = false) {
+    const DevGrid &g = A.grids[inst];
+    if (!known) {
+      obj.ro = xyz(mul(g.world2obj_inst, mk4(o, 1.0f)));
+      obj.rd = xyz(mul(g.world2obj_inst, mk4(d, 0.0f)));
+      obj.ird = safe_inverse(obj.rd);
+    }
+    WalkRay r;
+    if (walk_init(A, g, obj.ro, obj.rd, obj.ird, 0.f, fminf(R.tmax, R.target_t), r, s)) {
+      R.r = r;
+      R.ro = obj.ro;
+      R.rd = obj.rd;
+      R.ird = obj.ird;
+      R.inst = inst;
+      return true;
+    }
+  }
+  return false;
+}
+
+// VisibilityVisitor::visit on the stored ray: true when voxel
 // (x, y, z) = primitive `prim` of the instance blocks the ray
 __device__ __forceinline__ bool shadow_blocks(const DevAccel &A, const DevGrid &g, const ShadowRay &R, int x, int y,
                                               int z, uint32_t prim) {

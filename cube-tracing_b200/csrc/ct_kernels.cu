@@ -999,10 +999,18 @@ __device__ __forceinline__ void shadow_walker(const DevAccel &A, Rays src, RaySt
   bool active = false;      // the lane holds an unanswered ray
   bool exhausted = false;
   uint32_t qid = 0, slot = 0;
+  // the instance a lane's ray is to be walked through next: one piece of code
+  // sets up new rays and rays that go on to another instance (the walker's
+  // code is large enough for its instruction fetch to stall it)
+  bool begin = false;
+  uint32_t inst = 0;
   for (;;) {
     // refill
     const bool need = !active && !exhausted;
     const unsigned needmask = __ballot_sync(0xFFFFFFFFu, need);
+    f3 o = mk3(0.f), d = mk3(0.f);
+    ObjRay obj = {};
+    bool known = false;
     if (needmask) {
       const uint32_t base = src.reserve((uint32_t)__popc(needmask), (uint32_t)__ffs(needmask) - 1u);
       if (need) {
@@ -1010,21 +1018,30 @@ __device__ __forceinline__ void shadow_walker(const DevAccel &A, Rays src, RaySt
         if (qid >= n) {
           exhausted = true;
         } else {
-          f3 o, d;
           float dist;
-          uint32_t inst, prim;
+          uint32_t t_inst, t_prim;
           slot = src.ray(qid, o, d, dist);
-          const bool check = src.target(qid, inst, prim);
+          const bool check = src.target(qid, t_inst, t_prim);
           rs.shadow++;
-          ShadowRay &R = rays[lane];
-          if (shadow_ray_begin(A, R, st, o, d, dist, inst, prim, check)) {
-            active = true;
-            walk = WALK_MORE;
-            lim = walk_limit(R.r, fminf(R.tmax, R.target_t));
-          } else {
-            src.answer(slot, 1);  // nothing to walk: visible
-          }
+          known = shadow_ray_target(A, rays[lane], obj, o, d, dist, t_inst, t_prim, check);
+          active = begin = true;
+          inst = 0;
         }
+      }
+    }
+    if (begin) {
+      begin = false;
+      ShadowRay &R = rays[lane];
+      if (inst > 0) {
+        float dist;
+        src.ray(qid, o, d, dist);
+      }
+      if (shadow_ray_next(A, R, obj, st, inst, o, d, known)) {
+        walk = WALK_MORE;
+        lim = walk_limit(R.r, fminf(R.tmax, R.target_t));
+      } else {
+        src.answer(slot, 1);  // nothing (more) to walk: visible
+        active = false;
       }
     }
     if (!__any_sync(0xFFFFFFFFu, active || !exhausted)) break;
@@ -1066,17 +1083,9 @@ __device__ __forceinline__ void shadow_walker(const DevAccel &A, Rays src, RaySt
         walk = WALK_DONE;
       } else if (walk != WALK_MORE) {
         // the walk of this instance ended unblocked: the next instance, if any
-        f3 o, d;
-        float dist;
-        ShadowRay &R = rays[lane];
-        bool more = false;
-        if (R.inst + 1 < A.n_grids) {
-          src.ray(qid, o, d, dist);
-          more = shadow_ray_next(A, R, st, R.inst + 1, o, d);
-        }
-        if (more) {
-          walk = WALK_MORE;
-          lim = walk_limit(R.r, fminf(R.tmax, R.target_t));
+        inst = rays[lane].inst + 1u;
+        if (inst < A.n_grids) {
+          begin = true;
         } else {
           src.answer(slot, 1);
           active = false;
