@@ -245,13 +245,13 @@ extern "C" ct_status ct_restir_di(const ct_push_constant *pc, const ct_params *P
   // address the kernels read on the device, so the host only forwards the
   // round's source/destination choice.
   for (uint32_t r = 0; r + 1 < P->spatial_passes; r++) {
-    cudaError_t e = ct_launch_spatial_round(*pc, A, *P, w, (int)(r & 1u), 0, (int)((r & 1u) ^ 1u), s);
+    cudaError_t e = ct_launch_spatial_round(*pc, A, *P, w, r, (int)(r & 1u), 0, (int)((r & 1u) ^ 1u), s);
     if (e != cudaSuccess) return cuda_status(e);
   }
-  return cuda_status(ct_launch_spatial_round(*pc, A, *P, w, (int)((P->spatial_passes - 1) & 1u), 1, 0, s));
+  return cuda_status(ct_launch_spatial_round(*pc, A, *P, w, P->spatial_passes - 1, (int)((P->spatial_passes - 1) & 1u), 1, 0, s));
 }
 
-extern "C" ct_status ct_restir_pt(const ct_push_constant *pc, const ct_params *P, int stage, ct_stream stream) {
+static ct_status restir_pt(const ct_push_constant *pc, const ct_params *P, int stage, bool alone, ct_stream stream) {
   ct_status st = check_pc(pc, true);
   if (st == CT_OK) st = check_params(P);
   if (st == CT_OK) st = check_extent(pc, P);
@@ -260,7 +260,11 @@ extern "C" ct_status ct_restir_pt(const ct_push_constant *pc, const ct_params *P
   CtWorkspace w;
   st = get_workspace(pc, P, &w);
   if (st != CT_OK) return st;
-  return cuda_status(ct_launch_pt(*pc, walk_accel(pc->tlas, P), *P, w, stage, (cudaStream_t)stream));
+  return cuda_status(ct_launch_pt(*pc, walk_accel(pc->tlas, P), *P, w, stage, alone, (cudaStream_t)stream));
+}
+
+extern "C" ct_status ct_restir_pt(const ct_push_constant *pc, const ct_params *P, int stage, ct_stream stream) {
+  return restir_pt(pc, P, stage, true, stream);
 }
 
 extern "C" ct_status ct_taa(const ct_push_constant *pc, const ct_params *P, ct_stream stream) {
@@ -270,19 +274,24 @@ extern "C" ct_status ct_taa(const ct_push_constant *pc, const ct_params *P, ct_s
   return cuda_status(ct_launch_taa(*pc, *P, (cudaStream_t)stream));
 }
 
-extern "C" ct_status ct_render_frame(const ct_push_constant *pc, const ct_params *P, uint32_t is_active,
-                                     ct_stream stream) {
+static ct_status render_frame(const ct_push_constant *pc, const ct_params *P, uint32_t is_active, bool alone,
+                              ct_stream stream) {
   ct_status st = ct_trace_frame(pc, P, stream);
   if (st != CT_OK) return st;
   const bool indirect = (P->flags & CT_PARAM_INDIRECT) != 0;
   st = ct_restir_di(pc, P, 0, stream);
-  if (st == CT_OK && indirect) st = ct_restir_pt(pc, P, 0, stream);
+  if (st == CT_OK && indirect) st = restir_pt(pc, P, 0, alone, stream);
   if (st != CT_OK) return st;
   st = ct_restir_di(pc, P, 1, stream);
-  if (st == CT_OK && indirect) st = ct_restir_pt(pc, P, 1, stream);
+  if (st == CT_OK && indirect) st = restir_pt(pc, P, 1, alone, stream);
   if (st != CT_OK) return st;
   if (is_active & CT_TAA_BIT) st = ct_taa(pc, P, stream);
   return st;
+}
+
+extern "C" ct_status ct_render_frame(const ct_push_constant *pc, const ct_params *P, uint32_t is_active,
+                                     ct_stream stream) {
+  return render_frame(pc, P, is_active, true, stream);
 }
 
 // fork/join events of ct_render_views, per device (created on first use)
@@ -336,7 +345,7 @@ extern "C" ct_status ct_render_views(const ct_view *views, uint32_t n_views, con
   for (uint32_t l = 0; l < n_lanes && e == cudaSuccess; l++) e = cudaStreamWaitEvent((cudaStream_t)lanes[l], ev[n_lanes], 0);
   if (e != cudaSuccess) return cuda_status(e);
   for (uint32_t i = 0; i < n_views; i++) {
-    st = ct_render_frame(&views[i].pc, &views[i].params, views[i].is_active, lanes[views[i].lane]);
+    st = render_frame(&views[i].pc, &views[i].params, views[i].is_active, n_views == 1, lanes[views[i].lane]);
     if (st != CT_OK) return st;
   }
   for (uint32_t l = 0; l < n_lanes && e == cudaSuccess; l++) {

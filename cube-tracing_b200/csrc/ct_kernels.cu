@@ -13,6 +13,34 @@
 #include "ct_profile.cuh"
 
 // ---------------------------------------------------------------------------
+// The frame's kernels are launched with programmatic stream serialisation: a
+// kernel is placed as the blocks of the one before it end, and waits in
+// grid_begin for that one's writes to be visible.  Every kernel launched by
+// frame_launch therefore begins with grid_begin, before any access to memory.
+// A frame is some 40 dependent kernels, and small ones pay a launch's latency
+// for each: 256x256 frames 1.18 -> 1.10 ms, 1080p 10.37 -> 10.27 ms.  Letting
+// the next kernel in as soon as all blocks of this one have begun
+// (griddepcontrol.launch_dependents) gave that back: its waiting blocks take
+// the places of the walkers' later blocks (1.15 and 10.51 ms).
+__device__ __forceinline__ void grid_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... Params, class... Args>
+static cudaError_t frame_launch(int kid, cudaStream_t s, dim3 grid, dim3 block, void (*kernel)(Params...),
+                                const Args &...args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaSuccess;
+  CT_TIMED(kid, s, e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...));
+  return e;
+}
+
+// ---------------------------------------------------------------------------
 // per-block frame constants
 struct BlockConsts {
   FrameView F;
@@ -169,6 +197,7 @@ __device__ __forceinline__ void pixel_of(uint32_t &x, uint32_t &y) {
 #define CT_PRIMARY_MIN_BLOCKS 6
 #endif
 __global__ void __launch_bounds__(128, CT_PRIMARY_MIN_BLOCKS) k_trace_primary(ct_push_constant pc, DevAccel A, ct_params P) {
+  grid_begin();
   __shared__ BlockConsts B;
   __shared__ m4 inv_prev_mvp;
   load_frame_view(pc, B);
@@ -507,6 +536,7 @@ __device__ __forceinline__ void emit_ray(const RayQueue &q, const VisCapture &ra
 template <bool BRDF>
 __global__ void __launch_bounds__(128, BRDF ? 1 : CT_GEN0_MIN_BLOCKS) k_di_gen0(ct_push_constant pc, ct_params P,
                                                                           Workspace ws, DevAccel A) {
+  grid_begin();
   __shared__ BlockConsts B;
   // the flag first: the instantiation that does not run returns before
   // building the frame view
@@ -565,13 +595,14 @@ __global__ void __launch_bounds__(128, BRDF ? 1 : CT_GEN0_MIN_BLOCKS) k_di_gen0(
 
 // queue counter (in the workspace's counter block) of the rays traced against
 // the previous scene after an edit
-#define CT_PREV_COUNT 4u
+#define CT_PREV_COUNT 2u
 
 // stage 0, second generate: apply the RIS visibility answer, then ask for the
 // current sample's ray at the previous pixel (slot 2).  After a scene edit
 // (CT_REMAP_BIT) that ray goes to the previous-scene count instead, for
 // k_trace_prev.
 __global__ void __launch_bounds__(128) k_di_gen1(ct_push_constant pc, ct_params P, Workspace ws) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view(pc, B);
   __syncthreads();
@@ -634,6 +665,7 @@ __global__ void __launch_bounds__(128) k_di_gen1(ct_push_constant pc, ct_params 
 #define CT_DI_RESOLVE0_MIN_BLOCKS 8
 #endif
 __global__ void __launch_bounds__(128, CT_DI_RESOLVE0_MIN_BLOCKS) k_di_resolve0(ct_push_constant pc, ct_params P, Workspace ws) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view(pc, B);
   __syncthreads();
@@ -704,6 +736,7 @@ __device__ uint32_t spatial_select(const FrameView &F, const ct_params &P, float
 }
 
 __global__ void __launch_bounds__(128) k_spatial_select(ct_push_constant pc, ct_params P, Workspace ws, int src_sel) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view<false>(pc, B);
   __syncthreads();
@@ -736,6 +769,7 @@ __global__ void __launch_bounds__(128) k_spatial_select(ct_push_constant pc, ct_
 #endif
 __global__ void __launch_bounds__(CT_SPATIAL_SAMPLE_THREADS, CT_SPATIAL_SAMPLE_MIN_BLOCKS) k_spatial_sample(ct_push_constant pc, ct_params P, Workspace ws, int src_sel,
                                                        uint32_t R) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view<false>(pc, B);
   __syncthreads();
@@ -792,6 +826,7 @@ __global__ void __launch_bounds__(CT_SPATIAL_SAMPLE_THREADS, CT_SPATIAL_SAMPLE_M
 // round shades (rgen.glsl:405-509).
 __global__ void __launch_bounds__(128) k_spatial_resolve(ct_push_constant pc, ct_params P, Workspace ws, int src_sel,
                                                         int final_pass, int dst_sel) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view<false>(pc, B);
   __syncthreads();
@@ -1098,6 +1133,7 @@ __device__ __forceinline__ void shadow_walker(const DevAccel &A, Rays src, RaySt
 
 template <bool COUNT>
 __global__ void __launch_bounds__(256, CT_SHADOW_MIN_BLOCKS) k_trace_shadow(DevAccel A, ct_params P, Workspace ws) {
+  grid_begin();
   RayStats rs = {};
   shadow_walker<COUNT>(A, QueueRays{ws}, rs);
   rs.walker_bricks = rs.bricks;
@@ -1114,6 +1150,7 @@ __global__ void __launch_bounds__(256, CT_SHADOW_MIN_BLOCKS) k_query_visibility(
 // (vertex_visible_prev), one thread per ray; returns at once in the frames
 // without an edit, whose previous-scene count is 0.
 __global__ void __launch_bounds__(128) k_trace_prev(ct_push_constant pc, DevAccel A_prev, ct_params P, Workspace ws) {
+  grid_begin();
   const uint32_t n = ws.q.count[CT_PREV_COUNT];
   if (n == 0) return;  // the same for every thread
   const ct_world *wd = (const ct_world *)(uintptr_t)pc.world_buffer;
@@ -1139,6 +1176,7 @@ __global__ void __launch_bounds__(128) k_trace_prev(ct_push_constant pc, DevAcce
 // TAA (taa.glsl:16-109); the grid covers (W/8)*8 x (H/8)*8 pixels like the
 // reference dispatch.
 __global__ void __launch_bounds__(64) k_taa(ct_push_constant pc, ct_params P) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view<false>(pc, B);
   __syncthreads();
@@ -1374,6 +1412,7 @@ static_assert(kPathCols * 16 <= CT_PT_STATE_BYTES, "PathState outgrew its worksp
 // pass 1, ReSTIR PT block, part 1: the path starts at the primary hit; its
 // first bounce ray goes to queue 0
 __global__ void __launch_bounds__(128) k_pt_start(ct_push_constant pc, DevAccel A, ct_params P, PtWork w) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view(pc, B);
   __syncthreads();
@@ -1423,9 +1462,13 @@ __global__ void __launch_bounds__(128) k_pt_start(ct_push_constant pc, DevAccel 
 #endif
 template <bool COUNT>
 __global__ void __launch_bounds__(256, CT_EXTEND_MIN_BLOCKS) k_pt_extend(DevAccel A, ct_params P, PtWork w, int qi) {
+  grid_begin();
   const uint32_t n = w.count[2 * qi];
   uint32_t *cursor = w.count + 2 * qi + 1;
   const float4 *q = w.q[qi];
+  // the other queue, whose rays were shaded before this launch, is empty for
+  // the shading that follows it
+  if (blockIdx.x == 0 && threadIdx.x < 2u) w.count[2 * (qi ^ 1) + threadIdx.x] = 0u;
   const uint32_t lane = threadIdx.x & 31u;
   __shared__ WalkRay s_walk[256];
   __shared__ ObjRay s_obj[256];
@@ -1485,6 +1528,7 @@ __global__ void __launch_bounds__(256, CT_EXTEND_MIN_BLOCKS) k_pt_extend(DevAcce
 #endif
 __global__ void __launch_bounds__(256, CT_SHADE_MIN_BLOCKS) k_pt_shade(ct_push_constant pc, DevAccel A, ct_params P, Workspace ws,
                                                   PtWork w, int qi) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view(pc, B);
   __syncthreads();
@@ -1531,20 +1575,31 @@ __global__ void __launch_bounds__(256, CT_SHADE_MIN_BLOCKS) k_pt_shade(ct_push_c
   count_rays(P, rs);
 }
 
-// The paths still running after CT_PT_TAIL_ROUND wavefront rounds are few,
-// and each later round would wait for its slowest walk: one thread per path
-// finishes them here, walking each bounce ray in place and shading its
-// vertex, for the remaining rounds of the CT_PT_MAX_ITER bound.  Light-sample
-// rays go to the shadow-ray queue while it has room (their answers are not
-// read) and are walked in place otherwise.  With 8 wavefront rounds, paths
-// of up to 8 bounces never get here and the launch replaces the empty
-// rounds; earlier switches were measured slower on the 1080p terrain (one
-// thread per path walks and shades much slower per path than the wavefront).
+// Paths finished by one thread each: it walks each bounce ray in place and
+// shades its vertex, from `first_round` on to the CT_PT_MAX_ITER bound.
+// Light-sample rays go to the shadow-ray queue while it has room (their
+// answers are not read) and are walked in place otherwise.
+//  * After CT_PT_TAIL_ROUND wavefront rounds the paths still running are few,
+//    and each later round would wait for its slowest walk.  With 8 rounds,
+//    paths of up to 8 bounces never get here and the launch replaces the empty
+//    rounds.
+//  * A view that renders alone with at most CT_PT_ALONE_PIXELS pixels comes
+//    here at once: its paths fit the GPU as one thread each, and the 16
+//    launches of the rounds cost more than the divergence (256x256: 1.20 ->
+//    1.09 ms on a terrain to depth 8 and 1.14 -> 1.10 ms on a grid to depth
+//    4; 480x270: 1.52 -> 1.40 and 1.30 -> 1.30 ms; 640x360: 1.67 -> 1.80 ms,
+//    the wavefront is better).  Views rendered side by side fill the GPU
+//    together and keep the wavefront (8 views: 2.90 ms against 3.45 ms).
+#define CT_PT_ALONE_PIXELS (1u << 17)
 #ifndef CT_PT_TAIL_ROUND
 #define CT_PT_TAIL_ROUND 8
 #endif
-__global__ void __launch_bounds__(128) k_pt_finish(ct_push_constant pc, DevAccel A, ct_params P, Workspace ws,
-                                                   PtWork w, int qi) {
+#ifndef CT_PT_FINISH_MIN_BLOCKS
+#define CT_PT_FINISH_MIN_BLOCKS 4
+#endif
+__global__ void __launch_bounds__(128, CT_PT_FINISH_MIN_BLOCKS) k_pt_finish(ct_push_constant pc, DevAccel A, ct_params P,
+                                                                            Workspace ws, PtWork w, int qi, int first_round) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view(pc, B);
   __syncthreads();
@@ -1555,7 +1610,7 @@ __global__ void __launch_bounds__(128) k_pt_finish(ct_push_constant pc, DevAccel
   for (uint32_t id = blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
     const uint32_t pixel = __float_as_uint(w.q[qi][2u * id].w);
     PathState path = w.state.load(pixel);
-    for (int round = CT_PT_TAIL_ROUND; round < CT_PT_MAX_ITER; round++) {
+    for (int round = first_round; round < CT_PT_MAX_ITER; round++) {
       rs.bounce++;
       ClosestWalk cw;
       if (closest_walk<false>(A, cw, path.origin, path.dir, CT_MAX_DISTANCE, pixel, rs)) rs.bounce_hits++;
@@ -1678,6 +1733,7 @@ __device__ __forceinline__ bool needs_replay(const PathRes &src) {
 // the new path, which is shifted only when its weight is positive) and
 // marks the others as not asked for.
 __global__ void __launch_bounds__(128) k_pt_replay_jobs(ct_push_constant pc, PtWork w) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view(pc, B);
   __syncthreads();
@@ -1708,6 +1764,7 @@ __global__ void __launch_bounds__(128) k_pt_replay_jobs(ct_push_constant pc, PtW
 // stride, so that a warp walks 32 replays side by side instead of waiting
 // on one lane of a pixel kernel.
 __global__ void __launch_bounds__(128) k_pt_replay(ct_push_constant pc, DevAccel A, ct_params P, PtWork w) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view(pc, B);
   __syncthreads();
@@ -1780,6 +1837,7 @@ template <int PHASE, bool HYBRID>
 #endif
 __global__ void __launch_bounds__(128, PHASE == 0 ? CT_PT_TEMPORAL0_MIN_BLOCKS : CT_PT_TEMPORAL1_MIN_BLOCKS) k_pt_temporal(ct_push_constant pc, DevAccel A, ct_params P, Workspace ws,
                                                      PtWork w) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view(pc, B);
   __syncthreads();
@@ -1842,6 +1900,7 @@ __global__ void __launch_bounds__(128, PHASE == 0 ? CT_PT_TEMPORAL0_MIN_BLOCKS :
 #endif
 template <bool HYBRID>
 __global__ void __launch_bounds__(128, CT_PT_SPATIAL_MIN_BLOCKS) k_pt_spatial(ct_push_constant pc, DevAccel A, ct_params P) {
+  grid_begin();
   __shared__ BlockConsts B;
   load_frame_view(pc, B);
   __syncthreads();
@@ -2047,15 +2106,31 @@ static dim3 frame_grid(uint32_t W, uint32_t H, dim3 blk) {
 
 cudaError_t ct_launch_trace(const ct_push_constant &pc, const DevAccel &A, const ct_params &P, cudaStream_t s) {
   dim3 blk(16, 8);
-  CT_TIMED(CT_K_TRACE_PRIMARY, s, k_trace_primary<<<frame_grid(pc.size[0], pc.size[1], blk), blk, 0, s>>>(pc, A, P));
-  return cudaGetLastError();
+  return frame_launch(CT_K_TRACE_PRIMARY, s, frame_grid(pc.size[0], pc.size[1], blk), blk, k_trace_primary, pc, A, P);
 }
-static Workspace make_ws(const CtWorkspace &w) {
+
+// Words of the workspace's counter block.  Every walker launch has a shadow
+// queue count and cursor of its own, so that a call clears its part of the
+// block once instead of before each pass.
+enum : uint32_t {
+  CT_CTR_DI = 0,        // stage 0: first generation; + 2: second; + 4: rays against the previous scene
+  CT_CTR_DI_END = 6,
+  CT_CTR_SPATIAL = 8,   // 2 per spatial round (up to 16)
+  CT_CTR_SPATIAL_END = 40,
+  CT_CTR_PT = 40,       // path queues, replay jobs
+  CT_CTR_PT_SHADOW = 46, // 2 per walker launch of ReSTIR PT
+  CT_CTR_END = 64       // 256 bytes
+};
+static_assert(CT_PREV_COUNT == 2u, "previous-scene count behind the second generation's");
+static cudaError_t clear_counters(const CtWorkspace &w, uint32_t first, uint32_t end, cudaStream_t s) {
+  return cudaMemsetAsync(w.counter + first, 0, (end - first) * sizeof(uint32_t), s);
+}
+static Workspace make_ws(const CtWorkspace &w, uint32_t counter) {
   Workspace ws;
   ws.q.a = (float4 *)w.ray_a;
   ws.q.b = (float4 *)w.ray_b;
   ws.q.c = (uint2 *)w.ray_c;
-  ws.q.count = w.counter;
+  ws.q.count = w.counter + counter;
   ws.q.capacity = w.capacity;
   ws.vis = w.vis;
   ws.rad = w.rad;
@@ -2072,96 +2147,90 @@ static uint32_t walker_grid(const ct_params &P) {
 // the frame accumulates work counters (CT_PARAM_COUNT_RAYS)
 static bool counting(const ct_params &P) { return (P.flags & CT_PARAM_COUNT_RAYS) && P.counters_address; }
 
-static cudaError_t trace_queue(const ct_push_constant &pc, const DevAccel &A, const ct_params &P,
-                               const CtWorkspace &w, cudaStream_t s) {
+static cudaError_t trace_queue(const DevAccel &A, const ct_params &P, const Workspace &ws, cudaStream_t s) {
   // the queue length is only known on the device: a grid that fills the GPU
   // walks the queue with a grid stride
-  if (counting(P))
-    CT_TIMED(CT_K_TRACE_SHADOW, s, k_trace_shadow<true><<<walker_grid(P), 256, 0, s>>>(A, P, make_ws(w)));
-  else
-    CT_TIMED(CT_K_TRACE_SHADOW, s, k_trace_shadow<false><<<walker_grid(P), 256, 0, s>>>(A, P, make_ws(w)));
-  return cudaGetLastError();
+  return frame_launch(CT_K_TRACE_SHADOW, s, walker_grid(P), 256,
+                      counting(P) ? k_trace_shadow<true> : k_trace_shadow<false>, A, P, ws);
 }
 
 cudaError_t ct_launch_di_stage0(const ct_push_constant &pc, const DevAccel &A, const DevAccel &A_prev,
                                 const ct_params &P, const CtWorkspace &w, cudaStream_t s) {
   dim3 blk(16, 8);
   const dim3 grid = frame_grid(pc.size[0], pc.size[1], blk);
-  const Workspace ws = make_ws(w);
-  cudaError_t e;
-  if ((e = cudaMemsetAsync(w.counter, 0, 2 * sizeof(uint32_t), s)) != cudaSuccess) return e;
-  CT_TIMED(CT_K_DI_GEN0, s, k_di_gen0<false><<<grid, blk, 0, s>>>(pc, P, ws, A));
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  CT_TIMED(CT_K_DI_GEN0, s, k_di_gen0<true><<<grid, blk, 0, s>>>(pc, P, ws, A));
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if ((e = trace_queue(pc, A, P, w, s)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(w.counter, 0, (CT_PREV_COUNT + 1) * sizeof(uint32_t), s)) != cudaSuccess) return e;
-  CT_TIMED(CT_K_DI_GEN1, s, k_di_gen1<<<grid, blk, 0, s>>>(pc, P, ws));
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if ((e = trace_queue(pc, A, P, w, s)) != cudaSuccess) return e;
-  CT_TIMED(CT_K_TRACE_PREV, s, k_trace_prev<<<sm_count() * 8, 128, 0, s>>>(pc, A_prev, P, ws));
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  CT_TIMED(CT_K_DI_RESOLVE0, s, k_di_resolve0<<<grid, blk, 0, s>>>(pc, P, ws));
-  return cudaGetLastError();
+  const Workspace ws0 = make_ws(w, CT_CTR_DI), ws1 = make_ws(w, CT_CTR_DI + 2);
+  cudaError_t e = clear_counters(w, CT_CTR_DI, CT_CTR_DI_END, s);
+  if (e == cudaSuccess) e = frame_launch(CT_K_DI_GEN0, s, grid, blk, k_di_gen0<false>, pc, P, ws0, A);
+  if (e == cudaSuccess) e = frame_launch(CT_K_DI_GEN0, s, grid, blk, k_di_gen0<true>, pc, P, ws0, A);
+  if (e == cudaSuccess) e = trace_queue(A, P, ws0, s);
+  if (e == cudaSuccess) e = frame_launch(CT_K_DI_GEN1, s, grid, blk, k_di_gen1, pc, P, ws1);
+  if (e == cudaSuccess) e = trace_queue(A, P, ws1, s);
+  if (e == cudaSuccess) e = frame_launch(CT_K_TRACE_PREV, s, sm_count() * 8, 128, k_trace_prev, pc, A_prev, P, ws1);
+  if (e == cudaSuccess) e = frame_launch(CT_K_DI_RESOLVE0, s, grid, blk, k_di_resolve0, pc, P, ws1);
+  return e;
 }
 
 cudaError_t ct_launch_spatial_round(const ct_push_constant &pc, const DevAccel &A, const ct_params &P,
-                                    const CtWorkspace &w, int src_sel, int final_pass, int dst_sel, cudaStream_t s) {
+                                    const CtWorkspace &w, uint32_t round, int src_sel, int final_pass, int dst_sel,
+                                    cudaStream_t s) {
   dim3 blk(16, 8);
   const dim3 grid = frame_grid(pc.size[0], pc.size[1], blk);
-  const Workspace ws = make_ws(w);
-  cudaError_t e;
-  if ((e = cudaMemsetAsync(w.counter, 0, 2 * sizeof(uint32_t), s)) != cudaSuccess) return e;
-  CT_TIMED(CT_K_SPATIAL_SELECT, s, k_spatial_select<<<grid, blk, 0, s>>>(pc, P, ws, src_sel));
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  const Workspace ws = make_ws(w, CT_CTR_SPATIAL + 2u * round);
+  cudaError_t e = round == 0 ? clear_counters(w, CT_CTR_SPATIAL, CT_CTR_SPATIAL_END, s) : cudaSuccess;
+  if (e == cudaSuccess) e = frame_launch(CT_K_SPATIAL_SELECT, s, grid, blk, k_spatial_select, pc, P, ws, src_sel);
   uint32_t nmax = P.max_num_of_neighbors > P.min_num_of_neighbors ? P.max_num_of_neighbors : P.min_num_of_neighbors;
   if (nmax > CT_MAX_NEIGHBORS) nmax = CT_MAX_NEIGHBORS;
-  if (nmax > 0) {
+  if (nmax > 0 && e == cudaSuccess) {
     const uint32_t R = 2u * nmax;
     const uint64_t threads = (uint64_t)pc.size[0] * pc.size[1] * R;
-    CT_TIMED(CT_K_SPATIAL_SAMPLE, s,
-             k_spatial_sample<<<(uint32_t)((threads + CT_SPATIAL_SAMPLE_THREADS - 1) / CT_SPATIAL_SAMPLE_THREADS),
-                                CT_SPATIAL_SAMPLE_THREADS, 0, s>>>(pc, P, ws, src_sel, R));
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = frame_launch(CT_K_SPATIAL_SAMPLE, s,
+                     (uint32_t)((threads + CT_SPATIAL_SAMPLE_THREADS - 1) / CT_SPATIAL_SAMPLE_THREADS),
+                     CT_SPATIAL_SAMPLE_THREADS, k_spatial_sample, pc, P, ws, src_sel, R);
   }
-  if ((e = trace_queue(pc, A, P, w, s)) != cudaSuccess) return e;
-  CT_TIMED(CT_K_SPATIAL_RESOLVE, s, k_spatial_resolve<<<grid, blk, 0, s>>>(pc, P, ws, src_sel, final_pass, dst_sel));
-  return cudaGetLastError();
+  if (e == cudaSuccess) e = trace_queue(A, P, ws, s);
+  if (e == cudaSuccess)
+    e = frame_launch(CT_K_SPATIAL_RESOLVE, s, grid, blk, k_spatial_resolve, pc, P, ws, src_sel, final_pass, dst_sel);
+  return e;
 }
 cudaError_t ct_launch_taa(const ct_push_constant &pc, const ct_params &P, cudaStream_t s) {
   const uint32_t gx = pc.size[0] / 8, gy = pc.size[1] / 8;
   if (gx == 0 || gy == 0) return cudaSuccess;
-  dim3 blk(8, 8);
-  CT_TIMED(CT_K_TAA, s, k_taa<<<dim3(gx, gy, 1), blk, 0, s>>>(pc, P));
-  return cudaGetLastError();
+  return frame_launch(CT_K_TAA, s, dim3(gx, gy, 1), dim3(8, 8), k_taa, pc, P);
 }
 
 cudaError_t ct_launch_pt(const ct_push_constant &pc, const DevAccel &A, const ct_params &P, const CtWorkspace &w,
-                         int stage, cudaStream_t s) {
+                         int stage, bool alone, cudaStream_t s) {
   dim3 blk(16, 8);
   const dim3 grid = frame_grid(pc.size[0], pc.size[1], blk);
-  if (stage != 0) {
-    if (P.pt_shift_mapping == CT_SHIFT_HYBRID)
-      CT_TIMED(CT_K_PT_SPATIAL, s, k_pt_spatial<true><<<grid, blk, 0, s>>>(pc, A, P));
-    else
-      CT_TIMED(CT_K_PT_SPATIAL, s, k_pt_spatial<false><<<grid, blk, 0, s>>>(pc, A, P));
-    return cudaGetLastError();
-  }
+  const bool hybrid = P.pt_shift_mapping == CT_SHIFT_HYBRID;
+  if (stage != 0)
+    return frame_launch(CT_K_PT_SPATIAL, s, grid, blk, hybrid ? k_pt_spatial<true> : k_pt_spatial<false>, pc, A, P);
   PtWork pw;
   pw.state.col = (uint4 *)w.pt_state;
   pw.state.n = pc.size[0] * pc.size[1];
   pw.hit = (uint4 *)w.pt_hit;
   pw.q[0] = (float4 *)w.pt_q[0];
   pw.q[1] = (float4 *)w.pt_q[1];
-  pw.count = w.counter + 8;
+  pw.count = w.counter + CT_CTR_PT;
   pw.capacity = w.pt_capacity;
   pw.replay = (ReplayOut *)w.pt_replay;
   pw.jobs = (uint32_t *)w.pt_jobs;
-  const Workspace ws = make_ws(w);
-  cudaError_t e;
-  if ((e = cudaMemsetAsync(pw.count, 0, 4 * sizeof(uint32_t), s)) != cudaSuccess) return e;
-  CT_TIMED(CT_K_PT_START, s, k_pt_start<<<grid, blk, 0, s>>>(pc, A, P, pw));
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  cudaError_t e = clear_counters(w, CT_CTR_PT, CT_CTR_END, s);
+  if (e == cudaSuccess) e = frame_launch(CT_K_PT_START, s, grid, blk, k_pt_start, pc, A, P, pw);
+  // the counters of the walker launches in turn; past the last pair, the pair
+  // is cleared and used again
+  uint32_t shadow = CT_CTR_PT_SHADOW;
+  Workspace ws = make_ws(w, shadow);
+  const auto flush = [&]() {
+    cudaError_t r = trace_queue(A, P, ws, s);
+    if (shadow + 4u <= CT_CTR_END) {
+      shadow += 2u;
+      ws = make_ws(w, shadow);
+    } else if (r == cudaSuccess) {
+      r = clear_counters(w, shadow, shadow + 2u, s);
+    }
+    return r;
+  };
   // the queue lengths are only known on the device: a fixed number of rounds,
   // enough for the longest path (max_depth < CT_PT_MAX_ITER), each a no-op
   // once the queues are empty.  A round queues at most one light-sample ray
@@ -2170,49 +2239,34 @@ cudaError_t ct_launch_pt(const ct_push_constant &pc, const DevAccel &A, const ct
   // rays of `group` rounds share the shadow-ray queue and one walker launch.
   const uint64_t px = (uint64_t)pc.size[0] * pc.size[1];
   const int group = px && w.capacity / px > 0 ? (int)(w.capacity / px) : 1;
-  if ((e = cudaMemsetAsync(w.counter, 0, 2 * sizeof(uint32_t), s)) != cudaSuccess) return e;
-  const int rounds = CT_PT_TAIL_ROUND < CT_PT_MAX_ITER ? CT_PT_TAIL_ROUND : CT_PT_MAX_ITER;
-  for (int it = 0; it < rounds; it++) {
+  const int rounds = alone && px <= CT_PT_ALONE_PIXELS ? 0 : CT_PT_TAIL_ROUND;
+  for (int it = 0; it < rounds && e == cudaSuccess; it++) {
     const int qi = it & 1;
-    if (counting(P))
-      CT_TIMED(CT_K_PT_EXTEND, s, k_pt_extend<true><<<walker_grid(P), 256, 0, s>>>(A, P, pw, qi));
-    else
-      CT_TIMED(CT_K_PT_EXTEND, s, k_pt_extend<false><<<walker_grid(P), 256, 0, s>>>(A, P, pw, qi));
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(pw.count + 2 * (qi ^ 1), 0, 2 * sizeof(uint32_t), s)) != cudaSuccess) return e;
-    CT_TIMED(CT_K_PT_SHADE, s, k_pt_shade<<<(walker_grid(P) + 1) / 2, 256, 0, s>>>(pc, A, P, ws, pw, qi));
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((it + 1) % group == 0 || it + 1 == rounds) {
-      if ((e = trace_queue(pc, A, P, w, s)) != cudaSuccess) return e;
-      if ((e = cudaMemsetAsync(w.counter, 0, 2 * sizeof(uint32_t), s)) != cudaSuccess) return e;
-    }
+    e = frame_launch(CT_K_PT_EXTEND, s, walker_grid(P), 256, counting(P) ? k_pt_extend<true> : k_pt_extend<false>, A, P,
+                     pw, qi);
+    if (e == cudaSuccess)
+      e = frame_launch(CT_K_PT_SHADE, s, (walker_grid(P) + 1) / 2, 256, k_pt_shade, pc, A, P, ws, pw, qi);
+    if (e == cudaSuccess && ((it + 1) % group == 0 || it + 1 == rounds)) e = flush();
   }
   if (rounds < CT_PT_MAX_ITER) {
-    CT_TIMED(CT_K_PT_FINISH, s, k_pt_finish<<<walker_grid(P), 128, 0, s>>>(pc, A, P, ws, pw, rounds & 1));
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = trace_queue(pc, A, P, w, s)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(w.counter, 0, 2 * sizeof(uint32_t), s)) != cudaSuccess) return e;
+    if (e == cudaSuccess)
+      e = frame_launch(CT_K_PT_FINISH, s, walker_grid(P), 128, k_pt_finish, pc, A, P, ws, pw, rounds & 1, rounds);
+    if (e == cudaSuccess) e = flush();
   }
-  const bool hybrid = P.pt_shift_mapping == CT_SHIFT_HYBRID;
   if (hybrid) {
     // the replays temporal reuse will ask for, walked side by side first
-    if ((e = cudaMemsetAsync(pw.count + 4, 0, sizeof(uint32_t), s)) != cudaSuccess) return e;
-    CT_TIMED(CT_K_PT_REPLAY, s, k_pt_replay_jobs<<<grid, blk, 0, s>>>(pc, pw));
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    CT_TIMED(CT_K_PT_REPLAY, s, k_pt_replay<<<sm_count() * 8, 128, 0, s>>>(pc, A, P, pw));
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (e == cudaSuccess) e = frame_launch(CT_K_PT_REPLAY, s, grid, blk, k_pt_replay_jobs, pc, pw);
+    if (e == cudaSuccess) e = frame_launch(CT_K_PT_REPLAY, s, sm_count() * 8, 128, k_pt_replay, pc, A, P, pw);
   }
-  if (hybrid)
-    CT_TIMED(CT_K_PT_TEMPORAL, s, k_pt_temporal<0, true><<<grid, blk, 0, s>>>(pc, A, P, ws, pw));
-  else
-    CT_TIMED(CT_K_PT_TEMPORAL, s, k_pt_temporal<0, false><<<grid, blk, 0, s>>>(pc, A, P, ws, pw));
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if ((e = trace_queue(pc, A, P, w, s)) != cudaSuccess) return e;
-  if (hybrid)
-    CT_TIMED(CT_K_PT_TEMPORAL, s, k_pt_temporal<1, true><<<grid, blk, 0, s>>>(pc, A, P, ws, pw));
-  else
-    CT_TIMED(CT_K_PT_TEMPORAL, s, k_pt_temporal<1, false><<<grid, blk, 0, s>>>(pc, A, P, ws, pw));
-  return cudaGetLastError();
+  if (e == cudaSuccess)
+    e = frame_launch(CT_K_PT_TEMPORAL, s, grid, blk, hybrid ? k_pt_temporal<0, true> : k_pt_temporal<0, false>, pc, A, P,
+                     ws, pw);
+  const Workspace answers = ws;
+  if (e == cudaSuccess) e = flush();
+  if (e == cudaSuccess)
+    e = frame_launch(CT_K_PT_TEMPORAL, s, grid, blk, hybrid ? k_pt_temporal<1, true> : k_pt_temporal<1, false>, pc, A, P,
+                     answers, pw);
+  return e;
 }
 
 // device status word access for ct_get_error

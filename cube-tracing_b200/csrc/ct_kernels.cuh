@@ -28,10 +28,12 @@ struct CtWorkspace {
 cudaError_t ct_launch_di_stage0(const ct_push_constant &pc, const DevAccel &A, const DevAccel &A_prev,
                                 const ct_params &P, const CtWorkspace &w, cudaStream_t s);
 cudaError_t ct_launch_spatial_round(const ct_push_constant &pc, const DevAccel &A, const ct_params &P,
-                                    const CtWorkspace &w, int src_sel, int final_pass, int dst_sel, cudaStream_t s);
+                                    const CtWorkspace &w, uint32_t round, int src_sel, int final_pass, int dst_sel,
+                                    cudaStream_t s);
 cudaError_t ct_launch_taa(const ct_push_constant &pc, const ct_params &P, cudaStream_t s);
+// alone: no other view's frame runs beside this one
 cudaError_t ct_launch_pt(const ct_push_constant &pc, const DevAccel &A, const ct_params &P, const CtWorkspace &w,
-                         int stage, cudaStream_t s);
+                         int stage, bool alone, cudaStream_t s);
 cudaError_t ct_launch_brush(const ct_push_constant &pc, cudaStream_t s);
 cudaError_t ct_launch_rearrange(const ct_push_constant &pc, uint32_t instance_count, uint32_t primitive_count,
                                 cudaStream_t s);

@@ -84,8 +84,8 @@ extern "C" ct_status ct_restir_di_static(const ct_push_constant *pc, const ct_pa
   const DevAccel A_prev = pc->tlas_previous ? walk_accel(pc->tlas_previous, P) : A;
   if (stage == 0) return cuda_status(ct_launch_di_stage0(*pc, A, A_prev, *P, w, s));
   for (uint32_t r = 0; r + 1 < P->spatial_passes; r++) {
-    cudaError_t e = ct_launch_spatial_round(*pc, A, *P, w, (int)(r & 1u), 0, (int)((r & 1u) ^ 1u), s);
+    cudaError_t e = ct_launch_spatial_round(*pc, A, *P, w, r, (int)(r & 1u), 0, (int)((r & 1u) ^ 1u), s);
     if (e != cudaSuccess) return cuda_status(e);
   }
-  return cuda_status(ct_launch_spatial_round(*pc, A, *P, w, (int)((P->spatial_passes - 1) & 1u), 1, 0, s));
+  return cuda_status(ct_launch_spatial_round(*pc, A, *P, w, P->spatial_passes - 1, (int)((P->spatial_passes - 1) & 1u), 1, 0, s));
 }
