@@ -9,20 +9,24 @@
 // in tensor memory; each hidden activation is rounded to bf16 before the
 // next layer reads it.
 //
-// One CTA of 256 threads per SM: two warpgroups, each walking its own tiles
-// of 128 queries with its own input tile in shared memory, its own 64
-// tensor-memory columns and its own mbarrier, so that one warpgroup's
-// encoding and epilogues overlap the other's MMAs.  The weights (66 KB) are
-// shared; with the two input tiles the CTA holds 195 KB.  Per tile:
-//  * every thread encodes its query into the tile (row = thread), stored
-//    K-major in 128-byte-swizzled atoms of 8 rows x 64 bf16, chunk by chunk
-//    as it computes them;
+// One CTA of 512 threads per SM: four warpgroups, each walking its own tiles
+// of 128 queries with two 16 KB input buffers (64 of the 256 inputs each), its
+// own 64 tensor-memory columns and two mbarriers, so that the warpgroups'
+// encodings, epilogues and MMAs overlap.  The weights (66 KB) are shared; with
+// the buffers the CTA holds 194 KB.  Per tile:
+//  * every thread encodes its query into the buffers (row = thread), K-major
+//    in 128-byte-swizzled atoms of 8 rows x 64 bf16, one block of 64 inputs
+//    after the other; the block's MMAs run while the next one is encoded;
 //  * one thread of the warpgroup issues tcgen05.mma (M 128, N 64, K 16 per
-//    instruction, bf16 inputs, fp32 accumulator) over the layer's K and
-//    commits to the warpgroup's mbarrier;
-//  * every warp reads its 32 TMEM lanes (tcgen05.ld 32x32b), applies ReLU,
-//    rounds to bf16 and writes the next layer's input tile in place;
+//    instruction, bf16 inputs, fp32 accumulator) and commits to the buffer's
+//    mbarrier;
+//  * every warp reads its 32 TMEM lanes (tcgen05.ld 32x32b), rounds to bf16,
+//    applies ReLU and writes the next layer's input into the first buffer;
 //  * the last layer (N 16) writes RGB to global memory.
+// What bounds it is instruction issue: the encoding's 48 sincospi and 128
+// exponentials and the epilogues are some 3000 instructions per query against
+// 42 kFLOP of MMAs.  With whole 64 KB tiles only two warpgroups fitted (8
+// warps per SM, issue 44% active): 2.07 M queries took 573 us.
 // Warpgroups synchronise on their own named barriers.  Operands are staged
 // with ordinary 16-byte shared stores (no TMA).  Every wait is bounded
 // (about one second); a warpgroup that gives up latches an error in the
@@ -31,6 +35,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <type_traits>
 #include "ct.h"
 #include "ct_profile.cuh"
 
@@ -41,18 +46,22 @@ constexpr int kIn = CT_NRC_INPUT_DIMS;     // 256
 constexpr int kWidth = CT_NRC_WIDTH;       // 64
 constexpr int kOut = CT_NRC_OUTPUT_DIMS;   // 16
 constexpr int kHidden = CT_NRC_HIDDEN_LAYERS;  // 5
-constexpr int kGroups = 2;                    // warpgroups per CTA, one tile each
-constexpr int kThreads = kTile * kGroups;     // 256
+constexpr int kGroups = 4;                    // warpgroups per CTA, one tile each
+constexpr int kThreads = kTile * kGroups;     // 512
 constexpr int kTmemCols = 64 * kGroups;       // 64 accumulator columns per warpgroup
+constexpr int kBlockK = 64;                   // inputs per buffer
+static_assert(kIn == 4 * kBlockK, "blocks of the first layer");
 
 // shared memory regions, each 1024-byte aligned (128-byte swizzle atoms)
-constexpr uint32_t kABytes = 4 * 16384;                     // 4 K-blocks of [128 x 64] bf16 = 64 KB
-constexpr uint32_t kSmemA = 0;                              // one input tile per warpgroup
-constexpr uint32_t kSmemW0 = kSmemA + kGroups * kABytes;    // 4 K-blocks of [64 x 64] = 32 KB
+constexpr uint32_t kBufBytes = kTile * kBlockK * 2;         // 16 KB
+constexpr uint32_t kSmemA = 0;                              // two buffers per warpgroup
+constexpr uint32_t kSmemW0 = kSmemA + kGroups * 2 * kBufBytes;  // 4 K-blocks of [64 x 64] = 32 KB
 constexpr uint32_t kSmemWh = kSmemW0 + 4 * 8192;            // 4 hidden layers of [64 x 64] = 32 KB
 constexpr uint32_t kSmemW5 = kSmemWh + 4 * 8192;            // [16 x 64] = 2 KB
-constexpr uint32_t kSmemBar = kSmemW5 + 2048;               // an mbarrier (8 B) per warpgroup + TMEM address
-constexpr uint32_t kSmemBytes = kSmemBar + 64 + 1024;       // + slack to align the base to 1024
+constexpr uint32_t kSmemBar = kSmemW5 + 2048;               // two mbarriers (8 B) per warpgroup
+constexpr uint32_t kSmemFail = kSmemBar + 16 * kGroups;     // a word per warpgroup: a wait ran out
+constexpr uint32_t kSmemTmem = kSmemFail + 4 * kGroups;     // TMEM address
+constexpr uint32_t kSmemBytes = kSmemTmem + 16 + 1024;      // + slack to align the base to 1024
 static_assert(kSmemBytes <= 227 * 1024, "shared memory per CTA");
 
 // weight offsets in the packed bf16 buffer (elements)
@@ -112,37 +121,45 @@ __device__ __forceinline__ uint64_t now_ns() {
   return t;
 }
 
-// waits for the mbarrier phase `parity`, for at most about one second
+__device__ __forceinline__ bool try_bar(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// waits for the mbarrier phase `parity`, for at most about one second; the
+// clock is read only by waits that the first try does not end
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity) {
+  if (try_bar(bar, parity)) return true;
   const uint64_t t0 = now_ns();
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-    if (now_ns() - t0 > 1000000000ull) return false;
-  }
+  while (now_ns() - t0 <= 1000000000ull)
+    if (try_bar(bar, parity)) return true;
+  return false;
 }
 
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// 16 fp32 columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v) {
-  uint32_t r[16];
+// 16 fp32 columns of this thread's TMEM lane; tmem_wait before they are read
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+// the loaded registers pass through the wait, so that no use moves before it
+__device__ __forceinline__ void tmem_wait16(uint32_t *r) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
 }
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
@@ -160,93 +177,115 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 //              1/2) / 32) * 32)^2 / 2);
 //   [160, 224) the normal, the same way;
 //   [224, 227) albedo; [227, 256) zero.
-__device__ __forceinline__ float onehot_bin(float u, int i) {
-  const float d = (u - ((float)i + 0.5f) * (1.0f / 32.0f)) * 32.0f;
-  return __expf(-0.5f * d * d);
+// Bin i of a one-blob with u32 = 32 u: exp(-d^2 / 2), d = u32 - (i + 1/2), as
+// 2^(d^2 * (-log2(e) / 2)).  FTZ: bins below 2^-126 become 0 (the fused
+// network, whose outputs they cannot reach; two instructions less per bin).
+template <bool FTZ>
+__device__ __forceinline__ float blob_bin(float u32, int i) {
+  const float d = u32 - ((float)i + 0.5f), x = (d * d) * -0.72134752044448170368f;
+  float r;
+  if (FTZ) asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  else asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
-
-// The encoding in 16-byte chunks of 8 values, emitted as they are computed
-// (emit(chunk, v)): chunk 4c + j holds bands 4j .. 4j + 3 of axis c,
-// chunks 12 + 8v + j (j < 4) the first angle's bins 8j .. 8j + 7 of vector
-// v, chunks 12 + 8v + 4 + j the second angle's, chunk 28 the albedo and
-// chunks 29-31 zeros.  (q_c 2^k) mod 2 is s - 2 floor(s / 2) with s = q_c 2^k:
-// every step is exact for s < 2^23, as fmod is.
-template <class Emit>
-__device__ __forceinline__ void encode_chunks(const ct_nrc_query &q, const float *bmin, const float *bext, Emit &&emit) {
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    float x = (q.position[c] - bmin[c]) / bext[c];
-    x = fminf(fmaxf(x, 0.0f), 1.0f);
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      float v[8];
-#pragma unroll
-      for (int b = 0; b < 4; b++) {
-        const float sc = x * (float)(1u << (4 * j + b));
-        const float t = sc - 2.0f * floorf(sc * 0.5f);
-        sincospif(t, &v[2 * b], &v[2 * b + 1]);
-      }
-      emit(4 * c + j, v);
-    }
-  }
-  const float *vec[2] = {q.direction, q.normal};
-#pragma unroll
-  for (int w = 0; w < 2; w++) {
-    const float u[2] = {atan2f(vec[w][2], vec[w][0]) * (0.5f / 3.14159265358979323846f) + 0.5f,
-                        vec[w][1] * 0.5f + 0.5f};
-#pragma unroll
-    for (int a = 0; a < 2; a++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        float v[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = onehot_bin(u[a], 8 * j + i);
-        emit(12 + 8 * w + 4 * a + j, v);
-      }
-  }
-  float v[8] = {q.albedo[0], q.albedo[1], q.albedo[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-  emit(28, v);
-#pragma unroll
-  for (int i = 0; i < 3; i++) v[i] = 0.0f;
-#pragma unroll
-  for (int ch = 29; ch < 32; ch++) emit(ch, v);
-}
-
 __device__ __forceinline__ uint4 pack8(const float *v) {
   return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
 }
 
-__global__ void __launch_bounds__(256) k_nrc_encode(const ct_nrc_query *q, uint32_t n, float3 bmin, float3 bext,
-                                                    __nv_bfloat16 *out) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// The encoding in 16-byte chunks of 8 values: chunk 4c + j holds bands 4j ..
+// 4j + 3 of axis c, chunks 12 + 8v + j (j < 4) the first angle's bins 8j .. 8j
+// + 7 of vector v, chunks 12 + 8v + 4 + j the second angle's, chunk 28 the
+// albedo and chunks 29-31 zeros.  sincospi reduces its argument itself, so a
+// band's phase is q_c 2^k, an exact product, as it stands.
+//
+// encode_block<KB> emits (emit(chunk, v)) the 8 chunks of block KB.
+template <class Emit>
+__device__ __forceinline__ void encode_axis(float p, float bmin, float bext, int chunk, Emit &&emit) {
+  const float x = fminf(fmaxf((p - bmin) / bext, 0.0f), 1.0f);
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    float v[8];
+#pragma unroll
+    for (int b = 0; b < 4; b++) sincospif(x * (float)(1u << (4 * j + b)), &v[2 * b], &v[2 * b + 1]);
+    emit(chunk + j, pack8(v));
+  }
+}
+template <bool FTZ, class Emit>
+__device__ __forceinline__ void encode_blob(float u, int chunk, Emit &&emit) {
+  const float u32 = u * 32.0f;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = blob_bin<FTZ>(u32, 8 * j + i);
+    emit(chunk + j, pack8(v));
+  }
+}
+__device__ __forceinline__ float azimuth(const float *w) {
+  return atan2f(w[2], w[0]) * (0.5f / 3.14159265358979323846f) + 0.5f;
+}
+__device__ __forceinline__ float elevation(const float *w) { return w[1] * 0.5f + 0.5f; }
+template <int KB, bool FTZ, class Emit>
+__device__ __forceinline__ void encode_block(const ct_nrc_query &q, const float *bmin, const float *bext, Emit &&emit) {
+  if (KB == 0) {
+    encode_axis(q.position[0], bmin[0], bext[0], 0, emit);
+    encode_axis(q.position[1], bmin[1], bext[1], 4, emit);
+  } else if (KB == 1) {
+    encode_axis(q.position[2], bmin[2], bext[2], 8, emit);
+    encode_blob<FTZ>(azimuth(q.direction), 12, emit);
+  } else if (KB == 2) {
+    encode_blob<FTZ>(elevation(q.direction), 16, emit);
+    encode_blob<FTZ>(azimuth(q.normal), 20, emit);
+  } else {
+    encode_blob<FTZ>(elevation(q.normal), 24, emit);
+    const float v[8] = {q.albedo[0], q.albedo[1], q.albedo[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    emit(28, pack8(v));
+#pragma unroll
+    for (int ch = 29; ch < 32; ch++) emit(ch, make_uint4(0u, 0u, 0u, 0u));
+  }
+}
+
+// A warp encodes 32 queries, block by block through its own shared memory, so
+// that the rows (512 B each) leave in whole 128-byte lines: a thread storing
+// its own row sends each 16-byte chunk to a sector of its own.
+constexpr int kEncodeThreads = 128;
+__global__ void __launch_bounds__(kEncodeThreads) k_nrc_encode(const ct_nrc_query *q, uint32_t n, float3 bmin,
+                                                               float3 bext, __nv_bfloat16 *out) {
+  __shared__ uint4 s_rows[kEncodeThreads / 32][32][9];  // 8 chunks a row, padded against bank conflicts
+  const uint32_t lane = threadIdx.x & 31u, first = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;
+  uint4(*rows)[9] = s_rows[threadIdx.x >> 5];
+  if (first >= n) return;  // whole warps
   const float mn[3] = {bmin.x, bmin.y, bmin.z}, ex[3] = {bext.x, bext.y, bext.z};
-  uint4 *dst = reinterpret_cast<uint4 *>(out + 256ull * i);
-  encode_chunks(q[i], mn, ex, [&](int ch, const float *v) { dst[ch] = pack8(v); });
+  const ct_nrc_query qq = q[min(first + lane, n - 1u)];
+  const auto store = [&](int kb) {
+    __syncwarp();
+#pragma unroll
+    for (uint32_t i = 0; i < 8; i++) {
+      const uint32_t r = i * 4u + (lane >> 3), ch = lane & 7u;
+      if (first + r < n) reinterpret_cast<uint4 *>(out + (uint64_t)(first + r) * kIn)[kb * 8 + ch] = rows[r][ch];
+    }
+    __syncwarp();
+  };
+  const auto put = [&](int ch, uint4 v) { rows[lane][ch & 7] = v; };
+  encode_block<0, false>(qq, mn, ex, put);
+  store(0);
+  encode_block<1, false>(qq, mn, ex, put);
+  store(1);
+  encode_block<2, false>(qq, mn, ex, put);
+  store(2);
+  encode_block<3, false>(qq, mn, ex, put);
+  store(3);
 }
 
-// warpgroup g's named barrier (ids 1 and 2; 0 is __syncthreads), and the
-// same barrier with a vote: true when every thread's `v` is true
+// warpgroup g's named barrier (ids 1 to kGroups; 0 is __syncthreads)
 __device__ __forceinline__ void group_sync(uint32_t g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1u) : "memory"); }
-__device__ __forceinline__ bool group_all(uint32_t g, bool v) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, 128, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}\n"
-      : "=r"(r)
-      : "r"((uint32_t)v), "r"(g + 1u)
-      : "memory");
-  return r != 0;
-}
 
-// one MLP layer: D[128 x N] = A[128 x K] * W[N x K]^T, K in 64-element blocks
-__device__ __forceinline__ void layer_mma(uint32_t tmem, uint32_t a_base, uint32_t a_block_bytes, uint32_t w_base,
-                                          uint32_t w_block_bytes, int k_blocks, uint32_t idesc, uint32_t bar) {
+// a block of an MLP layer: D[128 x N] (+)= A[128 x 64] * W[N x 64]^T
+__device__ __forceinline__ void block_mma(uint32_t tmem, uint32_t a_base, uint32_t w_base, uint32_t idesc,
+                                          bool accumulate, uint32_t bar) {
   fence_after();
-  for (int kb = 0; kb < k_blocks; kb++)
-    for (int j = 0; j < 4; j++)
-      mma(tmem, smem_desc(a_base + kb * a_block_bytes + j * 32), smem_desc(w_base + kb * w_block_bytes + j * 32), idesc,
-          (kb | j) != 0);
+  for (int j = 0; j < 4; j++)
+    mma(tmem, smem_desc(a_base + j * 32), smem_desc(w_base + j * 32), idesc, (accumulate || j != 0) ? 1u : 0u);
   commit(bar);
 }
 
@@ -259,7 +298,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_nrc_mlp(const ct_nrc_query *q, 
   const uint32_t base = smem_u32(smem);
   const uint32_t tid = threadIdx.x, warp = tid >> 5;
   const uint32_t g = tid >> 7, row = tid & (kTile - 1);  // warpgroup, and this thread's row of its tile
-  uint32_t *tmem_slot = (uint32_t *)(smem + kSmemBar + 8 * kGroups);
+  uint32_t *tmem_slot = (uint32_t *)(smem + kSmemTmem);
+  volatile uint32_t *fail = (volatile uint32_t *)(smem + kSmemFail) + g;
 
   // weights into their swizzled regions (16-byte chunks)
   for (uint32_t i = tid; i < (uint32_t)(kWidth * (kIn / 8)); i += kThreads) {  // W0: 64 rows x 32 chunks
@@ -278,96 +318,138 @@ __global__ void __launch_bounds__(kThreads, 1) k_nrc_mlp(const ct_nrc_query *q, 
     *reinterpret_cast<uint4 *>(smem + kSmemW5 + sw128(r, ch)) = v;
   }
   if (tid == 0) {
-    for (uint32_t k = 0; k < (uint32_t)kGroups; k++)
+    for (uint32_t k = 0; k < 2u * kGroups; k++)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(base + kSmemBar + 8u * k) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (row == 0) *fail = 0u;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(kTmemCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  fence_async_smem();
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem = tmem_base + 64u * g;                      // this warpgroup's accumulator columns
   const uint32_t lane_addr = tmem + (((warp & 3u) * 32u) << 16);  // a warp reads TMEM lanes 32 (warp % 4) + 0..31
-  const uint32_t bar = base + kSmemBar + 8u * g;
-  const uint32_t a_off = kSmemA + g * kABytes;
+  const uint32_t bar0 = base + kSmemBar + 16u * g, bar1 = bar0 + 8u;
+  const uint32_t buf0 = kSmemA + g * 2u * kBufBytes, buf1 = buf0 + kBufBytes;
   const float mn[3] = {bmin.x, bmin.y, bmin.z}, ex[3] = {bext.x, bext.y, bext.z};
-  uint32_t parity = 0;
-  const uint32_t tiles = (n + kTile - 1) / kTile;
-  for (uint32_t tile = blockIdx.x * kGroups + g; tile < tiles; tile += gridDim.x * kGroups) {
-    const uint32_t qi = tile * kTile + row;
-    // layer-0 input tile
-    const auto put = [&](int ch, const float *v) {
-      *reinterpret_cast<uint4 *>(smem + a_off + (ch >> 3) * 16384u + sw128(row, ch & 7u)) = pack8(v);
-    };
-    if (ENCODE) {
-      if (qi < n) {
-        encode_chunks(q[qi], mn, ex, put);
-      } else {
-        for (uint32_t ch = 0; ch < 32; ch++)
-          *reinterpret_cast<uint4 *>(smem + a_off + (ch >> 3) * 16384u + sw128(row, ch & 7u)) = make_uint4(0, 0, 0, 0);
-      }
-    } else {
-      for (uint32_t ch = 0; ch < 32; ch++) {
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (qi < n) v = *reinterpret_cast<const uint4 *>(encoded + (uint64_t)qi * kIn + ch * 8u);
-        *reinterpret_cast<uint4 *>(smem + a_off + (ch >> 3) * 16384u + sw128(row, ch & 7u)) = v;
-      }
-    }
-    bool ok = true;
-    for (int layer = 0; layer <= kHidden; layer++) {
-      fence_async_smem();
-      fence_before();
-      group_sync(g);
-      const bool last = layer == kHidden;
-      if (row == 0) {
-        if (layer == 0)
-          layer_mma(tmem, base + a_off, 16384u, base + kSmemW0, 8192u, 4, instr_desc(128, kWidth), bar);
-        else if (!last)
-          layer_mma(tmem, base + a_off, 16384u, base + kSmemWh + (layer - 1) * 8192u, 8192u, 1,
-                    instr_desc(128, kWidth), bar);
-        else
-          layer_mma(tmem, base + a_off, 16384u, base + kSmemW5, 2048u, 1, instr_desc(128, kOut), bar);
-      }
-      // the warpgroup's threads leave together when any wait ran out
-      if (!group_all(g, wait_bar(bar, parity))) {
-        ok = false;
-        if (row == 0) atomicCAS(&g_nrc_status, 0u, 1u);
-        break;
-      }
-      parity ^= 1u;
-      fence_after();
-      if (!last) {
-        // ReLU, bf16, next layer's input tile (the first K-block of the warpgroup's tile)
-        for (uint32_t c0 = 0; c0 < (uint32_t)kWidth; c0 += 16) {
-          float v[16];
-          tmem_ld16(lane_addr + c0, v);
-#pragma unroll
-          for (int k = 0; k < 16; k++) v[k] = fmaxf(v[k], 0.0f);
-          *reinterpret_cast<uint4 *>(smem + a_off + sw128(row, c0 >> 3)) = pack8(v);
-          *reinterpret_cast<uint4 *>(smem + a_off + sw128(row, (c0 >> 3) + 1)) = pack8(v + 8);
-        }
-      } else {
-        float v[16];
-        tmem_ld16(lane_addr, v);
-        if (qi < n) {
-          rgb[3ull * qi] = v[0];
-          rgb[3ull * qi + 1] = v[1];
-          rgb[3ull * qi + 2] = v[2];
-        }
-      }
-    }
-    if (!ok) break;
-    // the next tile's encoding overwrites the input tile: every thread of the
-    // warpgroup has read its accumulator rows (tcgen05.wait::ld) by now
+  uint32_t par0 = 0, par1 = 0;  // phase each mbarrier is in
+  // a wait that ran out shows at the warpgroup's next barrier
+  const auto wait0 = [&]() {
+    if (!wait_bar(bar0, par0)) *fail = 1u;
+    par0 ^= 1u;
+    __syncwarp();  // tcgen05.ld is a warp's
+  };
+  const auto wait1 = [&]() {
+    if (!wait_bar(bar1, par1)) *fail = 1u;
+    par1 ^= 1u;
+    __syncwarp();
+  };
+  // the warpgroup's writes to its buffers are complete and visible to the
+  // MMAs; false when it has given up
+  const auto ready = [&]() {
+    fence_async_smem();
     fence_before();
     group_sync(g);
+    return *fail == 0u;
+  };
+  const uint32_t tiles = (n + kTile - 1) / kTile;
+  // tiles in turn over the CTAs' first warpgroups, then their second ones, ...:
+  // a few tiles spread over the SMs
+  for (uint32_t tile = g * gridDim.x + blockIdx.x; tile < tiles; tile += gridDim.x * kGroups) {
+    const uint32_t qi = tile * kTile + row;
+    ct_nrc_query qq;
+    if (ENCODE) qq = q[min(qi, n - 1u)];  // rows past the end repeat the last query; their results are not stored
+    const auto fill = [&](auto kb_c, uint32_t buf) {
+      constexpr int kb = decltype(kb_c)::value;
+      if (ENCODE) {
+        encode_block<kb, true>(qq, mn, ex, [&](int ch, uint4 v) {
+          *reinterpret_cast<uint4 *>(smem + buf + sw128(row, (uint32_t)ch & 7u)) = v;
+        });
+      } else {
+        // 8 threads per row: whole 128-byte lines of the encoded rows
+#pragma unroll
+        for (uint32_t i = 0; i < 8; i++) {
+          const uint32_t r = i * 16u + (row >> 3), ch = row & 7u, at = tile * kTile + r;
+          uint4 v = make_uint4(0, 0, 0, 0);
+          if (at < n) v = *reinterpret_cast<const uint4 *>(encoded + (uint64_t)at * kIn + kb * kBlockK + ch * 8u);
+          *reinterpret_cast<uint4 *>(smem + buf + sw128(r, ch)) = v;
+        }
+      }
+    };
+    const auto start = [&](int kb, uint32_t buf, uint32_t bar) {
+      if (row == 0) block_mma(tmem, base + buf, base + kSmemW0 + kb * 8192u, instr_desc(128, kWidth), kb != 0, bar);
+    };
+    fill(std::integral_constant<int, 0>{}, buf0);
+    if (!ready()) break;
+    start(0, buf0, bar0);
+    fill(std::integral_constant<int, 1>{}, buf1);
+    if (!ready()) break;
+    start(1, buf1, bar1);
+    wait0();
+    fill(std::integral_constant<int, 2>{}, buf0);
+    if (!ready()) break;
+    start(2, buf0, bar0);
+    wait1();
+    fill(std::integral_constant<int, 3>{}, buf1);
+    if (!ready()) break;
+    start(3, buf1, bar1);
+    wait0();
+    wait1();
+    bool ok = true;
+    for (int layer = 1; layer <= kHidden; layer++) {
+      fence_after();
+      // round to bf16 and ReLU (which commute) into the first buffer
+#pragma unroll
+      for (uint32_t c0 = 0; c0 < (uint32_t)kWidth; c0 += 32) {
+        uint32_t r[32];
+        tmem_ld16(lane_addr + c0, r);
+        tmem_ld16(lane_addr + c0 + 16, r + 16);
+        tmem_wait16(r);
+        tmem_wait16(r + 16);
+#pragma unroll
+        for (int k = 0; k < 32; k += 8) {
+          uint32_t h[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[k + 2 * j]), __uint_as_float(r[k + 2 * j + 1]));
+            const __nv_bfloat162 m = __hmax2(v, __nv_bfloat162(__ushort_as_bfloat16(0), __ushort_as_bfloat16(0)));
+            h[j] = *reinterpret_cast<const uint32_t *>(&m);
+          }
+          *reinterpret_cast<uint4 *>(smem + buf0 + sw128(row, (c0 + k) >> 3)) = make_uint4(h[0], h[1], h[2], h[3]);
+        }
+      }
+      if (!ready()) {
+        ok = false;
+        break;
+      }
+      if (row == 0) {
+        const bool last = layer == kHidden;
+        block_mma(tmem, base + buf0, base + (last ? kSmemW5 : kSmemWh + (layer - 1) * 8192u),
+                  last ? instr_desc(128, kOut) : instr_desc(128, kWidth), false, bar0);
+      }
+      wait0();
+    }
+    if (!ok) break;
+    fence_after();
+    uint32_t r[16];
+    tmem_ld16(lane_addr, r);
+    tmem_wait16(r);
+    if (qi < n) {
+      rgb[3ull * qi] = __uint_as_float(r[0]);
+      rgb[3ull * qi + 1] = __uint_as_float(r[1]);
+      rgb[3ull * qi + 2] = __uint_as_float(r[2]);
+    }
+    // the next tile's first barrier orders these tensor-memory reads before
+    // the MMAs that overwrite the columns
   }
+  if (*fail != 0u && row == 0) atomicCAS(&g_nrc_status, 0u, 1u);
   // every tensor-memory read of this CTA is complete (tcgen05.wait::ld)
   fence_before();
   __syncthreads();
@@ -400,8 +482,8 @@ static int nrc_grid(uint32_t n) {
     cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
     sms = v > 0 ? v : 148;
   }
-  const uint32_t pairs = (n + 2u * ct_nrc::kTile - 1) / (2u * ct_nrc::kTile);  // a tile per warpgroup
-  return (int)(pairs < (uint32_t)sms ? pairs : (uint32_t)sms);
+  const uint32_t tiles = (uint32_t)(((uint64_t)n + ct_nrc::kTile - 1) / ct_nrc::kTile);
+  return (int)(tiles < (uint32_t)sms ? tiles : (uint32_t)sms);
 }
 
 static cudaError_t launch_mlp(bool encode, const ct_nrc_net *net, const ct_nrc_query *q, const void *encoded,
@@ -440,7 +522,7 @@ extern "C" ct_status ct_nrc_encode(const ct_nrc_net *net, const ct_nrc_query *qu
   const float3 bext = make_float3(net->bbox_extent[0], net->bbox_extent[1], net->bbox_extent[2]);
   cudaStream_t s = (cudaStream_t)stream;
   CT_TIMED(CT_K_NRC_ENCODE, s,
-           ct_nrc::k_nrc_encode<<<(n + 255) / 256, 256, 0, s>>>(queries, n, bmin, bext, (__nv_bfloat16 *)encoded));
+           ct_nrc::k_nrc_encode<<<(n + ct_nrc::kEncodeThreads - 1) / ct_nrc::kEncodeThreads, ct_nrc::kEncodeThreads, 0, s>>>(queries, n, bmin, bext, (__nv_bfloat16 *)encoded));
   return nrc_status(cudaGetLastError());
 }
 
