@@ -10,23 +10,25 @@
 // next layer reads it.
 //
 // One CTA of 512 threads per SM: four warpgroups, each walking its own tiles
-// of 128 queries with two 16 KB input buffers (64 of the 256 inputs each), its
-// own 64 tensor-memory columns and two mbarriers, so that the warpgroups'
-// encodings, epilogues and MMAs overlap.  The weights (66 KB) are shared; with
-// the buffers the CTA holds 194 KB.  Per tile:
-//  * every thread encodes its query into the buffers (row = thread), K-major
-//    in 128-byte-swizzled atoms of 8 rows x 64 bf16, one block of 64 inputs
-//    after the other; the block's MMAs run while the next one is encoded;
+// of 128 queries with two 16 KB buffers, 128 tensor-memory columns and two
+// mbarriers of its own.  The weights (66 KB) are shared; with the buffers the
+// CTA holds 194 KB.  Per tile:
+//  * every thread encodes its query (row = thread), K-major in
+//    128-byte-swizzled atoms of 8 rows x 64 bf16, one block of 64 of the 256
+//    inputs at a time in one buffer, while the MMAs of the previous tile's
+//    layers run on the other;
 //  * one thread of the warpgroup issues tcgen05.mma (M 128, N 64, K 16 per
 //    instruction, bf16 inputs, fp32 accumulator) and commits to the buffer's
 //    mbarrier;
 //  * every warp reads its 32 TMEM lanes (tcgen05.ld 32x32b), rounds to bf16,
-//    applies ReLU and writes the next layer's input into the first buffer;
+//    applies ReLU and writes the next layer's input;
 //  * the last layer (N 16) writes RGB to global memory.
 // What bounds it is instruction issue: the encoding's 48 sincospi and 128
 // exponentials and the epilogues are some 3000 instructions per query against
-// 42 kFLOP of MMAs.  With whole 64 KB tiles only two warpgroups fitted (8
-// warps per SM, issue 44% active): 2.07 M queries took 573 us.
+// 42 kFLOP of MMAs, at 4 warps per scheduler (issue 59% active): 2.07 M queries
+// take 341 us.  Whole 64 KB tiles let only two warpgroups in (issue 44%, 573
+// us); encoding a tile before its layers instead of during the previous
+// tile's took 353 us, one barrier for a layer and a block 357 us.
 // Warpgroups synchronise on their own named barriers.  Operands are staged
 // with ordinary 16-byte shared stores (no TMA).  Every wait is bounded
 // (about one second); a warpgroup that gives up latches an error in the
@@ -48,7 +50,7 @@ constexpr int kOut = CT_NRC_OUTPUT_DIMS;   // 16
 constexpr int kHidden = CT_NRC_HIDDEN_LAYERS;  // 5
 constexpr int kGroups = 4;                    // warpgroups per CTA, one tile each
 constexpr int kThreads = kTile * kGroups;     // 512
-constexpr int kTmemCols = 64 * kGroups;       // 64 accumulator columns per warpgroup
+constexpr int kTmemCols = 128 * kGroups;      // two tiles' 64 accumulator columns per warpgroup
 constexpr int kBlockK = 64;                   // inputs per buffer
 static_assert(kIn == 4 * kBlockK, "blocks of the first layer");
 
@@ -334,8 +336,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_nrc_mlp(const ct_nrc_query *q, 
   __syncthreads();
   fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem = tmem_base + 64u * g;                      // this warpgroup's accumulator columns
-  const uint32_t lane_addr = tmem + (((warp & 3u) * 32u) << 16);  // a warp reads TMEM lanes 32 (warp % 4) + 0..31
+  const uint32_t tmem = tmem_base + 128u * g;              // this warpgroup's accumulator columns, two tiles'
+  const uint32_t lane_bits = ((warp & 3u) * 32u) << 16;    // a warp reads TMEM lanes 32 (warp % 4) + 0..31
   const uint32_t bar0 = base + kSmemBar + 16u * g, bar1 = bar0 + 8u;
   const uint32_t buf0 = kSmemA + g * 2u * kBufBytes, buf1 = buf0 + kBufBytes;
   const float mn[3] = {bmin.x, bmin.y, bmin.z}, ex[3] = {bext.x, bext.y, bext.z};
@@ -361,56 +363,46 @@ __global__ void __launch_bounds__(kThreads, 1) k_nrc_mlp(const ct_nrc_query *q, 
   };
   const uint32_t tiles = (n + kTile - 1) / kTile;
   // tiles in turn over the CTAs' first warpgroups, then their second ones, ...:
-  // a few tiles spread over the SMs
-  for (uint32_t tile = g * gridDim.x + blockIdx.x; tile < tiles; tile += gridDim.x * kGroups) {
-    const uint32_t qi = tile * kTile + row;
-    ct_nrc_query qq;
-    if (ENCODE) qq = q[min(qi, n - 1u)];  // rows past the end repeat the last query; their results are not stored
-    const auto fill = [&](auto kb_c, uint32_t buf) {
+  // a few tiles spread over the SMs.  A warpgroup runs the hidden layers of
+  // tile `cur` (activations in buffer 0) and the first layer of tile `next`
+  // (a block of inputs at a time in buffer 1) in turn, so that it encodes while
+  // a layer's MMAs run.  The two tiles' accumulators alternate.
+  const uint32_t stride = gridDim.x * kGroups;
+  uint32_t cur = 0, next = g * gridDim.x + blockIdx.x;
+  uint32_t acc = 0;  // columns of tile `cur`: 64 acc
+  bool have = false, ok = true;
+  ct_nrc_query qq;
+  while (ok && (have || next < tiles)) {
+    const bool feed = next < tiles;
+    const uint32_t t_cur = tmem + 64u * acc, t_next = tmem + 64u * (acc ^ 1u);
+    // rows past the end repeat the last query; their results are not stored
+    if (ENCODE && feed) qq = q[min(next * kTile + row, n - 1u)];
+    const auto fill = [&](auto kb_c) {
       constexpr int kb = decltype(kb_c)::value;
       if (ENCODE) {
         encode_block<kb, true>(qq, mn, ex, [&](int ch, uint4 v) {
-          *reinterpret_cast<uint4 *>(smem + buf + sw128(row, (uint32_t)ch & 7u)) = v;
+          *reinterpret_cast<uint4 *>(smem + buf1 + sw128(row, (uint32_t)ch & 7u)) = v;
         });
       } else {
         // 8 threads per row: whole 128-byte lines of the encoded rows
 #pragma unroll
         for (uint32_t i = 0; i < 8; i++) {
-          const uint32_t r = i * 16u + (row >> 3), ch = row & 7u, at = tile * kTile + r;
+          const uint32_t r = i * 16u + (row >> 3), ch = row & 7u, at = next * kTile + r;
           uint4 v = make_uint4(0, 0, 0, 0);
           if (at < n) v = *reinterpret_cast<const uint4 *>(encoded + (uint64_t)at * kIn + kb * kBlockK + ch * 8u);
-          *reinterpret_cast<uint4 *>(smem + buf + sw128(r, ch)) = v;
+          *reinterpret_cast<uint4 *>(smem + buf1 + sw128(r, ch)) = v;
         }
       }
     };
-    const auto start = [&](int kb, uint32_t buf, uint32_t bar) {
-      if (row == 0) block_mma(tmem, base + buf, base + kSmemW0 + kb * 8192u, instr_desc(128, kWidth), kb != 0, bar);
-    };
-    fill(std::integral_constant<int, 0>{}, buf0);
-    if (!ready()) break;
-    start(0, buf0, bar0);
-    fill(std::integral_constant<int, 1>{}, buf1);
-    if (!ready()) break;
-    start(1, buf1, bar1);
-    wait0();
-    fill(std::integral_constant<int, 2>{}, buf0);
-    if (!ready()) break;
-    start(2, buf0, bar0);
-    wait1();
-    fill(std::integral_constant<int, 3>{}, buf1);
-    if (!ready()) break;
-    start(3, buf1, bar1);
-    wait0();
-    wait1();
-    bool ok = true;
-    for (int layer = 1; layer <= kHidden; layer++) {
+    // hidden layer (or output) `layer` of cur: the accumulator, rounded to
+    // bf16, then ReLU (which commutes), into buffer 0, and the layer's MMAs
+    const auto layer_begin = [&](int layer) {
       fence_after();
-      // round to bf16 and ReLU (which commute) into the first buffer
 #pragma unroll
       for (uint32_t c0 = 0; c0 < (uint32_t)kWidth; c0 += 32) {
         uint32_t r[32];
-        tmem_ld16(lane_addr + c0, r);
-        tmem_ld16(lane_addr + c0 + 16, r + 16);
+        tmem_ld16(t_cur + lane_bits + c0, r);
+        tmem_ld16(t_cur + lane_bits + c0 + 16, r + 16);
         tmem_wait16(r);
         tmem_wait16(r + 16);
 #pragma unroll
@@ -425,29 +417,56 @@ __global__ void __launch_bounds__(kThreads, 1) k_nrc_mlp(const ct_nrc_query *q, 
           *reinterpret_cast<uint4 *>(smem + buf0 + sw128(row, (c0 + k) >> 3)) = make_uint4(h[0], h[1], h[2], h[3]);
         }
       }
-      if (!ready()) {
-        ok = false;
-        break;
-      }
+      if (!ready()) return false;
       if (row == 0) {
         const bool last = layer == kHidden;
-        block_mma(tmem, base + buf0, base + (last ? kSmemW5 : kSmemWh + (layer - 1) * 8192u),
+        block_mma(t_cur, base + buf0, base + (last ? kSmemW5 : kSmemWh + (layer - 1) * 8192u),
                   last ? instr_desc(128, kOut) : instr_desc(128, kWidth), false, bar0);
       }
-      wait0();
+      return true;
+    };
+    // block kb of next's inputs and its MMAs
+    const auto feed_block = [&](auto kb_c) {
+      constexpr int kb = decltype(kb_c)::value;
+      if (kb > 0) wait1();
+      fill(kb_c);
+      if (!ready()) return false;
+      if (row == 0)
+        block_mma(t_next, base + buf1, base + kSmemW0 + kb * 8192u, instr_desc(128, kWidth), kb != 0, bar1);
+      return true;
+    };
+    const auto step = [&](int layer, auto kb_c) {
+      if (ok && have) ok = layer_begin(layer);
+      if (ok && feed) ok = feed_block(kb_c);
+      if (ok && have) wait0();
+    };
+    step(1, std::integral_constant<int, 0>{});
+    step(2, std::integral_constant<int, 1>{});
+    step(3, std::integral_constant<int, 2>{});
+    step(4, std::integral_constant<int, 3>{});
+    if (ok && have) {
+      ok = layer_begin(kHidden);
+      if (ok) wait0();
     }
-    if (!ok) break;
-    fence_after();
-    uint32_t r[16];
-    tmem_ld16(lane_addr, r);
-    tmem_wait16(r);
-    if (qi < n) {
-      rgb[3ull * qi] = __uint_as_float(r[0]);
-      rgb[3ull * qi + 1] = __uint_as_float(r[1]);
-      rgb[3ull * qi + 2] = __uint_as_float(r[2]);
+    if (ok && have) {
+      fence_after();
+      uint32_t r[16];
+      tmem_ld16(t_cur + lane_bits, r);
+      tmem_wait16(r);
+      const uint32_t qi = cur * kTile + row;
+      if (qi < n) {
+        rgb[3ull * qi] = __uint_as_float(r[0]);
+        rgb[3ull * qi + 1] = __uint_as_float(r[1]);
+        rgb[3ull * qi + 2] = __uint_as_float(r[2]);
+      }
+      // the next barrier orders these tensor-memory reads before the MMAs that
+      // overwrite the columns
     }
-    // the next tile's first barrier orders these tensor-memory reads before
-    // the MMAs that overwrite the columns
+    if (ok && feed) wait1();
+    have = feed;
+    cur = next;
+    next += stride;
+    acc ^= 1u;
   }
   if (*fail != 0u && row == 0) atomicCAS(&g_nrc_status, 0u, 1u);
   // every tensor-memory read of this CTA is complete (tcgen05.wait::ld)
