@@ -279,6 +279,79 @@ __global__ void __launch_bounds__(kEncodeThreads) k_nrc_encode(const ct_nrc_quer
   store(3);
 }
 
+// The encoding in single precision, for the training of the fp32 network
+// (float[n][256]): the values, and bit for bit the roundings, of the torch
+// expressions in cube_tracing/nrc.py (encode), which took some 45 launches.
+// One thread per 4 consecutive values, so that a warp stores 512 contiguous
+// bytes of a row; the warps of a row's two halves take one kind of value each.
+__device__ __forceinline__ float4 encode_f32_freq(float p, float bmin, float bext, int band) {
+  float x = (p - bmin) / bext;
+  if (!isnan(x)) x = fminf(fmaxf(x, 0.0f), 1.0f);  // torch's clamp keeps a NaN
+  float v[4];
+#pragma unroll
+  for (int b = 0; b < 2; b++) {
+    const float t = fmodf(x * (float)(1u << (band + b)), 2.0f);
+    const float a = 3.14159265358979323846f * t;
+    v[2 * b] = sinf(a);
+    v[2 * b + 1] = cosf(a);
+  }
+  return make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ float4 encode_f32_blob(float u, int bin) {
+  float v[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const float d = (u - ((float)(bin + i) + 0.5f) / 32.0f) * 32.0f;
+    v[i] = expf(-0.5f * d * d);
+  }
+  return make_float4(v[0], v[1], v[2], v[3]);
+}
+__global__ void __launch_bounds__(256) k_nrc_encode_f32(const ct_nrc_query *q, uint32_t n, float3 bmin, float3 bext,
+                                                        float4 *out) {
+  const uint64_t at = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = (uint32_t)(at >> 6), c = (uint32_t)(at & 63u);  // row, group of 4 values
+  if (i >= n) return;
+  const ct_nrc_query &r = q[i];
+  float4 v;
+  if (c < 24u) {
+    const uint32_t a = c >> 3;  // axis: 8 groups of 2 bands
+    const float mn = a == 0 ? bmin.x : (a == 1 ? bmin.y : bmin.z), ex = a == 0 ? bext.x : (a == 1 ? bext.y : bext.z);
+    v = encode_f32_freq(r.position[a], mn, ex, 2 * (int)(c & 7u));
+  } else if (c < 56u) {
+    const uint32_t k = (c - 24u) >> 3;  // direction's two angles, then the normal's: 8 groups of 4 bins
+    const float *w = k < 2u ? r.direction : r.normal;
+    const float u = (k & 1u) ? w[1] * 0.5f + 0.5f : atan2f(w[2], w[0]) * (0.5f / 3.14159265358979323846f) + 0.5f;
+    v = encode_f32_blob(u, 4 * (int)((c - 24u) & 7u));
+  } else {
+    v = c == 56u ? make_float4(r.albedo[0], r.albedo[1], r.albedo[2], 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  out[at] = v;
+}
+
+// The training loss's elementwise part and its gradient: per row and channel
+//   rel = (pred - target)^2 / (pred^2 + 0.01),   terms = rel w,
+//   grad = (((1 / total) w) / (pred^2 + 0.01)) (2 (pred - target))
+// in the operation order of the torch expressions and their autograd (15
+// launches): the caller sums `terms` and divides by `total`.  pred and grad
+// are rows of 16 (the network's outputs; channels 3 to 15 have no gradient).
+__global__ void __launch_bounds__(256) k_nrc_loss(const float *pred, const float *target, const float *weight,
+                                                  const float *total, uint32_t n, float *terms, float4 *grad) {
+  const uint64_t at = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = (uint32_t)(at >> 2);  // a row's four groups of 4 outputs
+  if (i >= n) return;
+  float g[4] = {0.f, 0.f, 0.f, 0.f};
+  if ((at & 3u) == 0u) {
+    const float w = weight[i], s = (1.0f / *total) * w;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const float p = pred[16ull * i + c], d = p - target[3ull * i + c], den = p * p + 0.01f;
+      terms[3ull * i + c] = (d * d) / den * w;
+      g[c] = s / den * (2.0f * d);
+    }
+  }
+  grad[at] = make_float4(g[0], g[1], g[2], g[3]);
+}
+
 // warpgroup g's named barrier (ids 1 to kGroups; 0 is __syncthreads)
 __device__ __forceinline__ void group_sync(uint32_t g) { asm volatile("bar.sync %0, 128;" ::"r"(g + 1u) : "memory"); }
 
@@ -542,6 +615,30 @@ extern "C" ct_status ct_nrc_encode(const ct_nrc_net *net, const ct_nrc_query *qu
   cudaStream_t s = (cudaStream_t)stream;
   CT_TIMED(CT_K_NRC_ENCODE, s,
            ct_nrc::k_nrc_encode<<<(n + ct_nrc::kEncodeThreads - 1) / ct_nrc::kEncodeThreads, ct_nrc::kEncodeThreads, 0, s>>>(queries, n, bmin, bext, (__nv_bfloat16 *)encoded));
+  return nrc_status(cudaGetLastError());
+}
+
+extern "C" ct_status ct_nrc_encode_f32(const ct_nrc_net *net, const ct_nrc_query *queries, uint32_t n, float *encoded,
+                                       ct_stream stream) {
+  ct_status st = check_net(net);
+  if (st != CT_OK) return st;
+  if (n == 0) return CT_OK;
+  if (!queries || !encoded || ((uintptr_t)encoded & 15u)) return CT_ERR_INVALID_ARG;
+  if (n > 1u << 24) return CT_ERR_CAPACITY;
+  const float3 bmin = make_float3(net->bbox_min[0], net->bbox_min[1], net->bbox_min[2]);
+  const float3 bext = make_float3(net->bbox_extent[0], net->bbox_extent[1], net->bbox_extent[2]);
+  cudaStream_t s = (cudaStream_t)stream;
+  CT_TIMED(CT_K_NRC_ENCODE, s, ct_nrc::k_nrc_encode_f32<<<(n + 3u) / 4u, 256, 0, s>>>(queries, n, bmin, bext, (float4 *)encoded));
+  return nrc_status(cudaGetLastError());
+}
+
+extern "C" ct_status ct_nrc_loss(const float *pred, const float *target, const float *weight, const float *total,
+                                 uint32_t n, float *terms, float *grad, ct_stream stream) {
+  if (n == 0) return CT_OK;
+  if (!pred || !target || !weight || !total || !terms || !grad || ((uintptr_t)grad & 15u)) return CT_ERR_INVALID_ARG;
+  if (n > 1u << 24) return CT_ERR_CAPACITY;
+  cudaStream_t s = (cudaStream_t)stream;
+  CT_TIMED(CT_K_NRC_LOSS, s, ct_nrc::k_nrc_loss<<<(n + 63u) / 64u, 256, 0, s>>>(pred, target, weight, total, n, terms, (float4 *)grad));
   return nrc_status(cudaGetLastError());
 }
 

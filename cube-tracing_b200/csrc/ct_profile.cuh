@@ -30,6 +30,7 @@ enum CtKernelId {
   CT_K_NRC_ENCODE,
   CT_K_NRC_MLP,
   CT_K_NRC_TRACE,
+  CT_K_NRC_LOSS,
   CT_K_COUNT
 };
 

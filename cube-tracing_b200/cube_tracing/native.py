@@ -139,6 +139,9 @@ _SIGS = {
                                        ctypes.c_void_p]),
     "ct_nrc_encode": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint32, ctypes.c_void_p,
                                      ctypes.c_void_p]),
+    "ct_nrc_encode_f32": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint32, ctypes.c_void_p,
+                                     ctypes.c_void_p]),
+    "ct_nrc_loss": (ctypes.c_int, [ctypes.c_void_p] * 4 + [ctypes.c_uint32] + [ctypes.c_void_p] * 3),
     "ct_nrc_infer": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint32, ctypes.c_void_p,
                                     ctypes.c_void_p]),
     "ct_nrc_infer_encoded": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint32, ctypes.c_void_p,

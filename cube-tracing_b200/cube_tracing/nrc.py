@@ -111,6 +111,11 @@ class NrcCache:
         self.bbox_extent = [float(v) for v in bbox_extent]
         self.weights = torch.zeros(WEIGHT_COUNT, dtype=torch.bfloat16, device=device)
         self.export()
+        if torch.device(device).type == "cuda":
+            # a training step's backward begins with a matrix product: let
+            # autograd's thread for the device make its context current here,
+            # which cuBLAS would warn about doing itself
+            torch.zeros(1, device=device, requires_grad=True).neg().backward()
 
     def export(self):
         self.weights.copy_(self.mlp.packed())
@@ -156,20 +161,48 @@ class NrcCache:
                                                                  enc.data_ptr(), self._stream()))
         return enc
 
+    def _encode_fp32(self, queries):
+        """encode() by one kernel, with the same roundings."""
+        queries = queries.contiguous()
+        n = queries.shape[0]
+        enc = torch.empty((n, IN), dtype=torch.float32, device=queries.device)
+        net = self.net()
+        native.check("ct_nrc_encode_f32", native.lib().ct_nrc_encode_f32(
+            ctypes.byref(net), queries.data_ptr(), n, enc.data_ptr(), self._stream()))
+        return enc
+
     def train_step(self, queries, targets, weights=None):
         """One Adam step on the relative L2 loss of the cache's RGB against
         `targets` (n, 3), each query weighted by `weights` (n,) if given;
         the bf16 export follows.  Returns the loss as a device scalar (no
         host synchronisation)."""
-        enc = encode(queries, self.bbox_min, self.bbox_extent)
-        pred = self.mlp(enc)[:, :3]
-        rel = ((pred - targets) ** 2) / (pred.detach() ** 2 + 1e-2)
-        if weights is None:
-            loss = rel.mean()
-        else:
-            loss = (rel * weights[:, None]).sum() / (3.0 * weights.sum()).clamp(min=1.0)
+        # rows the library's kernels take: plain fp32 values on this device
+        # that the caller does not want gradients of
+        plain = [queries, targets] + ([weights] if weights is not None else [])
+        plain = all(t.is_cuda and t.dtype == torch.float32 and not t.requires_grad for t in plain)
+        n = queries.shape[0]
+        plain = plain and 0 < n <= 1 << 24 and queries.shape == (n, QUERY_FLOATS)
+        enc = self._encode_fp32(queries) if plain else encode(queries, self.bbox_min, self.bbox_extent)
+        out = self.mlp(enc)
         self.opt.zero_grad()
-        loss.backward()
+        if plain and targets.shape == (n, 3) and weights is not None and weights.shape == (n,) and \
+                out.dtype == torch.float32 and out.shape == (n, OUT):
+            # the loss below and its gradient in one kernel
+            total = (3.0 * weights.sum()).clamp(min=1.0)
+            terms, grad = torch.empty_like(targets, memory_format=torch.contiguous_format), torch.empty_like(out)
+            rows = [out.detach().contiguous(), targets.contiguous(), weights.contiguous(), total]
+            native.check("ct_nrc_loss", native.lib().ct_nrc_loss(
+                *[t.data_ptr() for t in rows], n, terms.data_ptr(), grad.data_ptr(), self._stream()))
+            loss = terms.sum() / total
+            out.backward(grad)
+        else:
+            pred = out[:, :3]
+            rel = ((pred - targets) ** 2) / (pred.detach() ** 2 + 1e-2)
+            if weights is None:
+                loss = rel.mean()
+            else:
+                loss = (rel * weights[:, None]).sum() / (3.0 * weights.sum()).clamp(min=1.0)
+            loss.backward()
         self.opt.step()
         self.export()
         return loss.detach()

@@ -609,6 +609,21 @@ typedef struct ct_nrc_net {
   float bbox_extent[3];            /* > 0 */
 } ct_nrc_net;
 ct_status ct_nrc_encode(const ct_nrc_net *net, const ct_nrc_query *queries, uint32_t n, void *encoded, ct_stream stream);
+/* The same encoding in single precision, float[n][256] (16-byte aligned), for
+ * training the fp32 network: sin, cos, exp and atan2 of pi t, -((u - (i +
+ * 1/2) / 32) 32)^2 / 2 and v as their single-precision functions give them.
+ * n up to 2^24. */
+ct_status ct_nrc_encode_f32(const ct_nrc_net *net, const ct_nrc_query *queries, uint32_t n, float *encoded,
+                            ct_stream stream);
+/* The elementwise part of the cache's training loss and its gradient: pred
+ * float[n][16] (the network's outputs), target float[n][3], weight float[n],
+ * total one float (the loss's divisor); per channel c < 3, with d = pred -
+ * target and e = pred^2 + 0.01, terms float[n][3] = d^2 / e * weight and
+ * grad float[n][16] (16-byte aligned) = (1 / total) * weight / e * (2 d), 0 in
+ * the other channels.  The loss is sum(terms) / total.  All in device memory;
+ * n up to 2^24. */
+ct_status ct_nrc_loss(const float *pred, const float *target, const float *weight, const float *total, uint32_t n,
+                      float *terms, float *grad, ct_stream stream);
 ct_status ct_nrc_infer(const ct_nrc_net *net, const ct_nrc_query *queries, uint32_t n, float *rgb, ct_stream stream);
 ct_status ct_nrc_infer_encoded(const ct_nrc_net *net, const void *encoded, uint32_t n, float *rgb, ct_stream stream);
 ct_status ct_nrc_status(int reset, uint32_t *out);
