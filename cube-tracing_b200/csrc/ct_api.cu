@@ -227,7 +227,7 @@ extern "C" ct_status ct_trace_frame(const ct_push_constant *pc, const ct_params 
   return cuda_status(ct_launch_trace(*pc, walk_accel(pc->tlas, P), *P, (cudaStream_t)stream));
 }
 
-extern "C" ct_status ct_restir_di(const ct_push_constant *pc, const ct_params *P, int stage, ct_stream stream) {
+static ct_status restir_di(const ct_push_constant *pc, const ct_params *P, int stage, bool alone, ct_stream stream) {
   ct_status st = check_pc(pc, true);
   if (st == CT_OK) st = check_params(P);
   if (st == CT_OK) st = check_extent(pc, P);
@@ -238,6 +238,7 @@ extern "C" ct_status ct_restir_di(const ct_push_constant *pc, const ct_params *P
   CtWorkspace w;
   st = get_workspace(pc, P, &w);
   if (st != CT_OK) return st;
+  w.alone = alone;
   const DevAccel A_prev = pc->tlas_previous ? walk_accel(pc->tlas_previous, P) : A;
   if (stage == 0) return cuda_status(ct_launch_di_stage0(*pc, A, A_prev, *P, w, s));
   // spatial rounds: intermediate -> reservoir -> intermediate ... ; the last
@@ -251,6 +252,10 @@ extern "C" ct_status ct_restir_di(const ct_push_constant *pc, const ct_params *P
   return cuda_status(ct_launch_spatial_round(*pc, A, *P, w, P->spatial_passes - 1, (int)((P->spatial_passes - 1) & 1u), 1, 0, s));
 }
 
+extern "C" ct_status ct_restir_di(const ct_push_constant *pc, const ct_params *P, int stage, ct_stream stream) {
+  return restir_di(pc, P, stage, true, stream);
+}
+
 static ct_status restir_pt(const ct_push_constant *pc, const ct_params *P, int stage, bool alone, ct_stream stream) {
   ct_status st = check_pc(pc, true);
   if (st == CT_OK) st = check_params(P);
@@ -260,7 +265,8 @@ static ct_status restir_pt(const ct_push_constant *pc, const ct_params *P, int s
   CtWorkspace w;
   st = get_workspace(pc, P, &w);
   if (st != CT_OK) return st;
-  return cuda_status(ct_launch_pt(*pc, walk_accel(pc->tlas, P), *P, w, stage, alone, (cudaStream_t)stream));
+  w.alone = alone;
+  return cuda_status(ct_launch_pt(*pc, walk_accel(pc->tlas, P), *P, w, stage, (cudaStream_t)stream));
 }
 
 extern "C" ct_status ct_restir_pt(const ct_push_constant *pc, const ct_params *P, int stage, ct_stream stream) {
@@ -279,10 +285,10 @@ static ct_status render_frame(const ct_push_constant *pc, const ct_params *P, ui
   ct_status st = ct_trace_frame(pc, P, stream);
   if (st != CT_OK) return st;
   const bool indirect = (P->flags & CT_PARAM_INDIRECT) != 0;
-  st = ct_restir_di(pc, P, 0, stream);
+  st = restir_di(pc, P, 0, alone, stream);
   if (st == CT_OK && indirect) st = restir_pt(pc, P, 0, alone, stream);
   if (st != CT_OK) return st;
-  st = ct_restir_di(pc, P, 1, stream);
+  st = restir_di(pc, P, 1, alone, stream);
   if (st == CT_OK && indirect) st = restir_pt(pc, P, 1, alone, stream);
   if (st != CT_OK) return st;
   if (is_active & CT_TAA_BIT) st = ct_taa(pc, P, stream);

@@ -6,6 +6,7 @@
 // (camera matrices, table addresses) are read once per block into shared
 // memory.  Buffers keep the reference's array-of-structs layout so that the
 // caller's RESTIR/WORLD tables are used in place.
+#include <algorithm>
 #include <cuda_runtime.h>
 #include "ct_device.cuh"
 #include <cstddef>
@@ -2139,18 +2140,30 @@ static Workspace make_ws(const CtWorkspace &w, uint32_t counter) {
   return ws;
 }
 
-// blocks of the persistent walkers: ct_params.walker_blocks, else 8 per SM
-static uint32_t walker_grid(const ct_params &P) {
-  return P.walker_blocks ? P.walker_blocks : (uint32_t)sm_count() * 8u;
+// Blocks of the persistent walkers: ct_params.walker_blocks, else 8 per SM, but
+// no more than `threads` (most rays the queue can hold) fill: a block costs its
+// placement and its shared memory even when it finds the queue empty.  Views
+// rendered side by side keep each other's SMs busy and take half (8 views:
+// 2.85 ms with 8 per SM each, 2.34 ms bounded by their rays, 2.24 ms halved,
+// 2.23 ms quartered).
+static uint32_t walker_grid(const ct_params &P, const CtWorkspace &w, uint64_t threads, uint32_t block = 256u) {
+  const uint64_t most = std::max<uint64_t>(((w.alone ? threads : threads / 2u) + block - 1u) / block, 1u);
+  return P.walker_blocks ? P.walker_blocks : (uint32_t)std::min<uint64_t>((uint64_t)sm_count() * 8u, most);
+}
+
+// blocks of 128 for up to `jobs` grid-strided jobs
+static uint32_t job_grid(uint64_t jobs) {
+  return (uint32_t)std::min<uint64_t>((uint64_t)sm_count() * 8u, (jobs + 127u) / 128u);
 }
 
 // the frame accumulates work counters (CT_PARAM_COUNT_RAYS)
 static bool counting(const ct_params &P) { return (P.flags & CT_PARAM_COUNT_RAYS) && P.counters_address; }
 
-static cudaError_t trace_queue(const DevAccel &A, const ct_params &P, const Workspace &ws, cudaStream_t s) {
+static cudaError_t trace_queue(const DevAccel &A, const ct_params &P, const CtWorkspace &w, const Workspace &ws,
+                               uint64_t most_rays, cudaStream_t s) {
   // the queue length is only known on the device: a grid that fills the GPU
   // walks the queue with a grid stride
-  return frame_launch(CT_K_TRACE_SHADOW, s, walker_grid(P), 256,
+  return frame_launch(CT_K_TRACE_SHADOW, s, walker_grid(P, w, most_rays), 256,
                       counting(P) ? k_trace_shadow<true> : k_trace_shadow<false>, A, P, ws);
 }
 
@@ -2158,14 +2171,15 @@ cudaError_t ct_launch_di_stage0(const ct_push_constant &pc, const DevAccel &A, c
                                 const ct_params &P, const CtWorkspace &w, cudaStream_t s) {
   dim3 blk(16, 8);
   const dim3 grid = frame_grid(pc.size[0], pc.size[1], blk);
+  const uint64_t px = (uint64_t)pc.size[0] * pc.size[1];
   const Workspace ws0 = make_ws(w, CT_CTR_DI), ws1 = make_ws(w, CT_CTR_DI + 2);
   cudaError_t e = clear_counters(w, CT_CTR_DI, CT_CTR_DI_END, s);
   if (e == cudaSuccess) e = frame_launch(CT_K_DI_GEN0, s, grid, blk, k_di_gen0<false>, pc, P, ws0, A);
   if (e == cudaSuccess) e = frame_launch(CT_K_DI_GEN0, s, grid, blk, k_di_gen0<true>, pc, P, ws0, A);
-  if (e == cudaSuccess) e = trace_queue(A, P, ws0, s);
+  if (e == cudaSuccess) e = trace_queue(A, P, w, ws0, 2u * px, s);
   if (e == cudaSuccess) e = frame_launch(CT_K_DI_GEN1, s, grid, blk, k_di_gen1, pc, P, ws1);
-  if (e == cudaSuccess) e = trace_queue(A, P, ws1, s);
-  if (e == cudaSuccess) e = frame_launch(CT_K_TRACE_PREV, s, sm_count() * 8, 128, k_trace_prev, pc, A_prev, P, ws1);
+  if (e == cudaSuccess) e = trace_queue(A, P, w, ws1, px, s);
+  if (e == cudaSuccess) e = frame_launch(CT_K_TRACE_PREV, s, job_grid(px), 128, k_trace_prev, pc, A_prev, P, ws1);
   if (e == cudaSuccess) e = frame_launch(CT_K_DI_RESOLVE0, s, grid, blk, k_di_resolve0, pc, P, ws1);
   return e;
 }
@@ -2187,7 +2201,7 @@ cudaError_t ct_launch_spatial_round(const ct_push_constant &pc, const DevAccel &
                      (uint32_t)((threads + CT_SPATIAL_SAMPLE_THREADS - 1) / CT_SPATIAL_SAMPLE_THREADS),
                      CT_SPATIAL_SAMPLE_THREADS, k_spatial_sample, pc, P, ws, src_sel, R);
   }
-  if (e == cudaSuccess) e = trace_queue(A, P, ws, s);
+  if (e == cudaSuccess) e = trace_queue(A, P, w, ws, (uint64_t)pc.size[0] * pc.size[1] * 2u * nmax, s);
   if (e == cudaSuccess)
     e = frame_launch(CT_K_SPATIAL_RESOLVE, s, grid, blk, k_spatial_resolve, pc, P, ws, src_sel, final_pass, dst_sel);
   return e;
@@ -2199,7 +2213,7 @@ cudaError_t ct_launch_taa(const ct_push_constant &pc, const ct_params &P, cudaSt
 }
 
 cudaError_t ct_launch_pt(const ct_push_constant &pc, const DevAccel &A, const ct_params &P, const CtWorkspace &w,
-                         int stage, bool alone, cudaStream_t s) {
+                         int stage, cudaStream_t s) {
   dim3 blk(16, 8);
   const dim3 grid = frame_grid(pc.size[0], pc.size[1], blk);
   const bool hybrid = P.pt_shift_mapping == CT_SHIFT_HYBRID;
@@ -2221,8 +2235,8 @@ cudaError_t ct_launch_pt(const ct_push_constant &pc, const DevAccel &A, const ct
   // is cleared and used again
   uint32_t shadow = CT_CTR_PT_SHADOW;
   Workspace ws = make_ws(w, shadow);
-  const auto flush = [&]() {
-    cudaError_t r = trace_queue(A, P, ws, s);
+  const auto flush = [&](uint64_t most_rays) {
+    cudaError_t r = trace_queue(A, P, w, ws, most_rays, s);
     if (shadow + 4u <= CT_CTR_END) {
       shadow += 2u;
       ws = make_ws(w, shadow);
@@ -2239,30 +2253,30 @@ cudaError_t ct_launch_pt(const ct_push_constant &pc, const DevAccel &A, const ct
   // rays of `group` rounds share the shadow-ray queue and one walker launch.
   const uint64_t px = (uint64_t)pc.size[0] * pc.size[1];
   const int group = px && w.capacity / px > 0 ? (int)(w.capacity / px) : 1;
-  const int rounds = alone && px <= CT_PT_ALONE_PIXELS ? 0 : CT_PT_TAIL_ROUND;
+  const int rounds = w.alone && px <= CT_PT_ALONE_PIXELS ? 0 : CT_PT_TAIL_ROUND;
   for (int it = 0; it < rounds && e == cudaSuccess; it++) {
     const int qi = it & 1;
-    e = frame_launch(CT_K_PT_EXTEND, s, walker_grid(P), 256, counting(P) ? k_pt_extend<true> : k_pt_extend<false>, A, P,
+    e = frame_launch(CT_K_PT_EXTEND, s, walker_grid(P, w, px), 256, counting(P) ? k_pt_extend<true> : k_pt_extend<false>, A, P,
                      pw, qi);
     if (e == cudaSuccess)
-      e = frame_launch(CT_K_PT_SHADE, s, (walker_grid(P) + 1) / 2, 256, k_pt_shade, pc, A, P, ws, pw, qi);
-    if (e == cudaSuccess && ((it + 1) % group == 0 || it + 1 == rounds)) e = flush();
+      e = frame_launch(CT_K_PT_SHADE, s, (walker_grid(P, w, 2u * px) + 1) / 2, 256, k_pt_shade, pc, A, P, ws, pw, qi);
+    if (e == cudaSuccess && ((it + 1) % group == 0 || it + 1 == rounds)) e = flush(px * group);
   }
   if (rounds < CT_PT_MAX_ITER) {
     if (e == cudaSuccess)
-      e = frame_launch(CT_K_PT_FINISH, s, walker_grid(P), 128, k_pt_finish, pc, A, P, ws, pw, rounds & 1, rounds);
-    if (e == cudaSuccess) e = flush();
+      e = frame_launch(CT_K_PT_FINISH, s, walker_grid(P, w, px, 128u), 128, k_pt_finish, pc, A, P, ws, pw, rounds & 1, rounds);
+    if (e == cudaSuccess) e = flush(rounds ? px : w.capacity);
   }
   if (hybrid) {
     // the replays temporal reuse will ask for, walked side by side first
     if (e == cudaSuccess) e = frame_launch(CT_K_PT_REPLAY, s, grid, blk, k_pt_replay_jobs, pc, pw);
-    if (e == cudaSuccess) e = frame_launch(CT_K_PT_REPLAY, s, sm_count() * 8, 128, k_pt_replay, pc, A, P, pw);
+    if (e == cudaSuccess) e = frame_launch(CT_K_PT_REPLAY, s, job_grid(2u * px), 128, k_pt_replay, pc, A, P, pw);
   }
   if (e == cudaSuccess)
     e = frame_launch(CT_K_PT_TEMPORAL, s, grid, blk, hybrid ? k_pt_temporal<0, true> : k_pt_temporal<0, false>, pc, A, P,
                      ws, pw);
   const Workspace answers = ws;
-  if (e == cudaSuccess) e = flush();
+  if (e == cudaSuccess) e = flush(2u * px);
   if (e == cudaSuccess)
     e = frame_launch(CT_K_PT_TEMPORAL, s, grid, blk, hybrid ? k_pt_temporal<1, true> : k_pt_temporal<1, false>, pc, A, P,
                      answers, pw);

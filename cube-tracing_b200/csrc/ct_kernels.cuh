@@ -22,6 +22,7 @@ struct CtWorkspace {
   float *rad;
   uint32_t *nbr;
   void *smeta;
+  bool alone = true;  // no other view's frame runs beside this one
 };
 // A_prev: the scene of pc.tlas_previous (previous-frame visibility of
 // temporal reuse with CT_REMAP_BIT)
@@ -31,9 +32,8 @@ cudaError_t ct_launch_spatial_round(const ct_push_constant &pc, const DevAccel &
                                     const CtWorkspace &w, uint32_t round, int src_sel, int final_pass, int dst_sel,
                                     cudaStream_t s);
 cudaError_t ct_launch_taa(const ct_push_constant &pc, const ct_params &P, cudaStream_t s);
-// alone: no other view's frame runs beside this one
 cudaError_t ct_launch_pt(const ct_push_constant &pc, const DevAccel &A, const ct_params &P, const CtWorkspace &w,
-                         int stage, bool alone, cudaStream_t s);
+                         int stage, cudaStream_t s);
 cudaError_t ct_launch_brush(const ct_push_constant &pc, cudaStream_t s);
 cudaError_t ct_launch_rearrange(const ct_push_constant &pc, uint32_t instance_count, uint32_t primitive_count,
                                 cudaStream_t s);
