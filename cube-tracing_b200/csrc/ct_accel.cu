@@ -8,8 +8,8 @@
 //
 //   pass 1  per AABB: integer voxel coordinate, alignment check, per-instance
 //           bounds (atomic min/max)                        -> host reads bounds
-//   pass 2  per AABB: mark the brick as occupied and every brick its
-//           26-neighbourhood touches as NEAR
+//   pass 2  per AABB: mark, at its brick, the bricks it lies in or touches
+//           with its 26-neighbourhood, which are NEAR
 //   pass 3  per brick cell: give NEAR bricks a mask slot and bricks with
 //           voxels a primitive slot                       -> host reads counts
 //   pass 4  per AABB: set the occupancy bit, keep the lowest primitive id
@@ -41,30 +41,60 @@ struct InstBounds {
 __host__ __device__ inline uint32_t bound_key(int v) { return (uint32_t)v ^ 0x80000000u; }
 __host__ __device__ inline int bound_value(uint32_t k) { return (int)(k ^ 0x80000000u); }
 
-// Per thread minima and maxima over a grid stride, then one reduction and at
-// most 8 atomics per warp: 84 us for 4.1 M voxels, against 533 us with 6
-// atomics per voxel on one instance's 6 words.
+// The low 10 bits of a voxel's coordinates.  A grid has at most 1024 cells per
+// axis, so these give the voxel's place in it exactly, and the passes after
+// k_bounds read 4 bytes per voxel instead of its AABB.
+__device__ __forceinline__ uint32_t pack_low(const int *c) {
+  return ((uint32_t)c[0] & 1023u) | (((uint32_t)c[1] & 1023u) << 10) | (((uint32_t)c[2] & 1023u) << 20);
+}
+
+// An atomic maximum that most callers find done: same-address atomics queue up
+// (8 per warp took 80 us for the 4.1 M voxels below), and a stale load costs one more.
+__device__ __forceinline__ void raise(uint32_t *p, uint32_t v) {
+  if (v > *(volatile uint32_t *)p) atomicMax(p, v);
+}
+
+// Per thread minima and maxima over a grid stride, then one reduction per
+// warp.  Bounded by reading the AABBs: 46 us for 4.1 M voxels (98 MB),
+// against 533 us with 6 atomics per voxel on one instance's 6 words.
+// PAIRS: the AABBs are 8-byte aligned and read as 3 pairs; ie: 1 / e where
+// that makes x * ie the same as x / e (e a power of two), else 0.
+template <bool PAIRS>
 __global__ void __launch_bounds__(256) k_bounds(const ct_instance *inst, const ct_aabb *aabb, uint32_t n_aabb, float e,
-                                                InstBounds *B) {
+                                                float ie, InstBounds *B, uint32_t *low) {
   const uint32_t i = blockIdx.y;
   const uint32_t first = inst[i].first_primitive_index, count = inst[i].primitive_count;
   uint32_t mn[3] = {0u, 0u, 0u}, mx[3] = {0u, 0u, 0u}, inexact = 0u, misaligned = 0u;
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
     const uint32_t gi = first + k;
     if (gi >= n_aabb) { misaligned |= 2u; continue; }
-    const ct_aabb &b = aabb[gi];
+    float b[6];
+    if (PAIRS) {
+      const float2 *p = (const float2 *)aabb + 3ull * gi;
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        const float2 v = p[a];
+        b[2 * a] = v.x;
+        b[2 * a + 1] = v.y;
+      }
+    } else {
+#pragma unroll
+      for (int a = 0; a < 6; a++) b[a] = ((const float *)aabb)[6ull * gi + a];
+    }
     int c[3];
     bool ok = true, exact = true;
+#pragma unroll
     for (int a = 0; a < 3; a++) {
-      const float lo = b.minimum[a], hi = b.maximum[a];
-      const float v = lo / e;
+      const float lo = b[a], hi = b[3 + a];
+      const float v = ie != 0.0f ? lo * ie : lo / e, w = ie != 0.0f ? (hi - lo) * ie : (hi - lo) / e;
       const int iv = __float2int_rn(v);
-      if (!(fabsf(v - (float)iv) <= 1e-3f) || !(fabsf((hi - lo) / e - 1.0f) <= 1e-3f)) ok = false;
+      if (!(fabsf(v - (float)iv) <= 1e-3f) || !(fabsf(w - 1.0f) <= 1e-3f)) ok = false;
       if (!((float)iv * e == lo && (float)(iv + 1) * e == hi)) exact = false;
       c[a] = iv;
     }
     if (!ok) { misaligned |= 1u; continue; }
     if (!exact) inexact = 1u;
+    low[gi] = pack_low(c);
     for (int a = 0; a < 3; a++) {
       mn[a] = max(mn[a], ~bound_key(c[a]));
       mx[a] = max(mx[a], bound_key(c[a]));
@@ -73,8 +103,10 @@ __global__ void __launch_bounds__(256) k_bounds(const ct_instance *inst, const c
   const bool leader = (threadIdx.x & 31u) == 0u;
   for (int a = 0; a < 3; a++) {
     const uint32_t lo = __reduce_max_sync(0xFFFFFFFFu, mn[a]), hi = __reduce_max_sync(0xFFFFFFFFu, mx[a]);
-    if (leader && lo) atomicMax(&B[i].mn[a], lo);
-    if (leader && hi) atomicMax(&B[i].mx[a], hi);
+    if (leader) {
+      raise(&B[i].mn[a], lo);
+      raise(&B[i].mx[a], hi);
+    }
   }
   inexact = __reduce_or_sync(0xFFFFFFFFu, inexact);
   misaligned = __reduce_or_sync(0xFFFFFFFFu, misaligned);
@@ -82,81 +114,83 @@ __global__ void __launch_bounds__(256) k_bounds(const ct_instance *inst, const c
   if (leader && misaligned) atomicOr(&B[i].misaligned, misaligned);
 }
 
-__device__ __forceinline__ bool voxel_local(const ct_aabb &b, float e, const DevGrid &g, int &x, int &y, int &z) {
-  x = __float2int_rn(b.minimum[0] / e) - g.gmin[0];
-  y = __float2int_rn(b.minimum[1] / e) - g.gmin[1];
-  z = __float2int_rn(b.minimum[2] / e) - g.gmin[2];
-  return x >= 0 && y >= 0 && z >= 0 && x < g.bdim[0] * CT_BRICK && y < g.bdim[1] * CT_BRICK && z < g.bdim[2] * CT_BRICK;
+__device__ __forceinline__ bool voxel_local(uint32_t low, const DevGrid &g, int &x, int &y, int &z) {
+  x = (int)((low - (uint32_t)g.gmin[0]) & 1023u);
+  y = (int)(((low >> 10) - (uint32_t)g.gmin[1]) & 1023u);
+  z = (int)(((low >> 20) - (uint32_t)g.gmin[2]) & 1023u);
+  return x < g.bdim[0] * CT_BRICK && y < g.bdim[1] * CT_BRICK && z < g.bdim[2] * CT_BRICK;
 }
 
-__device__ __forceinline__ uint32_t *table_at(uint32_t *table, const DevGrid &g, int bx, int by, int bz) {
-  return &table[g.table_offset + ((uint32_t)bz * g.bdim[1] + by) * g.bdim[0] + bx];
-}
+// Bricks a voxel at local coordinate l of its brick touches along one axis, as
+// bits for the offsets -1, 0, 1
+__device__ __forceinline__ uint32_t touch_axis(int l) { return 2u | (l == 0 ? 1u : 0u) | (l == 7 ? 4u : 0u); }
 
-// Sets bits of a table entry.  Voxels of one brick follow one another, so
-// most find their bits set: a load decides, and only the first few voxels of
-// a brick pay for the atomic (a stale load costs one more atomic, no bits):
-// k_mark takes 67 us for 4.1 M voxels, against 120 us with an atomic each.
-__device__ __forceinline__ void table_or(uint32_t *p, uint32_t bits) {
-  if ((*(volatile uint32_t *)p & bits) != bits) atomicOr(p, bits);
-}
-
-// bit 0 of a table entry marks "has voxels" until slots are assigned
-__global__ void k_mark(const DevGrid *grids, uint32_t n_inst, const ct_aabb *aabb, float e, uint32_t *table) {
-  const uint32_t i = blockIdx.y;
-  if (i >= n_inst) return;
-  const DevGrid g = grids[i];
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < g.primitive_count; k += gridDim.x * blockDim.x) {
+// Per brick, the 27 bricks around it (bit (dz+1)*9 + (dy+1)*3 + (dx+1), itself
+// bit 13) that its voxels lie in or touch.  Voxels of one brick follow one
+// another, so most find their bits set: a load decides, and only the first few
+// pay for the atomic (a stale load costs one more atomic, no bits).  35 us
+// for 4.1 M voxels, against 65 us marking the neighbours' own words (up to 8
+// loads a voxel) and 120 us with an atomic each.
+__global__ void __launch_bounds__(256) k_mark(const DevGrid *grids, const uint32_t *low, uint32_t *marks) {
+  const DevGrid &g = grids[blockIdx.y];
+  const uint32_t n = g.primitive_count;
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     int x, y, z;
-    if (!voxel_local(aabb[g.first_primitive_index + k], e, g, x, y, z)) continue;
-    const int b[3] = {x >> 3, y >> 3, z >> 3};
-    const int l[3] = {x & 7, y & 7, z & 7};
-    table_or(table_at(table, g, b[0], b[1], b[2]), 1u | CT_NEAR_BIT);
-    // bricks the voxel's 26-neighbourhood reaches
-    int lo[3], hi[3];
-    for (int a = 0; a < 3; a++) {
-      lo[a] = (l[a] == 0) ? -1 : 0;
-      hi[a] = (l[a] == 7) ? 1 : 0;
-    }
-    for (int dz = lo[2]; dz <= hi[2]; dz++)
-      for (int dy = lo[1]; dy <= hi[1]; dy++)
-        for (int dx = lo[0]; dx <= hi[0]; dx++) {
-          if (!dx && !dy && !dz) continue;
-          const int nb[3] = {b[0] + dx, b[1] + dy, b[2] + dz};
-          if (nb[0] < 0 || nb[1] < 0 || nb[2] < 0 || nb[0] >= g.bdim[0] || nb[1] >= g.bdim[1] || nb[2] >= g.bdim[2])
-            continue;
-          table_or(table_at(table, g, nb[0], nb[1], nb[2]), CT_NEAR_BIT);
-        }
+    if (!voxel_local(low[g.first_primitive_index + k], g, x, y, z)) continue;
+    const uint32_t tx = touch_axis(x & 7), ty = touch_axis(y & 7), tz = touch_axis(z & 7);
+    const uint32_t row = ((ty & 1u) ? tx : 0u) | (tx << 3) | ((ty & 4u) ? tx << 6 : 0u);
+    const uint32_t bits = ((tz & 1u) ? row : 0u) | (row << 9) | ((tz & 4u) ? row << 18 : 0u);
+    uint32_t *p = &marks[g.table_offset + ((uint32_t)(z >> 3) * g.bdim[1] + (y >> 3)) * g.bdim[0] + (x >> 3)];
+    if ((*(volatile uint32_t *)p & bits) != bits) atomicOr(p, bits);
   }
 }
 
 // counter[0]: mask slots (NEAR bricks), counter[1]: primitive slots (bricks with voxels)
-__global__ void k_assign_slots(uint32_t *table, uint32_t *pslot, uint32_t n_cells, uint32_t *counter) {
-  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n_cells; c += gridDim.x * blockDim.x) {
-    const uint32_t v = table[c];
-    uint32_t slot = CT_EMPTY_SLOT, ps = CT_EMPTY_SLOT;
-    if (v & CT_NEAR_BIT) slot = atomicAdd(&counter[0], 1u);
-    if (v & 1u) ps = atomicAdd(&counter[1], 1u);
-    table[c] = (v & CT_NEAR_BIT) | slot;
-    pslot[c] = ps;
+__global__ void __launch_bounds__(256) k_assign_slots(const DevGrid *grids, const uint32_t *marks, uint32_t *table,
+                                                      uint32_t *pslot, uint32_t *counter) {
+  const DevGrid &g = grids[blockIdx.y];
+  const int X = g.bdim[0], Y = g.bdim[1], Z = g.bdim[2];
+  const uint32_t n = (uint32_t)X * Y * Z;
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
+    const int x = (int)(c % X), y = (int)(c / X % Y), z = (int)(c / (X * Y));
+    const uint32_t *m = marks + g.table_offset;
+    bool near = false;
+    for (int k = 0; k < 27; k++) {
+      // the brick from which this one lies in direction k
+      const int nx = x - (k % 3 - 1), ny = y - (k / 3 % 3 - 1), nz = z - (k / 9 - 1);
+      if ((unsigned)nx < (unsigned)X && (unsigned)ny < (unsigned)Y && (unsigned)nz < (unsigned)Z)
+        near = near || ((m[((uint32_t)nz * Y + ny) * X + nx] >> k) & 1u) != 0u;
+    }
+    const uint32_t at = g.table_offset + c;
+    table[at] = near ? CT_NEAR_BIT | atomicAdd(&counter[0], 1u) : CT_EMPTY_SLOT;
+    pslot[at] = ((m[c] >> 13) & 1u) ? atomicAdd(&counter[1], 1u) : CT_EMPTY_SLOT;
   }
 }
 
-__global__ void k_fill(const DevGrid *grids, uint32_t n_inst, const ct_aabb *aabb, float e, const uint32_t *table,
-                       const uint32_t *pslot, uint32_t *mask, uint32_t *prim, uint32_t *vcoord) {
-  const uint32_t i = blockIdx.y;
-  if (i >= n_inst) return;
-  const DevGrid g = grids[i];
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < g.primitive_count; k += gridDim.x * blockDim.x) {
+// Occupancy bits, the lowest primitive of each voxel and each primitive's
+// voxel.  Whole warps go through the loop together: the lanes whose voxels
+// share an occupancy word (a row's voxels follow one another) set it with one
+// atomic (29 us for 4.1 M voxels, against 55 us with an atomic each).
+__global__ void __launch_bounds__(256) k_fill(const DevGrid *grids, const uint32_t *low, const uint32_t *table,
+                                              const uint32_t *pslot, uint32_t *mask, uint32_t *prim, uint32_t *vcoord) {
+  const DevGrid &g = grids[blockIdx.y];
+  const uint32_t n = g.primitive_count;
+  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+    const uint32_t k = base + threadIdx.x, gi = g.first_primitive_index + k;
+    uint32_t word = 0xFFFFFFFFu, bit = 0u;
     int x, y, z;
-    const uint32_t gi = g.first_primitive_index + k;
-    if (!voxel_local(aabb[gi], e, g, x, y, z)) continue;
-    const uint32_t cell = g.table_offset + ((uint32_t)(z >> 3) * g.bdim[1] + (y >> 3)) * g.bdim[0] + (x >> 3);
-    const uint32_t slot = table[cell] & CT_EMPTY_SLOT;
-    const uint32_t local = (uint32_t)(x & 7) + 8u * (uint32_t)(y & 7) + 64u * (uint32_t)(z & 7);
-    atomicOr(&mask[slot * CT_MASK_WORDS + (local >> 5)], 1u << (local & 31u));
-    atomicMin(&prim[pslot[cell] * 512u + local], k);
-    vcoord[gi] = (uint32_t)x | ((uint32_t)y << 10) | ((uint32_t)z << 20);
+    if (k < n && voxel_local(low[gi], g, x, y, z)) {
+      const uint32_t cell = g.table_offset + ((uint32_t)(z >> 3) * g.bdim[1] + (y >> 3)) * g.bdim[0] + (x >> 3);
+      const uint32_t slot = table[cell] & CT_EMPTY_SLOT;
+      const uint32_t local = (uint32_t)(x & 7) + 8u * (uint32_t)(y & 7) + 64u * (uint32_t)(z & 7);
+      word = slot * CT_MASK_WORDS + (local >> 5);
+      bit = 1u << (local & 31u);
+      atomicMin(&prim[pslot[cell] * 512u + local], k);
+      vcoord[gi] = (uint32_t)x | ((uint32_t)y << 10) | ((uint32_t)z << 20);
+    }
+    const uint32_t same = __match_any_sync(0xFFFFFFFFu, word);
+    const uint32_t bits = __reduce_or_sync(same, bit);
+    if (bit && (threadIdx.x & 31u) == (uint32_t)__ffs(same) - 1u) atomicOr(&mask[word], bits);
   }
 }
 
@@ -174,7 +208,7 @@ __global__ void k_fill(const DevGrid *grids, uint32_t n_inst, const ct_aabb *aab
 // the 8 corners {0, E_j - E_(j-1)}^3 (the smaller cubes cover the larger one
 // as long as that step is at most E_(j-1)).
 constexpr int kFieldCodes = 16;
-constexpr int field_edge_of(int code) {
+__host__ __device__ constexpr int field_edge_of(int code) {
   const uint32_t t[4] = {CT_FIELD_EDGES0, CT_FIELD_EDGES1, CT_FIELD_EDGES2, CT_FIELD_EDGES3};
   return (int)((t[code >> 2] >> (8 * (code & 3))) & 255u);
 }
@@ -230,16 +264,18 @@ __global__ void __launch_bounds__(256) k_occ_rows(const FieldGrid *fg, const uin
 // E_15 - 1 cells past it, and a step reads that much zero padding) are
 // dilated in shared memory, 15 levels from one buffer to the other; each
 // level adds one bit to the bit-sliced codes of the thread's 4 output rows.
-// Bounded by shared-memory reads (4 rows read, 1 written per row and level)
-// and the margin (2.1 rows worked on per row kept): 183 us on the 256^3
-// terrain (9.5 M cells, 8 octants), against 8.5 ms with one byte per cell in
-// HBM and 16 sweeps per octant.
+// Bounded by shared-memory reads (2.5 rows read, 1 written per row and level)
+// and the margin (2.1 rows worked on per row kept): 161 us on the 256^3
+// terrain (9.5 M cells, 8 octants), 183 us with a thread per row (4 read),
+// 8.5 ms with one byte per cell in HBM and 16 sweeps per octant.  512 threads
+// with longer strips (fewer reads, half the warps) made the build 5% slower.
 constexpr int kFieldTile = 64;
 constexpr int kFieldSpan = kFieldTile + CT_FIELD_MAX_EDGE - 1;  // rows per axis with the margin
 constexpr int kFieldPad = field_max_step();  // empty rows a step may read past the margin
-constexpr int kFieldPitch = kFieldSpan + kFieldPad;
 constexpr int kFieldThreads = 1024;
-constexpr uint32_t kFieldSmem = 2u * kFieldPitch * kFieldPitch * sizeof(uint64_t);
+constexpr int kFieldStrip = (kFieldSpan + kFieldThreads / kFieldSpan - 1) / (kFieldThreads / kFieldSpan);  // rows per thread
+constexpr int kFieldPadZ = kFieldPad + kFieldStrip;  // a strip's last rows may lie past the margin
+constexpr uint32_t kFieldSmem = 2u * (kFieldSpan + kFieldPad) * (kFieldSpan + kFieldPadZ) * sizeof(uint64_t);
 static_assert(kFieldSmem <= 227 * 1024, "shared memory per block");
 constexpr int kFieldOut = kFieldTile * kFieldTile / kFieldThreads;  // output rows per thread
 
@@ -258,6 +294,53 @@ __device__ __forceinline__ uint32_t spread_nibbles(uint32_t v) {
   return (v | (v << 3)) & 0x11111111u;
 }
 
+// A block's tile: rows along y and z inside the grid (with the margin, and of
+// the tile itself) and the pitch of a z plane.
+struct FieldTile {
+  int ny, nz, oy, oz, py;
+};
+// Level J on: one more code for the cells whose cube of edge E_J is empty,
+// then the dilation to E_(J+1).  A thread works on a strip of rows along z, so
+// that it reads a row's pair along y once for both ends of the step along z.
+template <int J>
+__device__ __forceinline__ void field_levels(const FieldTile &T, uint64_t *src, uint64_t *dst,
+                                             uint32_t (&c)[kFieldOut][4]) {
+  const int tid = (int)threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < kFieldOut; k++) {
+    const int o = tid + k * kFieldThreads, ly = o % kFieldTile, lz = o / kFieldTile;
+    if (ly < T.oy && lz < T.oz) {
+      uint32_t carry = ~(uint32_t)src[lz * T.py + ly];
+#pragma unroll
+      for (int b = 0; b < 4; b++) {
+        const uint32_t t = c[k][b] & carry;
+        c[k][b] ^= carry;
+        carry = t;
+      }
+    }
+  }
+  if constexpr (J + 1 < kFieldCodes) {
+    constexpr int d = field_edge_of(J + 1) - field_edge_of(J);
+    constexpr int need = CT_FIELD_MAX_EDGE - field_edge_of(J + 1);  // rows past the tile the later levels still read
+    const int rows_y = min(T.ny, kFieldTile + need), rows_z = min(T.nz, kFieldTile + need);
+    const int ly = tid % kFieldSpan, z0 = tid / kFieldSpan * kFieldStrip;
+    if (ly < rows_y && z0 < rows_z) {
+      const uint64_t *r = src + z0 * T.py + ly;
+      uint64_t *w = dst + z0 * T.py + ly;
+      uint64_t a[kFieldStrip + d];
+#pragma unroll
+      for (int i = 0; i < kFieldStrip + d; i++) a[i] = r[i * T.py] | r[i * T.py + d];
+#pragma unroll
+      for (int i = 0; i < kFieldStrip; i++) {
+        const uint64_t v = a[i] | a[i + d];
+        if (z0 + i < rows_z) w[i * T.py] = v | (v >> d);
+      }
+    }
+    __syncthreads();
+    field_levels<J + 1>(T, dst, src, c);
+  }
+}
+
 __global__ void __launch_bounds__(kFieldThreads) k_field(const FieldGrid *fg, const uint32_t *rows, uint32_t *field) {
   extern __shared__ uint64_t s_rows[];
   const FieldGrid f = fg[blockIdx.z];
@@ -268,56 +351,31 @@ __global__ void __launch_bounds__(kFieldThreads) k_field(const FieldGrid *fg, co
             z0 = kFieldTile * (int)(blockIdx.x / (f.xw * ty_n));
   const bool mx = octant & 1u, my = octant & 2u, mz = octant & 4u;
   // rows of the tile and its margin inside the grid; the others stay empty
-  const int ny = min(kFieldSpan, (int)f.Y - y0), nz = min(kFieldSpan, (int)f.Z - z0);
-  const int py = ny + kFieldPad;
+  FieldTile T;
+  T.ny = min(kFieldSpan, (int)f.Y - y0);
+  T.nz = min(kFieldSpan, (int)f.Z - z0);
+  T.oy = min(kFieldTile, T.ny);
+  T.oz = min(kFieldTile, T.nz);
+  T.py = T.ny + kFieldPad;
+  const int oy = T.oy, oz = T.oz;
   const uint32_t tid = threadIdx.x;
-  uint64_t *src = s_rows, *dst = s_rows + py * (nz + kFieldPad);
-  for (int i = (int)tid; i < 2 * py * (nz + kFieldPad); i += kFieldThreads) s_rows[i] = 0ull;
+  const int plane = T.py * (T.nz + kFieldPadZ);
+  uint64_t *src = s_rows, *dst = s_rows + plane;
+  for (int i = (int)tid; i < 2 * plane; i += kFieldThreads) s_rows[i] = 0ull;
   __syncthreads();
-  for (int i = (int)tid; i < ny * nz; i += kFieldThreads) {
-    const int ly = i % ny, lz = i / ny;
+  for (int i = (int)tid; i < T.ny * T.nz; i += kFieldThreads) {
+    const int ly = i % T.ny, lz = i / T.ny;
     const int y = my ? (int)f.Y - 1 - (y0 + ly) : y0 + ly, z = mz ? (int)f.Z - 1 - (z0 + lz) : z0 + lz;
     const uint32_t *row = rows + f.row0 + ((uint64_t)z * f.Y + y) * f.xw;
-    src[lz * py + ly] = mx ? __brevll(row_bits(row, (int)f.xw, (int)f.X - 64 - x0)) : row_bits(row, (int)f.xw, x0);
+    src[lz * T.py + ly] = mx ? __brevll(row_bits(row, (int)f.xw, (int)f.X - 64 - x0)) : row_bits(row, (int)f.xw, x0);
   }
   __syncthreads();
-  const int oy = min(kFieldTile, ny), oz = min(kFieldTile, nz);
   uint32_t c[kFieldOut][4];
 #pragma unroll
   for (int k = 0; k < kFieldOut; k++) {
     c[k][0] = c[k][1] = c[k][2] = c[k][3] = 0u;
   }
-#pragma unroll 1
-  for (int j = 1;; j++) {
-    // one more code for the cells whose cube of edge E_j is empty
-#pragma unroll
-    for (int k = 0; k < kFieldOut; k++) {
-      const int o = (int)tid + k * kFieldThreads, ly = o % kFieldTile, lz = o / kFieldTile;
-      if (ly < oy && lz < oz) {
-        uint32_t carry = ~(uint32_t)src[lz * py + ly];
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-          const uint32_t t = c[k][b] & carry;
-          c[k][b] ^= carry;
-          carry = t;
-        }
-      }
-    }
-    if (j == kFieldCodes - 1) break;
-    const int d = ct_field_edge((uint32_t)j + 1u) - ct_field_edge((uint32_t)j);
-    // rows the later levels still read
-    const int need = CT_FIELD_MAX_EDGE - ct_field_edge((uint32_t)j + 1u);
-    const int my_rows = min(ny, kFieldTile + need), mz_rows = min(nz, kFieldTile + need);
-    for (int i = (int)tid; i < my_rows * mz_rows; i += kFieldThreads) {
-      const uint64_t *r = src + i / my_rows * py + i % my_rows;
-      const uint64_t v = r[0] | r[d] | r[d * py] | r[d * py + d];
-      dst[r - src] = v | (v >> d);
-    }
-    __syncthreads();
-    uint64_t *t = src;
-    src = dst;
-    dst = t;
-  }
+  field_levels<1>(T, src, dst, c);
 #pragma unroll
   for (int k = 0; k < kFieldOut; k++) {
     const int o = (int)tid + k * kFieldThreads, ly = o % kFieldTile, lz = o / kFieldTile;
@@ -456,13 +514,14 @@ extern "C" ct_status ct_build_accel(const ct_scene_desc *scene, ct_accel **out, 
   std::vector<InstBounds> h_b(n_inst);
   std::vector<FieldGrid> hf(n_inst);
   cudaMemPool_t pool = nullptr;
-  Arena scratch, tables, bricks;
-  uint64_t o_fg, o_b, o_counter, o_rows, o_grids, o_table, o_pslot, o_vcoord, o_field, o_mask, o_prim;
+  Arena scratch, marks, tables, bricks;
+  uint64_t o_fg, o_b, o_counter, o_low, o_marks, o_rows, o_grids, o_table, o_pslot, o_vcoord, o_field, o_mask, o_prim;
   InstBounds *d_b = nullptr;
+  uint32_t *d_low = nullptr;      // per AABB: low bits of its coordinates
   uint32_t *d_counter = nullptr;  // [0] mask slots, [1] primitive slots, [2] voxels
   ct_accel *acc = new (std::nothrow) ct_accel();
   if (!acc) return CT_ERR_CAPACITY;
-  uint64_t total_cells = 0, max_prims = 0, field_words = 0, row_words = 0;
+  uint64_t total_cells = 0, max_cells = 0, max_prims = 0, field_words = 0, row_words = 0;
   uint32_t n_slots = 0, n_pslots = 0;
   uint32_t counts[3] = {0, 0, 0};
   uint32_t per_inst = 0;  // blocks per instance of the passes over AABBs
@@ -471,14 +530,25 @@ extern "C" ct_status ct_build_accel(const ct_scene_desc *scene, ct_accel **out, 
   CT_TRY(device_pool(acc->device, &pool));
   o_b = scratch.add(sizeof(InstBounds) * n_inst);
   o_counter = scratch.add(sizeof(counts));
+  o_low = scratch.add(sizeof(uint32_t) * (uint64_t)scene->aabb_count);
   CT_TRY(scratch.alloc(pool, stream));
   d_b = scratch.at<InstBounds>(o_b);
   d_counter = scratch.at<uint32_t>(o_counter);
-  CT_TRY(cudaMemsetAsync(scratch.base, 0, scratch.bytes, stream));
+  d_low = scratch.at<uint32_t>(o_low);
+  CT_TRY(cudaMemsetAsync(scratch.base, 0, o_low, stream));
   // the instances' primitive counts are on the device: a grid for the whole
   // table, spread over the instances
   per_inst = std::max(1u, std::min((scene->aabb_count + 255u) / 256u, std::max(1u, 2048u / n_inst)));
-  k_bounds<<<dim3(per_inst, n_inst), 256, 0, stream>>>(d_inst, d_aabb, scene->aabb_count, e, d_b);
+  {
+    // x / e is x * (1 / e) exactly when e is a power of two of moderate size
+    int exponent = 0;
+    const float ie = frexpf(e, &exponent) == 0.5f && e > 1e-30f && e < 1e30f ? 1.0f / e : 0.0f;
+    const dim3 grid(per_inst, n_inst);
+    if (scene->aabb_address & 7u)
+      k_bounds<false><<<grid, 256, 0, stream>>>(d_inst, d_aabb, scene->aabb_count, e, ie, d_b, d_low);
+    else
+      k_bounds<true><<<grid, 256, 0, stream>>>(d_inst, d_aabb, scene->aabb_count, e, ie, d_b, d_low);
+  }
   CT_TRY(cudaGetLastError());
   CT_TRY(cudaMemcpyAsync(h_inst.data(), d_inst, sizeof(ct_instance) * n_inst, cudaMemcpyDeviceToHost, stream));
   CT_TRY(cudaMemcpyAsync(h_b.data(), d_b, sizeof(InstBounds) * n_inst, cudaMemcpyDeviceToHost, stream));
@@ -520,6 +590,7 @@ extern "C" ct_status ct_build_accel(const ct_scene_desc *scene, ct_accel **out, 
     }
     g.table_offset = (uint32_t)total_cells;
     total_cells += (uint64_t)g.bdim[0] * g.bdim[1] * g.bdim[2];
+    max_cells = std::max(max_cells, (uint64_t)g.bdim[0] * g.bdim[1] * g.bdim[2]);
     if (total_cells > 0x7FFFFFFFull) { st = CT_ERR_CAPACITY; goto fail; }
     if (i == 0)
       for (int a = 0; a < 3; a++) { acc->info.grid_min[a] = mn[a]; acc->info.grid_dim[a] = mx[a] - mn[a] + 1; }
@@ -550,17 +621,22 @@ extern "C" ct_status ct_build_accel(const ct_scene_desc *scene, ct_accel **out, 
   acc->d_vcoord = tables.at<uint32_t>(o_vcoord);
   acc->d_field = tables.at<uint32_t>(o_field);
   CT_TRY(cudaMemcpyAsync(acc->d_grids, acc->h_grids.data(), sizeof(DevGrid) * n_inst, cudaMemcpyHostToDevice, stream));
-  CT_TRY(cudaMemsetAsync(acc->d_table, 0, sizeof(uint32_t) * total_cells, stream));
   acc->n_primitives = scene->aabb_count;
   CT_TRY(cudaMemsetAsync(acc->d_vcoord, 0xFF, sizeof(uint32_t) * (uint64_t)scene->aabb_count, stream));
   {
     dim3 grid((uint32_t)((max_prims + 255) / 256 < 4096 ? (max_prims + 255) / 256 : 4096), n_inst);
     if (grid.x == 0) grid.x = 1;
-    k_mark<<<grid, 256, 0, stream>>>(acc->d_grids, n_inst, d_aabb, e, acc->d_table);
+    o_marks = marks.add(sizeof(uint32_t) * total_cells);
+    CT_TRY(marks.alloc(pool, stream));
+    CT_TRY(cudaMemsetAsync(marks.base, 0, marks.bytes, stream));
+    k_mark<<<grid, 256, 0, stream>>>(acc->d_grids, d_low, marks.at<uint32_t>(o_marks));
     CT_TRY(cudaGetLastError());
-    uint32_t cb = (uint32_t)((total_cells + 255) / 256 < 8192 ? (total_cells + 255) / 256 : 8192);
-    k_assign_slots<<<cb ? cb : 1, 256, 0, stream>>>(acc->d_table, acc->d_pslot, (uint32_t)total_cells, d_counter);
+    const uint64_t cb = (max_cells + 255) / 256;
+    k_assign_slots<<<dim3((uint32_t)std::min<uint64_t>(cb, 8192), n_inst), 256, 0, stream>>>(
+        acc->d_grids, marks.at<uint32_t>(o_marks), acc->d_table, acc->d_pslot, d_counter);
     CT_TRY(cudaGetLastError());
+    CT_TRY(cudaFreeAsync(marks.base, stream));
+    marks.base = nullptr;
     CT_TRY(cudaMemcpyAsync(counts, d_counter, sizeof(counts), cudaMemcpyDeviceToHost, stream));
     CT_TRY(cudaStreamSynchronize(stream));
     n_slots = counts[0];
@@ -574,10 +650,11 @@ extern "C" ct_status ct_build_accel(const ct_scene_desc *scene, ct_accel **out, 
     acc->d_prim = bricks.at<uint32_t>(o_prim);
     CT_TRY(cudaMemsetAsync(acc->d_mask, 0, sizeof(uint32_t) * CT_MASK_WORDS * ns, stream));
     CT_TRY(cudaMemsetAsync(acc->d_prim, 0xFF, sizeof(uint32_t) * 512ull * nps, stream));
-    k_fill<<<grid, 256, 0, stream>>>(acc->d_grids, n_inst, d_aabb, e, acc->d_table, acc->d_pslot, acc->d_mask,
+    k_fill<<<grid, 256, 0, stream>>>(acc->d_grids, d_low, acc->d_table, acc->d_pslot, acc->d_mask,
                                      acc->d_prim, acc->d_vcoord);
     CT_TRY(cudaGetLastError());
-    // the field's scratch takes the place of the bounds'
+    // the field's scratch follows the bounds' (its block is free again once
+    // the kernels above are through with it)
     CT_TRY(cudaFreeAsync(scratch.base, stream));
     scratch = Arena();
     o_counter = scratch.add(sizeof(uint32_t));
@@ -612,6 +689,7 @@ extern "C" ct_status ct_build_accel(const ct_scene_desc *scene, ct_accel **out, 
   return CT_OK;
 fail:
   if (scratch.base) cudaFreeAsync(scratch.base, stream);
+  if (marks.base) cudaFreeAsync(marks.base, stream);
   delete acc;
   return st;
 }
