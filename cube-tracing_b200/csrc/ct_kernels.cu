@@ -191,11 +191,11 @@ __device__ __forceinline__ void pixel_of(uint32_t &x, uint32_t &y) {
 // ---------------------------------------------------------------------------
 // pass 1, front half: primary visibility (rgen.glsl:46-201, 319) with the
 // closest-hit shader (rchit.glsl:18-54) and miss shader (rmiss.glsl:25-28)
-// 6 blocks of 128 per SM (80 registers): 0.77 ms for a 1277x719 frame over
-// four instances against 0.86 ms at 8 blocks and 0.89 ms at 10 (48 registers,
-// spilling); on the 1080p terrain all three take 0.78 ms
+// 5 blocks of 128 per SM (96 registers): 0.655 ms for a 1277x719 frame over
+// four instances against 0.65 ms at 4 blocks, 0.685 ms at 6 and 0.79 ms at 8;
+// on the 1080p terrain 0.59 ms against 0.63, 0.59 and 0.60 ms
 #ifndef CT_PRIMARY_MIN_BLOCKS
-#define CT_PRIMARY_MIN_BLOCKS 6
+#define CT_PRIMARY_MIN_BLOCKS 5
 #endif
 __global__ void __launch_bounds__(128, CT_PRIMARY_MIN_BLOCKS) k_trace_primary(ct_push_constant pc, DevAccel A, ct_params P) {
   grid_begin();
@@ -1764,7 +1764,9 @@ __global__ void __launch_bounds__(128) k_pt_replay_jobs(ct_push_constant pc, PtW
 // Hybrid shift: the replays the jobs list, one per thread over a grid
 // stride, so that a warp walks 32 replays side by side instead of waiting
 // on one lane of a pixel kernel.
-__global__ void __launch_bounds__(128) k_pt_replay(ct_push_constant pc, DevAccel A, ct_params P, PtWork w) {
+// 8 blocks of 128 per SM (64 registers): 0.233 ms with the job list per 1080p
+// frame, against 0.26 ms with the register count left free
+__global__ void __launch_bounds__(128, 8) k_pt_replay(ct_push_constant pc, DevAccel A, ct_params P, PtWork w) {
   grid_begin();
   __shared__ BlockConsts B;
   load_frame_view(pc, B);
