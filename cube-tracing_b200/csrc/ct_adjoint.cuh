@@ -17,8 +17,8 @@
 // registers only while it gathers the suffix radiance S_k from the end of
 // the path back to the camera, then adds the gradients with atomics.
 //
-// One thread per pixel walks its samples in order, so the forward image is
-// the same sum in the same order on every run.
+// A pixel's samples lie on neighbouring lanes; the forward pass adds them up in
+// sample order, so the image is the same sum in the same order on every run.
 
 namespace ct_adjoint {
 
@@ -106,50 +106,101 @@ __device__ __forceinline__ bool emission_of(const Desc &D, const float *emission
 }
 
 // 8 blocks of 128 per SM (64 registers) for both passes: 512x512, 8 samples to
-// depth 3 in a 128^3 grid, forward and backward 3.16 ms, against 3.41 at 9,
-// 3.54 at 6 and 4.20 ms with the register count left free (110); one sample
-// to depth 8 at 1277x719 0.58, 0.60, 0.63 and 0.81 ms.
+// depth 3 in a 128^3 grid, forward and backward 2.54 ms, against 2.58 at 7 and
+// 2.71 at 6 (before the next change).  The walks are bound by instruction fetch: the loops
+// over a path's vertices and a pixel's lanes are kept rolled (2.51 -> 2.37 ms;
+// one sample to depth 8 at 1277x719 0.595 -> 0.543 ms).
 constexpr int kAdjointBlocks = 8;
+
+// A warp takes w x h pixels with `lanes` neighbouring lanes each, a block 2 x 2
+// such tiles.  Lane `sub` of a pixel takes samples sub, sub + lanes, ...: the
+// camera rays of a warp then walk the same cells and the first bounces leave
+// the same faces, and a small image with many samples still fills the GPU.
+// Against one lane per pixel, forward and backward in a 128^3 grid to depth 3:
+// 512x512 with 8 samples 3.06 -> 2.37 ms, 256x256 with 32 5.25 -> 2.43 ms,
+// 100x100 with 64 (terrain) 5.16 -> 0.60 ms.
+struct PixelLanes {
+  uint32_t lanes, w, h, tiles_x;
+};
+// lanes: the largest count up to spp that leaves at least 4/5 of the lanes of
+// all passes with a sample (3 samples at 512x512: 10 pixels of 3 lanes 1.11 ms,
+// 16 of 2, whose second pass is half empty, 1.34 ms, one lane 1.15 ms).
+inline uint32_t pixel_lanes(uint32_t spp) {
+  uint32_t l = spp < 32u ? spp : 32u;
+  while (l > 1u && 5ull * spp * (32u / l) < 4ull * 32u * ((spp + l - 1u) / l)) l--;
+  return l;
+}
+inline PixelLanes lane_layout(uint32_t spp, uint32_t width) {
+  PixelLanes L;
+  L.lanes = pixel_lanes(spp);
+  const uint32_t n = 32u / L.lanes;
+  L.h = n % 16u == 0u ? 4u : n % 2u == 0u ? 2u : 1u;
+  L.w = n / L.h;
+  L.tiles_x = (width + 2u * L.w - 1u) / (2u * L.w);
+  return L;
+}
+inline uint32_t lane_tiles(const PixelLanes &L, uint32_t height) {
+  return L.tiles_x * ((height + 2u * L.h - 1u) / (2u * L.h));
+}
+// this thread's pixel in block `tile` and its lane among the pixel's; false:
+// no pixel of the rectangle
+__device__ __forceinline__ bool lane_pixel(const Desc &D, const PixelLanes &L, uint32_t tile, uint32_t &x, uint32_t &y,
+                                           uint32_t &sub) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, i = lane / L.lanes;
+  sub = lane - i * L.lanes;
+  x = D.x0 + (2u * (tile % L.tiles_x) + (warp & 1u)) * L.w + i % L.w;
+  y = D.y0 + (2u * (tile / L.tiles_x) + (warp >> 1)) * L.h + i / L.w;
+  return i < L.w * L.h && x < D.x1 && y < D.y1;
+}
 
 // Forward: image[p] = (1/spp) sum_s sum_k T_k E[v_k].  Real is the type of
 // the throughput and sums (float for rendering, double for the finite
 // differences of a gradient check).
 template <class Real>
-__global__ void __launch_bounds__(128, sizeof(Real) == 4 ? kAdjointBlocks : 1) k_adjoint_forward(DevAccel A, Desc D, const float *albedo,
-                                                         const float *emission, Real *image) {
+__global__ void __launch_bounds__(128, sizeof(Real) == 4 ? kAdjointBlocks : 1)
+k_adjoint_forward(DevAccel A, Desc D, PixelLanes L, const float *albedo, const float *emission, Real *image) {
   __shared__ Camera C;
   load_camera(D, C);
-  const uint32_t x = D.x0 + blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t y = D.y0 + blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= D.x1 || y >= D.y1) return;
+  uint32_t x, y, sub;
+  const bool inside = lane_pixel(D, L, blockIdx.x, x, y, sub);
   RayStats rs = {};
   uint32_t verts[CT_ADJOINT_MAX_DEPTH];
   Real sx = 0, sy = 0, sz = 0;
-  for (uint32_t s = 0; s < D.spp; s++) {
-    bool missed;
-    const uint32_t n = trace_path(A, D, C, x, y, s, rs, verts, missed);
+  const uint32_t first = (threadIdx.x & 31u) - sub;  // the pixel's first lane
+  for (uint32_t base = 0; base < D.spp; base += L.lanes) {
     Real tx = 1, ty = 1, tz = 1, lx = 0, ly = 0, lz = 0;
-    for (uint32_t k = 0; k < n; k++) {
-      f3 e;
-      if (emission_of(D, emission, verts[k], e)) {
-        lx = lx + tx * (Real)e.x;
-        ly = ly + ty * (Real)e.y;
-        lz = lz + tz * (Real)e.z;
+    if (inside && base + sub < D.spp) {
+      bool missed;
+      const uint32_t n = trace_path(A, D, C, x, y, base + sub, rs, verts, missed);
+#pragma unroll 1
+      for (uint32_t k = 0; k < n; k++) {
+        f3 e;
+        if (emission_of(D, emission, verts[k], e)) {
+          lx = lx + tx * (Real)e.x;
+          ly = ly + ty * (Real)e.y;
+          lz = lz + tz * (Real)e.z;
+        }
+        const f3 a = albedo_of(albedo, verts[k]);
+        tx = tx * (Real)a.x;
+        ty = ty * (Real)a.y;
+        tz = tz * (Real)a.z;
       }
-      const f3 a = albedo_of(albedo, verts[k]);
-      tx = tx * (Real)a.x;
-      ty = ty * (Real)a.y;
-      tz = tz * (Real)a.z;
+      if (missed && D.miss != 0.f) {
+        lx = lx + tx * (Real)D.miss;
+        ly = ly + ty * (Real)D.miss;
+        lz = lz + tz * (Real)D.miss;
+      }
     }
-    if (missed && D.miss != 0.f) {
-      lx = lx + tx * (Real)D.miss;
-      ly = ly + ty * (Real)D.miss;
-      lz = lz + tz * (Real)D.miss;
+    __syncwarp();
+    const uint32_t run = min(L.lanes, D.spp - base);  // the same on every lane
+#pragma unroll 1
+    for (uint32_t j = first; j < first + run; j++) {
+      sx = sx + __shfl_sync(0xFFFFFFFFu, lx, j);
+      sy = sy + __shfl_sync(0xFFFFFFFFu, ly, j);
+      sz = sz + __shfl_sync(0xFFFFFFFFu, lz, j);
     }
-    sx = sx + lx;
-    sy = sy + ly;
-    sz = sz + lz;
   }
+  if (!inside || sub) return;
   const uint32_t p = 3u * (y * D.W + x);
   const Real inv = (Real)1 / (Real)D.spp;
   image[p] = sx * inv;
@@ -159,27 +210,28 @@ __global__ void __launch_bounds__(128, sizeof(Real) == 4 ? kAdjointBlocks : 1) k
 
 // Backward: replays each path, gathers S_k from the last vertex back, adds
 // g T_k S_k to d_albedo[v_k] and g T_k to d_emission[slot of v_k].
-__global__ void __launch_bounds__(128, kAdjointBlocks) k_adjoint_backward(DevAccel A, Desc D, const float *albedo,
-                                                          const float *emission, const float *d_image,
-                                                          float *d_albedo, float *d_emission) {
+__global__ void __launch_bounds__(128, kAdjointBlocks) k_adjoint_backward(DevAccel A, Desc D, PixelLanes L,
+                                                                          const float *albedo, const float *emission,
+                                                                          const float *d_image, float *d_albedo,
+                                                                          float *d_emission) {
   __shared__ Camera C;
   load_camera(D, C);
-  const uint32_t x = D.x0 + blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t y = D.y0 + blockIdx.y * blockDim.y + threadIdx.y;
-  if (x >= D.x1 || y >= D.y1) return;
+  uint32_t x, y, sub;
+  if (!lane_pixel(D, L, blockIdx.x, x, y, sub)) return;
   const uint32_t p = 3u * (y * D.W + x);
   const float inv = 1.0f / (float)D.spp;
   const f3 g = f3{d_image[p] * inv, d_image[p + 1] * inv, d_image[p + 2] * inv};
   if (g.x == 0.f && g.y == 0.f && g.z == 0.f) return;
   RayStats rs = {};
   uint32_t verts[CT_ADJOINT_MAX_DEPTH];
-  for (uint32_t s = 0; s < D.spp; s++) {
+  for (uint32_t s = sub; s < D.spp; s += L.lanes) {
     bool missed;
     const uint32_t n = trace_path(A, D, C, x, y, s, rs, verts, missed);
     if (n == 0) continue;
     // T_k for every vertex, front to back
     f3 T[CT_ADJOINT_MAX_DEPTH];
     f3 t = mk3(1.f);
+#pragma unroll 1
     for (uint32_t k = 0; k < n; k++) {
       T[k] = t;
       t = t * albedo_of(albedo, verts[k]);
@@ -187,6 +239,7 @@ __global__ void __launch_bounds__(128, kAdjointBlocks) k_adjoint_backward(DevAcc
     // S_k back to front: S_{n-1} = the miss light if the path left the
     // scene after v_{n-1}, else 0; S_k = a[v_{k+1}] S_{k+1} + E[v_{k+1}]
     f3 S = missed ? mk3(D.miss) : mk3(0.f);
+#pragma unroll 1
     for (int k = (int)n - 1; k >= 0; k--) {
       const uint32_t v = verts[k];
       const f3 gt = g * T[k];
@@ -349,9 +402,11 @@ __device__ __forceinline__ void nrc_train_path(const DevAccel &A, const Desc &D,
 // One launch for both: the first blocks take the self-training paths (each a
 // long chain of walks, few of them), the others 128 pixels each, so that the
 // pixels' paths fill the GPU while the training paths run.
-// 5 blocks of 128 per SM (96 registers)
+// 5 blocks of 128 per SM (96 registers); a pixel block is a 16 x 8 tile, a warp
+// 8 x 4 of it.  960x540: 303 -> 276 us with that tile and one walk set-up,
+// against rows of 128 pixels and two.
 __global__ void __launch_bounds__(128, 5) k_nrc_trace(DevAccel A, Desc D, const float *albedo, const float *emission,
-                                                   NrcOut out, uint32_t train_blocks) {
+                                                   NrcOut out, uint32_t train_blocks, PixelLanes L) {
   __shared__ Camera C;
   load_camera(D, C);
   if (blockIdx.x < train_blocks) {
@@ -359,9 +414,9 @@ __global__ void __launch_bounds__(128, 5) k_nrc_trace(DevAccel A, Desc D, const 
     if (i < out.train_paths) nrc_train_path(A, D, C, albedo, emission, out, i);
     return;
   }
-  const uint32_t pixel = (blockIdx.x - train_blocks) * blockDim.x + threadIdx.x;
-  if (pixel >= D.W * D.H) return;
-  nrc_trace_pixel(A, D, C, albedo, emission, out, pixel % D.W, pixel / D.W);
+  uint32_t x, y, sub;
+  if (lane_pixel(D, L, blockIdx.x - train_blocks, x, y, sub))
+    nrc_trace_pixel(A, D, C, albedo, emission, out, x, y);
 }
 
 }  // namespace ct_adjoint
@@ -394,10 +449,11 @@ cudaError_t ct_launch_nrc_trace(const DevAccel &A, const ct_adjoint_desc &d, con
   o.tpartial = (float *)(uintptr_t)f.train_partial_address;
   o.tthp = (float *)(uintptr_t)f.train_throughput_address;
   const uint32_t train_blocks = (f.train_paths + 127u) / 128u;
-  const uint32_t pixel_blocks = (uint32_t)(((uint64_t)D.W * D.H + 127u) / 128u);
+  const ct_adjoint::PixelLanes L = ct_adjoint::lane_layout(1u, D.W);
+  const uint32_t pixel_blocks = ct_adjoint::lane_tiles(L, D.H);
   CT_TIMED(CT_K_NRC_TRACE, s,
            ct_adjoint::k_nrc_trace<<<train_blocks + pixel_blocks, 128, 0, s>>>(A, D, albedo, emission, o,
-                                                                                 train_blocks));
+                                                                                 train_blocks, L));
   return cudaGetLastError();
 }
 
@@ -425,19 +481,19 @@ cudaError_t ct_launch_adjoint(const DevAccel &A, const ct_adjoint_desc &d, const
                               void *image, const float *d_image, float *d_albedo, float *d_emission, int backward,
                               cudaStream_t s) {
   const ct_adjoint::Desc D = adjoint_desc(d);
-  const dim3 blk(16, 8);
-  const dim3 grid((D.x1 - D.x0 + blk.x - 1) / blk.x, (D.y1 - D.y0 + blk.y - 1) / blk.y);
-  if (grid.x == 0 || grid.y == 0) return cudaSuccess;
+  const ct_adjoint::PixelLanes L = ct_adjoint::lane_layout(D.spp, D.x1 - D.x0);
+  const uint32_t grid = ct_adjoint::lane_tiles(L, D.y1 - D.y0);
+  if (grid == 0) return cudaSuccess;
   if (backward) {
     CT_TIMED(CT_K_ADJOINT_BACKWARD, s,
-             ct_adjoint::k_adjoint_backward<<<grid, blk, 0, s>>>(A, D, albedo, emission, d_image, d_albedo,
+             ct_adjoint::k_adjoint_backward<<<grid, 128, 0, s>>>(A, D, L, albedo, emission, d_image, d_albedo,
                                                                 d_emission));
   } else if (d.flags & CT_ADJOINT_IMAGE_F64) {
     CT_TIMED(CT_K_ADJOINT_FORWARD, s,
-             ct_adjoint::k_adjoint_forward<double><<<grid, blk, 0, s>>>(A, D, albedo, emission, (double *)image));
+             ct_adjoint::k_adjoint_forward<double><<<grid, 128, 0, s>>>(A, D, L, albedo, emission, (double *)image));
   } else {
     CT_TIMED(CT_K_ADJOINT_FORWARD, s,
-             ct_adjoint::k_adjoint_forward<float><<<grid, blk, 0, s>>>(A, D, albedo, emission, (float *)image));
+             ct_adjoint::k_adjoint_forward<float><<<grid, 128, 0, s>>>(A, D, L, albedo, emission, (float *)image));
   }
   return cudaGetLastError();
 }
