@@ -1148,6 +1148,9 @@ __device__ __forceinline__ f3 random_quad(f3 n, f3 p, f2 s, uint32_t &seed) {
 }
 __device__ __forceinline__ f3 random_unit_vector(uint32_t &seed, uint32_t pixel) {
   f3 p = f3{0.f, 0.f, 0.f};
+  // not unrolled: the copies cost more instruction fetch than they save
+  // (spatial_sample 1.235 -> 1.195 ms, first candidates 766 -> 753 us at 1080p)
+#pragma unroll 1
   for (int i = 0; i < CT_SAMPLER_MAX_TRIES; i++) {
     float a = -1.0f + rnd(seed) * (1.0f - -1.0f);
     float b = -1.0f + rnd(seed) * (1.0f - -1.0f);

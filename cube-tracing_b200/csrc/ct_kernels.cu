@@ -1611,6 +1611,7 @@ __global__ void __launch_bounds__(128, CT_PT_FINISH_MIN_BLOCKS) k_pt_finish(ct_p
   for (uint32_t id = blockIdx.x * blockDim.x + threadIdx.x; id < n; id += gridDim.x * blockDim.x) {
     const uint32_t pixel = __float_as_uint(w.q[qi][2u * id].w);
     PathState path = w.state.load(pixel);
+#pragma unroll 1
     for (int round = first_round; round < CT_PT_MAX_ITER; round++) {
       rs.bounce++;
       ClosestWalk cw;
