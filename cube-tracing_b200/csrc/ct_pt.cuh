@@ -790,21 +790,21 @@ __device__ f3 shift_reconnection(const FrameView &F, const DevAccel &A, float &d
   }
   auto invalid = [](float j) { return j <= 0.f || isnan(j) || isinf(j); };
   if (invalid(jacobian)) return mk3(0.f);
-  const float dst_pdf1 = sample_material_pdf(dst.mat, dst.world_nrm, dst.wo, dst_connection_v);
+  const float dst_pdf1 = sample_material_pdf_call(dst.mat, dst.world_nrm, dst.wo, dst_connection_v);
   const float dst_pdf1_all = dst_pdf1;
   dst_cached.x = dst_pdf1;
   const float src_pdf1 = use_cached_jacobian ? s.cached_jacobian.x
-                                             : sample_material_pdf(src.mat, src.world_nrm, src.wo, src_connection_v);
+                                             : sample_material_pdf_call(src.mat, src.world_nrm, src.wo, src_connection_v);
   jacobian = jacobian * (dst_pdf1 / src_pdf1);
   if (invalid(jacobian)) return mk3(0.f);
   const f3 dst_f1 = evaluate_material(dst.mat, dst.world_nrm, dst.wo, dst_connection_v);
   float dst_rc_pdf_all = 0.f, dst_pdf2 = 1.f, dst_rc_pdf = 1.f, src_rc_pdf = 1.f;
   if (!is_rc_escaped) {
-    dst_rc_pdf = sample_material_pdf(rc.mat, rc.world_nrm, rc.wo, s.rc_wi);
+    dst_rc_pdf = sample_material_pdf_call(rc.mat, rc.world_nrm, rc.wo, s.rc_wi);
     dst_rc_pdf_all = dst_rc_pdf;
     dst_cached.y = dst_rc_pdf;
     src_rc_pdf = use_cached_jacobian ? s.cached_jacobian.y
-                                     : sample_material_pdf(rc.mat, rc.world_nrm, -src_connection_v, s.rc_wi);
+                                     : sample_material_pdf_call(rc.mat, rc.world_nrm, -src_connection_v, s.rc_wi);
     dst_pdf2 = !is_rc_nee ? dst_rc_pdf : s.light_pdf;
   }
   f3 dst_f2 = mk3(1.0f);
