@@ -106,10 +106,11 @@ __device__ __forceinline__ bool emission_of(const Desc &D, const float *emission
 }
 
 // 8 blocks of 128 per SM (64 registers) for both passes: 512x512, 8 samples to
-// depth 3 in a 128^3 grid, forward and backward 2.54 ms, against 2.58 at 7 and
-// 2.71 at 6 (before the next change).  The walks are bound by instruction fetch: the loops
-// over a path's vertices and a pixel's lanes are kept rolled (2.51 -> 2.37 ms;
-// one sample to depth 8 at 1277x719 0.595 -> 0.543 ms).
+// depth 3 in a 128^3 grid, forward and backward 2.28 ms, the same at 7 and 9
+// (2.28, 2.25 ms), 2.71 at 6; one sample to depth 8 at 1277x719 0.534 ms against
+// 0.536 and 0.539.  The walks are bound by instruction fetch, so the loops over
+// a path's vertices and a pixel's lanes stay rolled (2.51 -> 2.37 ms when the
+// walk still called its neighbour test, 0.595 -> 0.543 ms).
 constexpr int kAdjointBlocks = 8;
 
 // A warp takes w x h pixels with `lanes` neighbouring lanes each, a block 2 x 2

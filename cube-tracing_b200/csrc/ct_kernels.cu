@@ -191,9 +191,9 @@ __device__ __forceinline__ void pixel_of(uint32_t &x, uint32_t &y) {
 // ---------------------------------------------------------------------------
 // pass 1, front half: primary visibility (rgen.glsl:46-201, 319) with the
 // closest-hit shader (rchit.glsl:18-54) and miss shader (rmiss.glsl:25-28)
-// 5 blocks of 128 per SM (96 registers): 0.655 ms for a 1277x719 frame over
-// four instances against 0.65 ms at 4 blocks, 0.685 ms at 6 and 0.79 ms at 8;
-// on the 1080p terrain 0.59 ms against 0.63, 0.59 and 0.60 ms
+// 5 blocks of 128 per SM (96 registers): 0.625 ms for a 1277x719 frame over
+// four instances against 0.623 ms at 4 blocks and 0.672 ms at 6; on the 1080p
+// terrain 0.55 ms against 0.585 and 0.55 ms
 #ifndef CT_PRIMARY_MIN_BLOCKS
 #define CT_PRIMARY_MIN_BLOCKS 5
 #endif
