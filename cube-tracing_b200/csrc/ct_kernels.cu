@@ -961,7 +961,9 @@ __global__ void __launch_bounds__(128) k_spatial_resolve(ct_push_constant pc, ct
 //   answer(slot, visible)  its result;  pixel(slot): for error reports
 struct QueueRays {
   Workspace ws;
-  __device__ uint32_t length() const { return ws.q.count[0]; }
+  // a count past the capacity is of rays that were not queued (k_pt_finish
+  // walks those in place; the other passes latch an error)
+  __device__ uint32_t length() const { return min(ws.q.count[0], ws.q.capacity); }
   // one atomic per warp refill on the queue's cursor
   __device__ uint32_t reserve(uint32_t n, uint32_t leader) {
     uint32_t base = 0;
