@@ -30,6 +30,7 @@
 #include <new>
 #include <vector>
 #include "ct_accel.cuh"
+#include "ct_range.h"
 
 // Bounds as unsigned keys that only grow from 0, so that zeroed memory is
 // their start: bound_key(v) is monotone in v, the minimum is kept as ~key.
@@ -58,16 +59,20 @@ __device__ __forceinline__ void raise(uint32_t *p, uint32_t v) {
 // warp.  Bounded by reading the AABBs: 46 us for 4.1 M voxels (98 MB),
 // against 533 us with 6 atomics per voxel on one instance's 6 words.
 // PAIRS: the AABBs are 8-byte aligned and read as 3 pairs; ie: 1 / e where
-// that makes x * ie the same as x / e (e a power of two), else 0.
+// that makes x * ie the same as x / e (e a power of two), else 0.  The ranges
+// come from the caller's table unchecked (the host reads them back with the
+// bounds, so that a build waits for the device once less): only their part
+// inside the AABB table is read, of at most CT_MAX_PRIMITIVES entries, so that
+// the stride cannot wrap either.
 template <bool PAIRS>
 __global__ void __launch_bounds__(256) k_bounds(const ct_instance *inst, const ct_aabb *aabb, uint32_t n_aabb, float e,
                                                 float ie, InstBounds *B, uint32_t *low) {
   const uint32_t i = blockIdx.y;
-  const uint32_t first = inst[i].first_primitive_index, count = inst[i].primitive_count;
+  const uint32_t first = inst[i].first_primitive_index;
+  const uint32_t count = ct_range_inside(first, inst[i].primitive_count, n_aabb);
   uint32_t mn[3] = {0u, 0u, 0u}, mx[3] = {0u, 0u, 0u}, inexact = 0u, misaligned = 0u;
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
     const uint32_t gi = first + k;
-    if (gi >= n_aabb) { misaligned |= 2u; continue; }
     float b[6];
     if (PAIRS) {
       const float2 *p = (const float2 *)aabb + 3ull * gi;
@@ -554,7 +559,7 @@ extern "C" ct_status ct_build_accel(const ct_scene_desc *scene, ct_accel **out, 
   CT_TRY(cudaMemcpyAsync(h_b.data(), d_b, sizeof(InstBounds) * n_inst, cudaMemcpyDeviceToHost, stream));
   CT_TRY(cudaStreamSynchronize(stream));
   for (uint32_t i = 0; i < n_inst; i++) {
-    if ((uint64_t)h_inst[i].first_primitive_index + h_inst[i].primitive_count > scene->aabb_count) {
+    if (ct_range_outside(h_inst[i].first_primitive_index, h_inst[i].primitive_count, scene->aabb_count)) {
       st = CT_ERR_INVALID_ARG;
       goto fail;
     }
@@ -563,7 +568,6 @@ extern "C" ct_status ct_build_accel(const ct_scene_desc *scene, ct_accel **out, 
   acc->h_grids.resize(n_inst);
   acc->info.grid_exact = 1;
   for (uint32_t i = 0; i < n_inst; i++) {
-    if (h_b[i].misaligned & 2u) { st = CT_ERR_INVALID_ARG; goto fail; }
     if (h_b[i].misaligned) { st = CT_ERR_NOT_GRID_ALIGNED; goto fail; }
     DevGrid &g = acc->h_grids[i];
     memset(&g, 0, sizeof(g));
