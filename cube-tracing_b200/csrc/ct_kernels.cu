@@ -38,6 +38,7 @@ static cudaError_t frame_launch(int kid, cudaStream_t s, dim3 grid, dim3 block, 
   cfg.numAttrs = 1;
   cudaError_t e = cudaSuccess;
   CT_TIMED(kid, s, e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...));
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by the next call's check
   return e;
 }
 
