@@ -99,6 +99,15 @@ class NrcMlp(torch.nn.Module):
         return torch.cat([w.detach().reshape(-1) for w in self.weights]).to(torch.bfloat16).contiguous()
 
 
+def _start_autograd(device):
+    """A backward pass of one element.  A training step's backward begins with
+    a matrix product: autograd's thread for the device makes its context
+    current here, which cuBLAS would warn about doing itself.  A cache made
+    for inference alone is made with gradients off, so they are turned on."""
+    with torch.inference_mode(False), torch.enable_grad():
+        torch.zeros(1, device=device, requires_grad=True).neg().backward()
+
+
 class NrcCache:
     """The cache on the device: bf16 weights for ct_nrc_infer, an fp32
     NrcMlp trained with Adam on (query, radiance) pairs."""
@@ -112,10 +121,7 @@ class NrcCache:
         self.weights = torch.zeros(WEIGHT_COUNT, dtype=torch.bfloat16, device=device)
         self.export()
         if torch.device(device).type == "cuda":
-            # a training step's backward begins with a matrix product: let
-            # autograd's thread for the device make its context current here,
-            # which cuBLAS would warn about doing itself
-            torch.zeros(1, device=device, requires_grad=True).neg().backward()
+            _start_autograd(device)
 
     def export(self):
         self.weights.copy_(self.mlp.packed())
