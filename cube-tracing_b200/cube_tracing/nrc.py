@@ -99,6 +99,14 @@ class NrcMlp(torch.nn.Module):
         return torch.cat([w.detach().reshape(-1) for w in self.weights]).to(torch.bfloat16).contiguous()
 
 
+def _kernel_rows(device, rows):
+    """Whether the training step's kernels take these rows: plain fp32 values
+    on the cache's device (torch decides about others, and refuses a mix of
+    devices) that the caller does not want gradients of."""
+    return device.type == "cuda" and all(
+        t.device == device and t.dtype == torch.float32 and not t.requires_grad for t in rows)
+
+
 def _start_autograd(device):
     """A backward pass of one element.  A training step's backward begins with
     a matrix product: autograd's thread for the device makes its context
@@ -173,8 +181,9 @@ class NrcCache:
         n = queries.shape[0]
         enc = torch.empty((n, IN), dtype=torch.float32, device=queries.device)
         net = self.net()
-        native.check("ct_nrc_encode_f32", native.lib().ct_nrc_encode_f32(
-            ctypes.byref(net), queries.data_ptr(), n, enc.data_ptr(), self._stream()))
+        with torch.cuda.device(queries.device):
+            native.check("ct_nrc_encode_f32", native.lib().ct_nrc_encode_f32(
+                ctypes.byref(net), queries.data_ptr(), n, enc.data_ptr(), self._stream()))
         return enc
 
     def train_step(self, queries, targets, weights=None):
@@ -182,23 +191,21 @@ class NrcCache:
         `targets` (n, 3), each query weighted by `weights` (n,) if given;
         the bf16 export follows.  Returns the loss as a device scalar (no
         host synchronisation)."""
-        # rows the library's kernels take: plain fp32 values on this device
-        # that the caller does not want gradients of
-        plain = [queries, targets] + ([weights] if weights is not None else [])
-        plain = all(t.is_cuda and t.dtype == torch.float32 and not t.requires_grad for t in plain)
+        plain = _kernel_rows(self.weights.device, [queries, targets] + ([weights] if weights is not None else []))
         n = queries.shape[0]
         plain = plain and 0 < n <= 1 << 24 and queries.shape == (n, QUERY_FLOATS)
         enc = self._encode_fp32(queries) if plain else encode(queries, self.bbox_min, self.bbox_extent)
         out = self.mlp(enc)
         self.opt.zero_grad()
         if plain and targets.shape == (n, 3) and weights is not None and weights.shape == (n,) and \
-                out.dtype == torch.float32 and out.shape == (n, OUT):
+                _kernel_rows(self.weights.device, [out.detach()]) and out.shape == (n, OUT):
             # the loss below and its gradient in one kernel
             total = (3.0 * weights.sum()).clamp(min=1.0)
             terms, grad = torch.empty_like(targets, memory_format=torch.contiguous_format), torch.empty_like(out)
             rows = [out.detach().contiguous(), targets.contiguous(), weights.contiguous(), total]
-            native.check("ct_nrc_loss", native.lib().ct_nrc_loss(
-                *[t.data_ptr() for t in rows], n, terms.data_ptr(), grad.data_ptr(), self._stream()))
+            with torch.cuda.device(self.weights.device):
+                native.check("ct_nrc_loss", native.lib().ct_nrc_loss(
+                    *[t.data_ptr() for t in rows], n, terms.data_ptr(), grad.data_ptr(), self._stream()))
             loss = terms.sum() / total
             out.backward(grad)
         else:

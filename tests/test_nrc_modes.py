@@ -1,6 +1,9 @@
 """The radiance cache made and used with gradients off, as a program that only
 renders with it does, and training steps whose inputs the library's kernels do
 not take."""
+import itertools
+import types
+
 import pytest
 import torch
 
@@ -24,3 +27,56 @@ def test_cache_without_gradients(mode):
     want = nrc.NrcCache(*BOX, seed=3).infer(q)
     with mode():
         assert torch.equal(nrc.NrcCache(*BOX, seed=3).infer(q), want)
+
+
+def row(device="cuda:0", dtype=torch.float32, requires_grad=False):
+    return types.SimpleNamespace(device=torch.device(device), dtype=dtype, requires_grad=requires_grad)
+
+
+def test_kernels_take_rows_of_the_caches_device_alone():
+    here = torch.device("cuda:0")
+    assert nrc._kernel_rows(here, [row(), row(), row()])
+    others = [row("cuda:1"), row("cpu"), row("meta"), row(dtype=torch.float64), row(requires_grad=True)]
+    for odd, at in itertools.product(others, range(3)):
+        rows = [row(), row(), row()]
+        rows[at] = odd
+        assert not nrc._kernel_rows(here, rows)
+    # a cache on another device than the current one takes its own rows
+    assert nrc._kernel_rows(torch.device("cuda:1"), [row("cuda:1")] * 3)
+    assert not nrc._kernel_rows(torch.device("cuda:1"), [row()] * 3)
+    assert not nrc._kernel_rows(torch.device("cpu"), [row("cpu")] * 3)
+
+
+def test_encoding_kernel_runs_on_the_rows_device(monkeypatch):
+    """The launch happens with the rows' device current, on its stream."""
+    current = ["cuda:0"]
+
+    class Device:
+        def __init__(self, device):
+            self.device = str(device)
+
+        def __enter__(self):
+            self.before, current[0] = current[0], self.device
+
+        def __exit__(self, *_):
+            current[0] = self.before
+
+    class Rows:
+        shape, device = (5, nrc.QUERY_FLOATS), torch.device("cuda:1")
+
+        def contiguous(self):
+            return self
+
+        def data_ptr(self):
+            return 4096
+
+    calls = []
+    cache = nrc.NrcCache(*BOX, device="cpu")
+    empty = torch.empty
+    monkeypatch.setattr(torch.cuda, "device", Device)
+    monkeypatch.setattr(torch, "empty", lambda *a, device=None, **kw: empty(*a, **kw))
+    monkeypatch.setattr(nrc.NrcCache, "_stream", staticmethod(lambda: f"stream of {current[0]}"))
+    monkeypatch.setattr(nrc.native, "lib", lambda: types.SimpleNamespace(
+        ct_nrc_encode_f32=lambda *a: calls.append((current[0], a[-1])) or nrc.native.CT_OK))
+    cache._encode_fp32(Rows())
+    assert calls == [("cuda:1", "stream of cuda:1")] and current == ["cuda:0"]
