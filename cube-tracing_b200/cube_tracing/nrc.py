@@ -101,10 +101,10 @@ class NrcMlp(torch.nn.Module):
 
 def _kernel_rows(device, rows):
     """Whether the training step's kernels take these rows: plain fp32 values
-    on the cache's device (torch decides about others, and refuses a mix of
-    devices) that the caller does not want gradients of."""
+    on the cache's device (torch decides about others, numbers among them, and
+    refuses a mix of devices) that the caller does not want gradients of."""
     return device.type == "cuda" and all(
-        t.device == device and t.dtype == torch.float32 and not t.requires_grad for t in rows)
+        getattr(t, "device", None) == device and t.dtype == torch.float32 and not t.requires_grad for t in rows)
 
 
 def _start_autograd(device):

@@ -80,3 +80,12 @@ def test_encoding_kernel_runs_on_the_rows_device(monkeypatch):
         ct_nrc_encode_f32=lambda *a: calls.append((current[0], a[-1])) or nrc.native.CT_OK))
     cache._encode_fp32(Rows())
     assert calls == [("cuda:1", "stream of cuda:1")] and current == ["cuda:0"]
+
+
+def test_one_target_for_all_rows():
+    """A number, or a tensor that broadcasts, as every row's target."""
+    q = nrc.random_queries(9, seed=2, device="cpu", bbox_min=BOX[0], bbox_extent=BOX[1])
+    full = torch.full((9, 3), 0.75)
+    losses = [nrc.NrcCache(*BOX, device="cpu", seed=1).train_step(q, t) for t in (full, 0.75, full[:1], full[0, 0])]
+    assert all(torch.equal(v, losses[0]) for v in losses)
+    assert not nrc._kernel_rows(torch.device("cuda:0"), [row(), 0.75])
