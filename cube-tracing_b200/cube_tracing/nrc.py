@@ -142,6 +142,11 @@ class NrcCache:
             n.bbox_extent[i] = self.bbox_extent[i]
         return n
 
+    def _box_in_range(self):
+        """Whether the library takes the box (ct_nrc_net)."""
+        n = self.net()
+        return all(math.isfinite(a) and math.isfinite(b) and b > 0 for a, b in zip(n.bbox_min, n.bbox_extent))
+
     @staticmethod
     def _stream():
         return torch.cuda.current_stream().cuda_stream
@@ -193,7 +198,7 @@ class NrcCache:
         host synchronisation)."""
         plain = _kernel_rows(self.weights.device, [queries, targets] + ([weights] if weights is not None else []))
         n = queries.shape[0]
-        plain = plain and 0 < n <= 1 << 24 and queries.shape == (n, QUERY_FLOATS)
+        plain = plain and 0 < n <= 1 << 24 and queries.shape == (n, QUERY_FLOATS) and self._box_in_range()
         enc = self._encode_fp32(queries) if plain else encode(queries, self.bbox_min, self.bbox_extent)
         out = self.mlp(enc)
         self.opt.zero_grad()

@@ -89,3 +89,18 @@ def test_one_target_for_all_rows():
     losses = [nrc.NrcCache(*BOX, device="cpu", seed=1).train_step(q, t) for t in (full, 0.75, full[:1], full[0, 0])]
     assert all(torch.equal(v, losses[0]) for v in losses)
     assert not nrc._kernel_rows(torch.device("cuda:0"), [row(), 0.75])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("extent", [(-256.0, 128.0, 250.0), (256.0, float("inf"), 250.0), (1e39, 128.0, 250.0)])
+@pytest.mark.parametrize("weighted", [True, False])
+def test_training_in_a_box_the_library_refuses(extent, weighted):
+    """Mirrored and unbounded boxes train by the torch expressions, on the GPU
+    as on the CPU."""
+    caches = [nrc.NrcCache(BOX[0], extent, device=d, seed=5) for d in ("cuda", "cpu")]
+    assert not caches[0]._box_in_range() and nrc.NrcCache(*BOX, device="cpu")._box_in_range()
+    q = nrc.random_queries(65, seed=3, bbox_min=BOX[0], bbox_extent=BOX[1])
+    rows = [q, torch.rand((65, 3), device="cuda")] + ([torch.ones(65, device="cuda")] if weighted else [])
+    gpu, cpu = [c.train_step(*[t.to(c.weights.device) for t in rows]) for c in caches]
+    # the networks differ by the order of fp32 sums of 256 and 64 products
+    assert torch.isfinite(gpu) and abs(float(gpu) - float(cpu)) <= 1e-3 * float(cpu)
