@@ -206,7 +206,8 @@ class NrcCache:
                 _kernel_rows(self.weights.device, [out.detach()]) and out.shape == (n, OUT):
             # the loss below and its gradient in one kernel
             total = (3.0 * weights.sum()).clamp(min=1.0)
-            terms, grad = torch.empty_like(targets, memory_format=torch.contiguous_format), torch.empty_like(out)
+            # the kernel writes whole rows, whatever strides the network's output has
+            terms, grad = (torch.empty_like(t, memory_format=torch.contiguous_format) for t in (targets, out))
             rows = [out.detach().contiguous(), targets.contiguous(), weights.contiguous(), total]
             with torch.cuda.device(self.weights.device):
                 native.check("ct_nrc_loss", native.lib().ct_nrc_loss(

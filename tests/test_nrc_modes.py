@@ -104,3 +104,23 @@ def test_training_in_a_box_the_library_refuses(extent, weighted):
     gpu, cpu = [c.train_step(*[t.to(c.weights.device) for t in rows]) for c in caches]
     # the networks differ by the order of fp32 sums of 256 and 64 products
     assert torch.isfinite(gpu) and abs(float(gpu) - float(cpu)) <= 1e-3 * float(cpu)
+
+
+@pytest.mark.gpu
+def test_gradient_of_a_transposed_output():
+    """A network whose output's storage is column by column: the loss kernel's
+    gradient is the torch expressions'."""
+    from test_gpu_nrc_train import torch_step
+    q = nrc.random_queries(65, seed=3, bbox_min=BOX[0], bbox_extent=BOX[1])
+    t, w = torch.rand((65, 3), device="cuda") * 5.0, torch.ones(65, device="cuda")
+    grads = []
+    for step in (nrc.NrcCache.train_step, torch_step):
+        cache = nrc.NrcCache(*BOX, seed=6)
+        forward = cache.mlp.forward
+        cache.mlp.forward = lambda enc: forward(enc).t().contiguous().t()
+        assert cache.mlp(torch.zeros((65, nrc.IN), device="cuda")).stride() == (1, 65)
+        step(cache, q, t, w)
+        grads.append([p.grad for p in cache.mlp.weights])
+    # sums of up to 256 fp32 products a layer, in another order
+    for a, b in zip(*grads):
+        assert bool((a - b).abs().max() <= 1e-4 * b.abs().max()) and bool(b.abs().max() > 0)
