@@ -24,11 +24,13 @@
 //    applies ReLU and writes the next layer's input;
 //  * the last layer (N 16) writes RGB to global memory.
 // What bounds it is instruction issue: the encoding's 48 sincospi and 128
-// exponentials and the epilogues are some 3000 instructions per query against
-// 42 kFLOP of MMAs, at 4 warps per scheduler (issue 59% active): 2.07 M queries
-// take 341 us.  Whole 64 KB tiles let only two warpgroups in (issue 44%, 573
-// us); encoding a tile before its layers instead of during the previous
-// tile's took 353 us, one barrier for a layer and a block 357 us.
+// exponentials and the epilogues are some 3400 instructions per query against
+// 68 kFLOP of MMAs, at 4 warps per scheduler: 2.07 M queries take 359 us (333
+// us with the bins below 2^-126 flushed to 0, which the weights can bring to
+// the output).  Whole 64 KB tiles let only two warpgroups in (issue 44%, 573
+// us).  With flushed bins, encoding a tile before its layers instead of during
+// the previous tile's took 353 us against 341, one barrier for a layer and a
+// block 357 us.
 // Warpgroups synchronise on their own named barriers.  Operands are staged
 // with ordinary 16-byte shared stores (no TMA).  Every wait is bounded
 // (about one second); a warpgroup that gives up latches an error in the
@@ -180,14 +182,11 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 //   [160, 224) the normal, the same way;
 //   [224, 227) albedo; [227, 256) zero.
 // Bin i of a one-blob with u32 = 32 u: exp(-d^2 / 2), d = u32 - (i + 1/2), as
-// 2^(d^2 * (-log2(e) / 2)).  FTZ: bins below 2^-126 become 0 (the fused
-// network, whose outputs they cannot reach; two instructions less per bin).
-template <bool FTZ>
+// 2^(d^2 * (-log2(e) / 2)), subnormal results kept.
 __device__ __forceinline__ float blob_bin(float u32, int i) {
   const float d = u32 - ((float)i + 0.5f), x = (d * d) * -0.72134752044448170368f;
   float r;
-  if (FTZ) asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  else asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+  asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
 __device__ __forceinline__ uint4 pack8(const float *v) {
@@ -212,14 +211,14 @@ __device__ __forceinline__ void encode_axis(float p, float bmin, float bext, int
     emit(chunk + j, pack8(v));
   }
 }
-template <bool FTZ, class Emit>
+template <class Emit>
 __device__ __forceinline__ void encode_blob(float u, int chunk, Emit &&emit) {
   const float u32 = u * 32.0f;
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     float v[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) v[i] = blob_bin<FTZ>(u32, 8 * j + i);
+    for (int i = 0; i < 8; i++) v[i] = blob_bin(u32, 8 * j + i);
     emit(chunk + j, pack8(v));
   }
 }
@@ -227,19 +226,19 @@ __device__ __forceinline__ float azimuth(const float *w) {
   return atan2f(w[2], w[0]) * (0.5f / 3.14159265358979323846f) + 0.5f;
 }
 __device__ __forceinline__ float elevation(const float *w) { return w[1] * 0.5f + 0.5f; }
-template <int KB, bool FTZ, class Emit>
+template <int KB, class Emit>
 __device__ __forceinline__ void encode_block(const ct_nrc_query &q, const float *bmin, const float *bext, Emit &&emit) {
   if (KB == 0) {
     encode_axis(q.position[0], bmin[0], bext[0], 0, emit);
     encode_axis(q.position[1], bmin[1], bext[1], 4, emit);
   } else if (KB == 1) {
     encode_axis(q.position[2], bmin[2], bext[2], 8, emit);
-    encode_blob<FTZ>(azimuth(q.direction), 12, emit);
+    encode_blob(azimuth(q.direction), 12, emit);
   } else if (KB == 2) {
-    encode_blob<FTZ>(elevation(q.direction), 16, emit);
-    encode_blob<FTZ>(azimuth(q.normal), 20, emit);
+    encode_blob(elevation(q.direction), 16, emit);
+    encode_blob(azimuth(q.normal), 20, emit);
   } else {
-    encode_blob<FTZ>(elevation(q.normal), 24, emit);
+    encode_blob(elevation(q.normal), 24, emit);
     const float v[8] = {q.albedo[0], q.albedo[1], q.albedo[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     emit(28, pack8(v));
 #pragma unroll
@@ -269,13 +268,13 @@ __global__ void __launch_bounds__(kEncodeThreads) k_nrc_encode(const ct_nrc_quer
     __syncwarp();
   };
   const auto put = [&](int ch, uint4 v) { rows[lane][ch & 7] = v; };
-  encode_block<0, false>(qq, mn, ex, put);
+  encode_block<0>(qq, mn, ex, put);
   store(0);
-  encode_block<1, false>(qq, mn, ex, put);
+  encode_block<1>(qq, mn, ex, put);
   store(1);
-  encode_block<2, false>(qq, mn, ex, put);
+  encode_block<2>(qq, mn, ex, put);
   store(2);
-  encode_block<3, false>(qq, mn, ex, put);
+  encode_block<3>(qq, mn, ex, put);
   store(3);
 }
 
@@ -453,7 +452,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_nrc_mlp(const ct_nrc_query *q, 
     const auto fill = [&](auto kb_c) {
       constexpr int kb = decltype(kb_c)::value;
       if (ENCODE) {
-        encode_block<kb, true>(qq, mn, ex, [&](int ch, uint4 v) {
+        encode_block<kb>(qq, mn, ex, [&](int ch, uint4 v) {
           *reinterpret_cast<uint4 *>(smem + buf1 + sw128(row, (uint32_t)ch & 7u)) = v;
         });
       } else {
