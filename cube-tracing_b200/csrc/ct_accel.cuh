@@ -8,10 +8,10 @@
 struct ct_accel {
   DevAccel dev = {};
   std::vector<DevGrid> h_grids;
-  // the pieces below lie in these two blocks of the device's pool
-  void *block[2] = {nullptr, nullptr};
   int device = 0;
   DevGrid *d_grids = nullptr;
+  // the pieces below lie in these two blocks of the device's pool
+  void *block[2] = {nullptr, nullptr};
   uint32_t *d_table = nullptr;
   uint32_t *d_pslot = nullptr;
   uint32_t *d_mask = nullptr;

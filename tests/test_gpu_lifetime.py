@@ -1,0 +1,61 @@
+"""Structures freed while other work goes on: the free waits for work in flight
+on any stream, and leaves the captures of other threads (and relaxed ones of
+its own) alone, as cudaFree does.  Builds and frees from several threads and
+streams share one pool of device memory."""
+import threading
+
+import pytest
+
+
+def scene_buffers(edge=16, seed=1):
+    from cube_tracing import scenes
+    from cube_tracing.frame import SceneBuffers
+    sc = scenes.random_grid_scene(edge, 0.3, seed=seed)
+    return sc, SceneBuffers(sc)
+
+
+def build(sc, sb):
+    from cube_tracing.frame import Accel
+    return Accel(sb.instances, sb.n_instances, sb.aabbs, sb.n_primitives, sc.voxel_extent)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode,thread", [("thread_local", True), ("relaxed", True), ("relaxed", False)])
+def test_free_leaves_captures_alone(mode, thread):
+    import torch
+    sc, sb = scene_buffers()
+    acc = build(sc, sb)
+    x = torch.arange(1024.0, device="cuda")
+    y = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        g.capture_begin(capture_error_mode=mode)
+        y.copy_(x * 2)
+        if thread:
+            t = threading.Thread(target=acc.free)
+            t.start()
+            t.join()
+        else:
+            acc.free()
+        y.add_(1.0)
+        g.capture_end()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, 2 * x + 1)
+
+
+@pytest.mark.gpu
+def test_free_waits_for_work_on_any_stream():
+    import torch
+    sc, sb = scene_buffers()
+    acc = build(sc, sb)
+    torch.cuda.synchronize()
+    done = torch.cuda.Event()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        torch.cuda._sleep(50_000_000)  # some 25 ms
+        done.record()
+    assert not done.query()
+    acc.free()
+    assert done.query()
+    torch.cuda.synchronize()
