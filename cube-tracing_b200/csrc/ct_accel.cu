@@ -441,9 +441,11 @@ static ct_status cuda_fail(cudaError_t e) {
 // Device memory of the structures, from one pool per device, so that a scene
 // that is rebuilt after every edit reuses the memory of the structure it
 // replaced instead of mapping and unmapping it (the 17 cudaMalloc / cudaFree
-// of a build and its release took 2.7 ms on the 256^3 terrain).  The pool
-// keeps at most kPoolKeep bytes beyond what live structures hold; a
-// structure's blocks go back to it when the structure is freed.
+// of a build and its release took 2.7 ms on the 256^3 terrain).  A structure's
+// blocks go back to the pool when it is freed; the pool keeps them as long as
+// all it holds, for live structures too, is at most kPoolKeep, and gives the
+// rest back to the driver (a scene above that maps its memory anew on every
+// rebuild).  ct_release_memory gives back what no structure uses.
 //
 // The structures' grids are small cudaMalloc blocks (see ~ct_accel).  The
 // pool's device keeps another one, so that the driver's slab they lie in stays
@@ -711,6 +713,16 @@ extern "C" ct_status ct_accel_free(ct_accel *acc) {
   if (!acc) return CT_ERR_INVALID_ARG;
   delete acc;
   return CT_OK;
+}
+
+extern "C" ct_status ct_release_memory(void) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return cuda_fail(e);
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if ((size_t)dev >= g_pools.size() || !g_pools[dev]) return CT_OK;  // nothing was built here
+  e = cudaMemPoolTrimTo(g_pools[dev], 0);
+  return e == cudaSuccess ? CT_OK : cuda_fail(e);
 }
 
 extern "C" ct_status ct_accel_get_info(const ct_accel *acc, ct_accel_info *out) {

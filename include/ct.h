@@ -313,7 +313,12 @@ void ct_params_default(ct_params *out);
  * size the allocation.  Duplicate voxels keep the lowest primitive id. */
 ct_status ct_build_accel(const ct_scene_desc *scene, ct_accel **out_accel, ct_stream stream);
 ct_status ct_accel_get_info(const ct_accel *accel, ct_accel_info *out);
+/* Waits for the work in flight on the structure's device.  The memory goes to
+ * a pool of the device for the next build, as long as the pool holds at most
+ * 256 MB (live structures included); ct_release_memory gives what no structure
+ * of the current device uses back to the driver. */
 ct_status ct_accel_free(ct_accel *accel);
+ct_status ct_release_memory(void);
 /* The walk's cell field of one instance's grid for one ray octant (bit 0: x
  * decreasing, bit 1: y, bit 2: z), decoded: one byte per cell, x fastest,
  * the edge of the cube without occupied cells that the walk may take from

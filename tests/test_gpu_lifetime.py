@@ -59,3 +59,35 @@ def test_free_waits_for_work_on_any_stream():
     acc.free()
     assert done.query()
     torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
+def test_release_memory():
+    """The pool's unused memory goes back to the driver; live structures stay."""
+    import gc
+
+    import torch
+    from cube_tracing import native
+    gc.collect()
+    sc, sb = scene_buffers(edge=96)  # a cell field of over 4 MB, brick tables of 30
+    release = native.lib().ct_release_memory
+
+    def free_bytes():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    assert release() == native.CT_OK
+    before = free_bytes()
+    accs = [build(sc, sb) for _ in range(4)]
+    held = before - free_bytes()
+    assert held >= 4 * 8 << 20
+    field = [a.field(0, 3)[0] for a in accs[:1]]
+    for a in accs[1:]:
+        a.free()
+    assert release() == native.CT_OK
+    assert before - free_bytes() <= held // 2  # three of four
+    assert (accs[0].field(0, 3)[0] == field[0]).all()
+    accs[0].free()
+    assert release() == native.CT_OK
+    assert abs(before - free_bytes()) <= 4 << 20
+    build(sc, sb).free()
