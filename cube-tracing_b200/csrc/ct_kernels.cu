@@ -2122,12 +2122,15 @@ cudaError_t ct_launch_trace(const ct_push_constant &pc, const DevAccel &A, const
 enum : uint32_t {
   CT_CTR_DI = 0,        // stage 0: first generation; + 2: second; + 4: rays against the previous scene
   CT_CTR_DI_END = 6,
-  CT_CTR_SPATIAL = 8,   // 2 per spatial round (up to 16)
-  CT_CTR_SPATIAL_END = 40,
-  CT_CTR_PT = 40,       // path queues, replay jobs
-  CT_CTR_PT_SHADOW = 46, // 2 per walker launch of ReSTIR PT
+  CT_CTR_SPATIAL = 6,   // 2 per spatial round (up to 16)
+  CT_CTR_SPATIAL_END = 38,
+  CT_CTR_PT = 38,       // path queues, replay jobs
+  CT_CTR_PT_SHADOW = 44, // 2 per walker launch of ReSTIR PT
   CT_CTR_END = 64       // 256 bytes
 };
+// a walker launch after each wavefront round at most, after the finishing pass
+// and for path reuse
+static_assert(CT_CTR_PT_SHADOW + 2 * (CT_PT_TAIL_ROUND + 2) <= CT_CTR_END, "counters of the walker launches");
 static_assert(CT_PREV_COUNT == 2u, "previous-scene count behind the second generation's");
 static cudaError_t clear_counters(const CtWorkspace &w, uint32_t first, uint32_t end, cudaStream_t s) {
   return cudaMemsetAsync(w.counter + first, 0, (end - first) * sizeof(uint32_t), s);
@@ -2237,18 +2240,12 @@ cudaError_t ct_launch_pt(const ct_push_constant &pc, const DevAccel &A, const ct
   pw.jobs = (uint32_t *)w.pt_jobs;
   cudaError_t e = clear_counters(w, CT_CTR_PT, CT_CTR_END, s);
   if (e == cudaSuccess) e = frame_launch(CT_K_PT_START, s, grid, blk, k_pt_start, pc, A, P, pw);
-  // the counters of the walker launches in turn; past the last pair, the pair
-  // is cleared and used again
+  // each walker launch has the next pair of counters
   uint32_t shadow = CT_CTR_PT_SHADOW;
   Workspace ws = make_ws(w, shadow);
   const auto flush = [&](uint64_t most_rays) {
-    cudaError_t r = trace_queue(A, P, w, ws, most_rays, s);
-    if (shadow + 4u <= CT_CTR_END) {
-      shadow += 2u;
-      ws = make_ws(w, shadow);
-    } else if (r == cudaSuccess) {
-      r = clear_counters(w, shadow, shadow + 2u, s);
-    }
+    const cudaError_t r = trace_queue(A, P, w, ws, most_rays, s);
+    ws = make_ws(w, shadow += 2u);
     return r;
   };
   // the queue lengths are only known on the device: a fixed number of rounds,
