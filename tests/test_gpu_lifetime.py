@@ -91,3 +91,41 @@ def test_release_memory():
     assert release() == native.CT_OK
     assert abs(before - free_bytes()) <= 4 << 20
     build(sc, sb).free()
+
+
+@pytest.mark.gpu
+def test_builds_and_frees_on_several_threads_and_streams():
+    """Every structure a thread builds, between other threads' builds and
+    frees, has the field of the one built alone."""
+    import numpy as np
+    import torch
+    work = [scene_buffers(edge=e, seed=e) for e in (24, 40, 56, 33)]
+    want = [build(*w).field(0, 5)[0] for w in work]
+    failures = []
+
+    def run(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                kept = []
+                for k in range(12):
+                    j = (i + k) % len(work)
+                    kept.append((build(*work[j]), j))
+                    if k % 3 == i % 3:
+                        acc, j = kept.pop(0)
+                        if not np.array_equal(acc.field(0, 5)[0], want[j]):
+                            failures.append((i, k, j))
+                        acc.free()
+                for acc, j in kept:
+                    if not np.array_equal(acc.field(0, 5)[0], want[j]):
+                        failures.append((i, "end", j))
+                    acc.free()
+        except Exception as e:  # noqa: BLE001
+            failures.append(repr(e))
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures

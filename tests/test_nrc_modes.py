@@ -124,3 +124,24 @@ def test_gradient_of_a_transposed_output():
     # sums of up to 256 fp32 products a layer, in another order
     for a, b in zip(*grads):
         assert bool((a - b).abs().max() <= 1e-4 * b.abs().max()) and bool(b.abs().max() > 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 257])
+def test_unweighted_step_matches_torch(n):
+    """Without weights the encoding is the kernel's and the loss torch's: bit
+    for bit the step written in torch."""
+    a, b = nrc.NrcCache(*BOX, seed=4), nrc.NrcCache(*BOX, seed=4)
+    for k in range(3):
+        q = nrc.random_queries(n, seed=k, bbox_min=BOX[0], bbox_extent=BOX[1])
+        t = torch.rand((n, 3), device="cuda", generator=torch.Generator("cuda").manual_seed(k)) * 5.0
+        pred = b.mlp(nrc.encode(q, b.bbox_min, b.bbox_extent))[:, :3]
+        loss = (((pred - t) ** 2) / (pred.detach() ** 2 + 1e-2)).mean()
+        b.opt.zero_grad()
+        loss.backward()
+        b.opt.step()
+        b.export()
+        assert torch.equal(a.train_step(q, t), loss.detach())
+        for x, y in zip(a.mlp.weights, b.mlp.weights):
+            assert torch.equal(x, y)
+        assert torch.equal(a.weights, b.weights)
