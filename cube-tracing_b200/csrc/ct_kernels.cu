@@ -2065,8 +2065,9 @@ __global__ void __launch_bounds__(256, CT_QUERY_MIN_BLOCKS) k_query_closest(DevA
   }
 }
 // ct_trace_closest on a batch the GPU holds at once: one thread per ray in
-// small blocks, nothing to refill (40 k rays: 40 us against 48 us, 2001 rays
-// 29 us against 34 us)
+// small blocks, nothing to refill (64^3 grid, L2 flushed: 2001 rays 33 us
+// against 37 us, 40 k rays 37 against 41, 113664 rays, the last batch that
+// comes here, 47 and 47)
 __global__ void __launch_bounds__(64) k_query_closest_once(DevAccel A, const ct_ray_query *q, uint32_t n,
                                                            ct_ray_hit *out) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

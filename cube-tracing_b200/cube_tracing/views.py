@@ -107,8 +107,8 @@ class MultiViewRenderer:
 
     def set_schedule(self, lanes, walker="default"):
         """lanes: streams the views are spread over (0: all on the current
-        stream, in order); walker: "default" (8 blocks per SM per view) or
-        "proportional" (blocks in proportion to the view's pixels, a
+        stream, in order); walker: "default" (the library's choice, at most 8 blocks
+        per SM per view) or "proportional" (blocks in proportion to the view's pixels, a
         1920x1080 view getting the default)."""
         px = self.pixels
         self.lane_of = [0] * len(px)

@@ -230,8 +230,9 @@ typedef struct ct_params {
   uint64_t workspace_address;      /* optional caller scratch for ct_restir_di (ct_workspace_size bytes, */
   uint64_t workspace_bytes;        /* 256-byte aligned); 0 = scratch owned by the acceleration structure */
   uint32_t walker_blocks;          /* blocks of 256 threads of the persistent ray walkers (shadow rays, PT
-                                      bounce rays); 0: 8 per SM.  A schedule knob for views rendered side by
-                                      side (ct_render_views); results do not depend on it */
+                                      bounce rays); 0: as many as their rays can fill, up to 8 per SM.  A
+                                      schedule knob for views rendered side by side (ct_render_views);
+                                      results do not depend on it */
   uint32_t pt_shift_mapping;       /* ReSTIR PT shift: CT_SHIFT_RECONNECTION (the reference's, rgen.glsl:282,
                                       437) or CT_SHIFT_HYBRID (reconnection after a random-number replay of
                                       the prefix, with the reconnection vertex chosen as the first vertex
@@ -420,7 +421,9 @@ ct_status ct_state_load(const ct_push_constant *pc, const void *blob, uint64_t b
 ct_status ct_taa(const ct_push_constant *pc, const ct_params *params, ct_stream stream);
 /* The whole frame in the reference's order: trace, DI stage 0, DI stage 1,
  * and TAA when the status block's is_active has CT_TAA_BIT.  `is_active` is
- * the host copy of that word (the library does not read device memory back). */
+ * the host copy of that word (the library does not read device memory back).
+ * The launches are chosen for a view that has the GPU to itself (one thread per
+ * path up to 2^17 pixels); ct_render_views chooses them for views side by side. */
 ct_status ct_render_frame(const ct_push_constant *pc, const ct_params *params, uint32_t is_active, ct_stream stream);
 
 /* Many views rendered side by side (no counterpart in the reference, which
