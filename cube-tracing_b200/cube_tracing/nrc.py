@@ -101,9 +101,10 @@ class NrcMlp(torch.nn.Module):
 
 def _kernel_rows(device, rows):
     """Whether the training step's kernels take these rows: plain fp32 values
-    on the cache's device (torch decides about others, numbers among them, and
-    refuses a mix of devices) that the caller does not want gradients of."""
-    return device.type == "cuda" and all(
+    on the cache's device, the current one, that the caller does not want
+    gradients of.  Torch decides about others, numbers among them, and refuses
+    a mix of devices."""
+    return device.type == "cuda" and device.index == torch.cuda.current_device() and all(
         getattr(t, "device", None) == device and t.dtype == torch.float32 and not t.requires_grad for t in rows)
 
 
@@ -143,9 +144,10 @@ class NrcCache:
         return n
 
     def _box_in_range(self):
-        """Whether the library takes the box (ct_nrc_net)."""
-        n = self.net()
-        return all(math.isfinite(a) and math.isfinite(b) and b > 0 for a, b in zip(n.bbox_min, n.bbox_extent))
+        """Whether the library takes the box (ct_nrc_net), whose extents are
+        finite and above 0 in single precision."""
+        return (all([1.2e-38 < v < 3.4e38 for v in self.bbox_extent]) and
+                all([-3.4e38 < v < 3.4e38 for v in self.bbox_min]))
 
     @staticmethod
     def _stream():
@@ -186,9 +188,8 @@ class NrcCache:
         n = queries.shape[0]
         enc = torch.empty((n, IN), dtype=torch.float32, device=queries.device)
         net = self.net()
-        with torch.cuda.device(queries.device):
-            native.check("ct_nrc_encode_f32", native.lib().ct_nrc_encode_f32(
-                ctypes.byref(net), queries.data_ptr(), n, enc.data_ptr(), self._stream()))
+        native.check("ct_nrc_encode_f32", native.lib().ct_nrc_encode_f32(
+            ctypes.byref(net), queries.data_ptr(), n, enc.data_ptr(), self._stream()))
         return enc
 
     def train_step(self, queries, targets, weights=None):
@@ -203,15 +204,14 @@ class NrcCache:
         out = self.mlp(enc)
         self.opt.zero_grad()
         if plain and targets.shape == (n, 3) and weights is not None and weights.shape == (n,) and \
-                _kernel_rows(self.weights.device, [out.detach()]) and out.shape == (n, OUT):
+                out.device == targets.device and out.dtype == torch.float32 and out.shape == (n, OUT):
             # the loss below and its gradient in one kernel
             total = (3.0 * weights.sum()).clamp(min=1.0)
             # the kernel writes whole rows, whatever strides the network's output has
             terms, grad = (torch.empty_like(t, memory_format=torch.contiguous_format) for t in (targets, out))
             rows = [out.detach().contiguous(), targets.contiguous(), weights.contiguous(), total]
-            with torch.cuda.device(self.weights.device):
-                native.check("ct_nrc_loss", native.lib().ct_nrc_loss(
-                    *[t.data_ptr() for t in rows], n, terms.data_ptr(), grad.data_ptr(), self._stream()))
+            native.check("ct_nrc_loss", native.lib().ct_nrc_loss(
+                *[t.data_ptr() for t in rows], n, terms.data_ptr(), grad.data_ptr(), self._stream()))
             loss = terms.sum() / total
             out.backward(grad)
         else:

@@ -33,7 +33,13 @@ def row(device="cuda:0", dtype=torch.float32, requires_grad=False):
     return types.SimpleNamespace(device=torch.device(device), dtype=dtype, requires_grad=requires_grad)
 
 
-def test_kernels_take_rows_of_the_caches_device_alone():
+@pytest.fixture
+def current_device(monkeypatch):
+    """Makes device 0 current, on a machine without one too."""
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+
+
+def test_kernels_take_rows_of_the_caches_device_alone(current_device):
     here = torch.device("cuda:0")
     assert nrc._kernel_rows(here, [row(), row(), row()])
     others = [row("cuda:1"), row("cpu"), row("meta"), row(dtype=torch.float64), row(requires_grad=True)]
@@ -41,48 +47,13 @@ def test_kernels_take_rows_of_the_caches_device_alone():
         rows = [row(), row(), row()]
         rows[at] = odd
         assert not nrc._kernel_rows(here, rows)
-    # a cache on another device than the current one takes its own rows
-    assert nrc._kernel_rows(torch.device("cuda:1"), [row("cuda:1")] * 3)
-    assert not nrc._kernel_rows(torch.device("cuda:1"), [row()] * 3)
+    # the kernels are launched on the current device: a cache on another one,
+    # whose rows lie there too, trains by the torch expressions
+    assert not nrc._kernel_rows(torch.device("cuda:1"), [row("cuda:1")] * 3)
     assert not nrc._kernel_rows(torch.device("cpu"), [row("cpu")] * 3)
 
 
-def test_encoding_kernel_runs_on_the_rows_device(monkeypatch):
-    """The launch happens with the rows' device current, on its stream."""
-    current = ["cuda:0"]
-
-    class Device:
-        def __init__(self, device):
-            self.device = str(device)
-
-        def __enter__(self):
-            self.before, current[0] = current[0], self.device
-
-        def __exit__(self, *_):
-            current[0] = self.before
-
-    class Rows:
-        shape, device = (5, nrc.QUERY_FLOATS), torch.device("cuda:1")
-
-        def contiguous(self):
-            return self
-
-        def data_ptr(self):
-            return 4096
-
-    calls = []
-    cache = nrc.NrcCache(*BOX, device="cpu")
-    empty = torch.empty
-    monkeypatch.setattr(torch.cuda, "device", Device)
-    monkeypatch.setattr(torch, "empty", lambda *a, device=None, **kw: empty(*a, **kw))
-    monkeypatch.setattr(nrc.NrcCache, "_stream", staticmethod(lambda: f"stream of {current[0]}"))
-    monkeypatch.setattr(nrc.native, "lib", lambda: types.SimpleNamespace(
-        ct_nrc_encode_f32=lambda *a: calls.append((current[0], a[-1])) or nrc.native.CT_OK))
-    cache._encode_fp32(Rows())
-    assert calls == [("cuda:1", "stream of cuda:1")] and current == ["cuda:0"]
-
-
-def test_one_target_for_all_rows():
+def test_one_target_for_all_rows(current_device):
     """A number, or a tensor that broadcasts, as every row's target."""
     q = nrc.random_queries(9, seed=2, device="cpu", bbox_min=BOX[0], bbox_extent=BOX[1])
     full = torch.full((9, 3), 0.75)
