@@ -24,13 +24,13 @@
 //    applies ReLU and writes the next layer's input;
 //  * the last layer (N 16) writes RGB to global memory.
 // What bounds it is instruction issue: the encoding's 48 sincospi and 128
-// exponentials and the epilogues are some 3400 instructions per query against
-// 68 kFLOP of MMAs, at 4 warps per scheduler: 2.07 M queries take 359 us (333
-// us with the bins below 2^-126 flushed to 0, which the weights can bring to
-// the output).  Whole 64 KB tiles let only two warpgroups in (issue 44%, 573
-// us).  With flushed bins, encoding a tile before its layers instead of during
-// the previous tile's took 353 us against 341, one barrier for a layer and a
-// block 357 us.
+// exponentials and the epilogues are some 3500 instructions per query against
+// 68 kFLOP of MMAs, at 4 warps per scheduler (issue 62% active): 2.07 M queries
+// take 359 us (3060 and 333 us with the bins below 2^-126 flushed to 0, which
+// the weights can bring to the output).  Whole 64 KB tiles let only two
+// warpgroups in (issue 44%, 573 us).  With flushed bins, encoding a tile before
+// its layers instead of during the previous tile's took 353 us against 341, one
+// barrier for a layer and a block 357 us.
 // Warpgroups synchronise on their own named barriers.  Operands are staged
 // with ordinary 16-byte shared stores (no TMA).  Every wait is bounded
 // (about one second); a warpgroup that gives up latches an error in the
