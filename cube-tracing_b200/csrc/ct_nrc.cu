@@ -540,10 +540,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_nrc_mlp(const ct_nrc_query *q, 
     next += stride;
     acc ^= 1u;
   }
-  if (*fail != 0u && row == 0) atomicCAS(&g_nrc_status, 0u, 1u);
-  // every tensor-memory read of this CTA is complete (tcgen05.wait::ld)
+  // every tensor-memory read of this CTA is complete (tcgen05.wait::ld), and
+  // every thread's word about its last wait is written
   fence_before();
   __syncthreads();
+  if (row == 0 && *fail != 0u) atomicCAS(&g_nrc_status, 0u, 1u);
   if (warp == 0) {
     fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
