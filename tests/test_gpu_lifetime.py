@@ -76,6 +76,9 @@ def test_release_memory():
         torch.cuda.synchronize()
         return torch.cuda.mem_get_info()[0]
 
+    warm = build(sc, sb)  # torch's own memory for what the test reads
+    warm.field(0, 3)
+    warm.free()
     assert release() == native.CT_OK
     before = free_bytes()
     accs = [build(sc, sb) for _ in range(4)]
